@@ -17,9 +17,11 @@
 
 #include "fsd_brownian.h"
 #include "fsd_device.cuh"
+#include "fsd_green.cuh"
 #include "fsd_kernels.cuh"
 #include "fsd_profile.h"
 #include "fsd_solver.h"
+#include "fsd_wavefft.h"
 
 namespace fsd {
 
@@ -97,8 +99,31 @@ __device__ __forceinline__ void noise_map(const float4 tk, const float2* f, floa
     }
 }
 
-__constant__ int kNzA[6] = {0, 3, 5, 7, 9, 2};
-__constant__ int kNzB[6] = {1, 4, 6, 8, 10, -1};
+// Spectra o[11] of the noise at grid point idx (a pair's smaller index; never
+// the zero mode), m its mirror point.
+__device__ __forceinline__ void noise_point(const float4* __restrict__ gridk, int idx, int m, bool nyq, float fac,
+                                            uint32_t key, uint32_t step, uint32_t stream, float2* o) {
+    const float4 z0 = normal4(key, step, stream, 2 * (uint32_t)idx);
+    const float4 z1 = normal4(key, step, stream, 2 * (uint32_t)idx + 1);
+    float2 f[3];
+    if (m == idx) {
+        const float s2 = 1.414213562373095f * fac;
+        f[0] = make_float2(s2 * z0.x, 0.f);
+        f[1] = make_float2(s2 * z0.y, 0.f);
+        f[2] = make_float2(s2 * z0.z, 0.f);
+    } else {
+        f[0] = make_float2(fac * z0.x, fac * z0.w);
+        f[1] = make_float2(fac * z0.y, fac * z1.x);
+        f[2] = make_float2(fac * z0.z, fac * z1.y);
+    }
+    noise_map(gridk[idx], f, o, 1.0f);
+    if (nyq) {
+        float2 o2[11];
+        noise_map(gridk[m], f, o2, -1.0f);
+#pragma unroll
+        for (int c = 0; c < 11; ++c) o[c] = make_float2(0.5f * (o[c].x + o2[c].x), 0.5f * (o[c].y + o2[c].y));
+    }
+}
 
 __global__ void k_noise_spectrum(float2* __restrict__ grid, const float4* __restrict__ gridk, int Nx, int Ny, int Nz,
                                  float fac, uint32_t key, uint32_t step, uint32_t stream) {
@@ -113,35 +138,39 @@ __global__ void k_noise_spectrum(float2* __restrict__ grid, const float4* __rest
         for (int p = 0; p < 6; ++p) grid[(size_t)p * G] = make_float2(0.f, 0.f);
         return;
     }
-    const float4 z0 = normal4(key, step, stream, 2 * (uint32_t)idx);
-    const float4 z1 = normal4(key, step, stream, 2 * (uint32_t)idx + 1);
-    float2 f[3];
-    if (m == idx) {
-        const float s2 = 1.414213562373095f * fac;
-        f[0] = make_float2(s2 * z0.x, 0.f);
-        f[1] = make_float2(s2 * z0.y, 0.f);
-        f[2] = make_float2(s2 * z0.z, 0.f);
-    } else {
-        f[0] = make_float2(fac * z0.x, fac * z0.w);
-        f[1] = make_float2(fac * z0.y, fac * z1.x);
-        f[2] = make_float2(fac * z0.z, fac * z1.y);
-    }
     float2 o[11];
-    noise_map(gridk[idx], f, o, 1.0f);
-    const bool nyq = (2 * i == Nx) || (2 * j == Ny) || (2 * l == Nz);
-    if (nyq) {
-        float2 o2[11];
-        noise_map(gridk[m], f, o2, -1.0f);
-#pragma unroll
-        for (int c = 0; c < 11; ++c) o[c] = make_float2(0.5f * (o[c].x + o2[c].x), 0.5f * (o[c].y + o2[c].y));
-    }
+    noise_point(gridk, idx, m, (2 * i == Nx) || (2 * j == Ny) || (2 * l == Nz), fac, key, step, stream, o);
 #pragma unroll
     for (int p = 0; p < 6; ++p) {
-        const float2 A = o[kNzA[p]];
-        const float2 Bv = (kNzB[p] >= 0) ? o[kNzB[p]] : make_float2(0.f, 0.f);
+        const float2 A = o[packA(p)];
+        const float2 Bv = (packB(p) >= 0) ? o[packB(p) >= 0 ? packB(p) : 0] : make_float2(0.f, 0.f);
         grid[(size_t)p * G + idx] = make_float2(A.x - Bv.y, A.y + Bv.x);
         if (m != idx) grid[(size_t)p * G + m] = make_float2(A.x + Bv.y, -A.y + Bv.x);
     }
+}
+
+// The same field as half spectra (z <= Nz / 2) of the 11 real grids: each
+// point takes the draws of its pair's smaller index, conjugated when that is
+// the mirror point.
+__global__ void k_noise_half(float2* __restrict__ spec, const float4* __restrict__ gridk, int Nx, int Ny, int Nz, int zp,
+                             float fac, uint32_t key, uint32_t step, uint32_t stream) {
+    const int l = blockIdx.x * blockDim.x + threadIdx.x;
+    if (l > Nz / 2) return;
+    const int i = blockIdx.y / Ny, j = blockIdx.y - i * Ny;
+    const int idx = (i * Ny + j) * Nz + l;
+    const int m = (((Nx - i) % Nx) * Ny + (Ny - j) % Ny) * Nz + (Nz - l) % Nz;
+    const size_t fs = (size_t)Nx * Ny * zp, pt = ((size_t)i * Ny + j) * zp + l;
+    float2 o[11];
+    if (idx == 0) {
+#pragma unroll
+        for (int c = 0; c < 11; ++c) o[c] = make_float2(0.f, 0.f);
+    } else {
+        noise_point(gridk, min(idx, m), max(idx, m), (2 * i == Nx) || (2 * j == Ny) || (2 * l == Nz), fac, key, step,
+                    stream, o);
+    }
+    const float sg = m < idx ? -1.f : 1.f;
+#pragma unroll
+    for (int c = 0; c < 11; ++c) spec[c * fs + pt] = make_float2(o[c].x, sg * o[c].y);
 }
 
 // ------------------------------------------------------------------ vectors
@@ -378,8 +407,12 @@ int brownian_farfield(fsd_handle* h, const float4* pos, uint32_t step, float* ou
     {
         ProfRegion prw(h, R_BROWNIAN_WAVE);
     count_launch();
-    k_noise_spectrum<<<(G + 255) / 256, 256, 0, h->stream>>>(w.grid, w.gridk, g.Nx, g.Ny, g.Nz, fac, h->seed_hashed,
-                                                             step, kStreamFFWave);
+    if (w.spec)
+        k_noise_half<<<dim3((g.Nz / 2 + 32) / 32, g.Nx * g.Ny), 32, 0, h->stream>>>(
+            w.spec, w.gridk, g.Nx, g.Ny, g.Nz, wave_zp(g.Nz), fac, h->seed_hashed, step, kStreamFFWave);
+    else
+        k_noise_spectrum<<<(G + 255) / 256, 256, 0, h->stream>>>(w.grid, w.gridk, g.Nx, g.Ny, g.Nz, fac,
+                                                                 h->seed_hashed, step, kStreamFFWave);
     mobility_wave_from_spectrum(h, pos);
     // Combine into generalized layout (wave part only): needs f4/c4 unused.
     mobility_combine(h, pos, nullptr, w.lz_c, true, false, nullptr);

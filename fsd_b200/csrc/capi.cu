@@ -12,6 +12,7 @@
 #include "fsd_mpnn.h"
 #include "fsd_solver.h"
 #include "fsd_profile.h"
+#include "fsd_wavefft.h"
 
 namespace fsd {
 
@@ -88,6 +89,10 @@ static int allocate(fsd_handle* h) {
     FSD_TRY(dalloc(&w.grid, 6 * G));
     FSD_TRY(dalloc(&w.gridk, G));
     FSD_TRY(dalloc(&w.twiddle, (size_t)h->g.Nx + h->g.Ny + h->g.Nz));
+    if (wave_fft_ok(h->g)) {
+        FSD_TRY(dalloc(&w.spec, wave_spec_elems(h->g)));
+        FSD_TRY(dalloc(&w.green_table, wave_table_elems(h->g)));
+    }
     FSD_TRY(dalloc(&w.f4, N));
     FSD_TRY(dalloc(&w.c4, 2 * (size_t)N));
     FSD_TRY(dalloc(&w.uwave, 11 * (size_t)N));
@@ -138,7 +143,7 @@ static void release(fsd_handle* h) {
     Workspace& w = h->w;
     void* dev[] = {w.nneigh, w.nlist, w.nl_overflow, w.scan_scratch, w.part_cell, w.cell_count, w.cell_start,
                    w.cell_fill, w.cell_parts, w.order, w.lub_n, w.lub_list, w.part_origin_key, w.part_origin, w.bin_count, w.bin_start, w.bin_fill,
-                   w.bin_parts, w.grid, w.gridk, w.twiddle, w.f4, w.c4, w.uwave, w.sx, w.sy, w.sz, w.V, w.Z, w.dred,
+                   w.bin_parts, w.grid, w.gridk, w.twiddle, w.spec, w.green_table, w.f4, w.c4, w.uwave, w.sx, w.sy, w.sz, w.V, w.Z, w.dred,
                    w.hcol, w.hcol2, w.ticket, w.gmres_state, w.pc_t, w.pc_y, w.rhs, w.sol, w.rfd_rhs, w.rfd_sol, w.psi,
                    w.pos_prime, w.vel, w.force, w.lanczos_V, w.lz_a, w.lz_b, w.lz_c, w.lz_dot, h->d_ewald,
                    h->d_res_dist, h->d_res_vals, w.rk_pos, w.rk_posw, w.rk_ori, w.rk_vel, w.rk_u1, w.rk_noise};

@@ -96,6 +96,8 @@ struct Workspace {
     float2* grid = nullptr;        // 6 packed complex grids of G points
     float4* gridk = nullptr;       // wave vector and Green's scale per grid point
     float2* twiddle = nullptr;     // Nx + Ny + Nz twiddles
+    float2* spec = nullptr;        // half spectra of the 11 real grids (specialised transforms only)
+    float4* green_table = nullptr; // wave vector and Green factors per half-spectrum point, 2 float4 each
     // particle work arrays
     float4* f4 = nullptr;          // force per particle
     float4* c4 = nullptr;          // couplet, two float4 per particle

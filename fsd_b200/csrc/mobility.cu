@@ -27,8 +27,10 @@
 #include <mutex>
 
 #include "fsd_device.cuh"
+#include "fsd_green.cuh"
 #include "fsd_kernels.cuh"
 #include "fsd_profile.h"
+#include "fsd_wavefft.h"
 
 namespace fsd {
 
@@ -86,24 +88,8 @@ __device__ __forceinline__ float2 conjf2(float2 a) { return make_float2(a.x, -a.
 // as constants (conjugated for the inverse).
 // cos and sin of -2 pi m / P for the radices used (m < P); folded to
 // constants once the DFT loops are unrolled.
-// Radix 9 uses cos and sin of 2 pi m / 9, m = 1..4, mirrored.
-__host__ __device__ constexpr float root9_c(int m) {
-    return (m == 0) ? 1.0f
-         : (m == 1 || m == 8) ? 0.76604444311897804f
-         : (m == 2 || m == 7) ? 0.17364817766693035f
-         : (m == 3 || m == 6) ? -0.5f
-         : -0.93969262078590838f;
-}
-__host__ __device__ constexpr float root9_s(int m) {
-    return (m == 0) ? 0.0f
-         : (m == 1) ? -0.64278760968653933f : (m == 8) ? 0.64278760968653933f
-         : (m == 2) ? -0.98480775301220806f : (m == 7) ? 0.98480775301220806f
-         : (m == 3) ? -0.86602540378443865f : (m == 6) ? 0.86602540378443865f
-         : (m == 4) ? -0.34202014332566873f : 0.34202014332566873f;
-}
 __host__ __device__ constexpr float root_c(int P, int m) {
-    return P == 9 ? root9_c(m)
-         : P == 2 ? (m == 0 ? 1.0f : -1.0f)
+    return P == 2 ? (m == 0 ? 1.0f : -1.0f)
          : P == 3 ? (m == 0 ? 1.0f : -0.5f)
          : P == 4 ? (m == 0 ? 1.0f : (m == 2 ? -1.0f : 0.0f))
          : P == 5 ? (m == 0 ? 1.0f : (m == 1 || m == 4) ? 0.30901699437494742f : -0.80901699437494742f)
@@ -111,8 +97,7 @@ __host__ __device__ constexpr float root_c(int P, int m) {
                     : (m == 1 || m == 7) ? 0.70710678118654752f : -0.70710678118654752f);
 }
 __host__ __device__ constexpr float root_s(int P, int m) {
-    return P == 9 ? root9_s(m)
-         : P == 2 ? 0.0f
+    return P == 2 ? 0.0f
          : P == 3 ? (m == 0 ? 0.0f : m == 1 ? -0.86602540378443865f : 0.86602540378443865f)
          : P == 4 ? (m == 1 ? -1.0f : m == 3 ? 1.0f : 0.0f)
          : P == 5 ? (m == 0 ? 0.0f : m == 1 ? -0.95105651629515357f : m == 2 ? -0.58778525229247313f
@@ -267,99 +252,6 @@ __global__ void __launch_bounds__(256, 4) k_fft_axis(float2* __restrict__ data, 
     }
 }
 
-// y and z passes of one (grid, x) plane in a single kernel, for Ny = Nz = N =
-// N1 * N2.  The N x N plane (contiguous in global memory, z fastest) sits in
-// shared memory with row stride N + 1.  Each length-N line is transformed in
-// two in-place stages (Cooley-Tukey, N = N1 N2): the N2-point DFTs over the
-// stride-N1 subsequences with the twiddles w_N^(n1 k2), then the N1-point DFTs
-// over contiguous runs of N1, each writing its outputs into the slots it
-// read.  Coefficient k = k2 + N2 k1 of a line therefore ends at slot
-// k1 + N1 k2; the store undoes that order on both axes.  Forward: z lines,
-// then y lines; inverse: y, then z (the order of the separate passes).
-template <int N1, int N2>
-__device__ __forceinline__ int plane_slot(int k) {
-    return k / N2 + N1 * (k % N2);
-}
-
-template <int N1, int N2>
-__device__ __forceinline__ void plane_lines(float2* pl, const float2* tw, bool rows, bool inv) {
-    constexpr int N = N1 * N2, RS = N + 1;
-    // element i of line l: rows (z lines) at l * RS + i, columns (y lines) at i * RS + l
-    const int es = rows ? 1 : RS, ls = rows ? RS : 1;
-    for (int t = threadIdx.x; t < N * N1; t += blockDim.x) {
-        const int l = t % N, n1 = t / N;  // consecutive threads: consecutive lines
-        float2* L = pl + l * ls + n1 * es;
-        float2 y[N2];
-#pragma unroll
-        for (int q = 0; q < N2; ++q) y[q] = L[q * N1 * es];
-        small_dft<N2>(y, inv);
-#pragma unroll
-        for (int q = 0; q < N2; ++q) {
-            float2 w = tw[n1 * q];
-            if (inv) w.y = -w.y;
-            L[q * N1 * es] = q == 0 ? y[0] : cmul(y[q], w);
-        }
-    }
-    __syncthreads();
-    for (int t = threadIdx.x; t < N * N2; t += blockDim.x) {
-        const int l = t % N, k2 = t / N;
-        float2* L = pl + l * ls + k2 * N1 * es;
-        float2 y[N1];
-#pragma unroll
-        for (int q = 0; q < N1; ++q) y[q] = L[q * es];
-        small_dft<N1>(y, inv);
-#pragma unroll
-        for (int q = 0; q < N1; ++q) L[q * es] = y[q];
-    }
-    __syncthreads();
-}
-
-template <int N1, int N2>
-__global__ void __launch_bounds__(256) k_fft_yz(float2* __restrict__ data, int Nx, const float2* __restrict__ tw_global,
-                                                bool inv) {
-    constexpr int N = N1 * N2, RS = N + 1;
-    extern __shared__ float2 smem[];
-    float2* tw = smem;
-    float2* pl = smem + N;
-    for (int i = threadIdx.x; i < N; i += blockDim.x) tw[i] = tw_global[i];
-    const size_t base = (size_t)blockIdx.x * N * N;  // blocks are (grid, x) planes in memory order
-    for (int e = threadIdx.x; e < N * N; e += blockDim.x) {
-        const int y = e / N, z = e - y * N;
-        pl[y * RS + z] = data[base + e];
-    }
-    __syncthreads();
-    if (!inv) {
-        plane_lines<N1, N2>(pl, tw, true, false);
-        plane_lines<N1, N2>(pl, tw, false, false);
-    } else {
-        plane_lines<N1, N2>(pl, tw, false, true);
-        plane_lines<N1, N2>(pl, tw, true, true);
-    }
-    for (int e = threadIdx.x; e < N * N; e += blockDim.x) {
-        const int y = e / N, z = e - y * N;
-        data[base + e] = pl[plane_slot<N1, N2>(y) * RS + plane_slot<N1, N2>(z)];
-    }
-}
-
-// Launches the plane kernel when Ny = Nz has a specialisation; false otherwise.
-static bool fft_yz(fsd_handle* h, bool inv, int ngrids, const float2* twyz) {
-    const int Nx = h->g.Nx, N = h->g.Ny;
-    if (h->g.Nz != N) return false;
-    const size_t shm = sizeof(float2) * ((size_t)N + (size_t)N * (N + 1));
-    const int nblocks = ngrids * Nx;
-    auto go = [&](auto kern) {
-        if (!smem_limit_ok((const void*)kern, shm, "k_fft_yz shared memory")) return;
-        count_launch();
-        kern<<<nblocks, 256, shm, h->stream>>>(h->w.grid, Nx, twyz, inv);
-    };
-    switch (N) {
-        case 72: go(k_fft_yz<8, 9>); return true;
-        case 36: go(k_fft_yz<4, 9>); return true;
-        case 27: go(k_fft_yz<3, 9>); return true;
-        default: return false;
-    }
-}
-
 static int fft_batch_z(int Nx, int Ny, int Nz) {
     // Batches must not straddle two grids: pick B dividing Nx*Ny.
     int B = std::max(1, 2048 / Nz);
@@ -400,19 +292,14 @@ static void fft3d(fsd_handle* h, bool inv, int ngrids, bool skip_x = false) {
         count_launch();
         k_fft_axis<<<nblocks, 256, shm, h->stream>>>(h->w.grid, Nx, Ny, Nz, axis, B, pl, tw, inv, ngrids);
     };
-    // y and z twiddles coincide when Ny = Nz (both tables are exp(-2 pi i m / N)).
     if (!inv) {
-        if (!fft_yz(h, false, ngrids, twz)) {
-            launch(2);
-            launch(1);
-        }
+        launch(2);
+        launch(1);
         if (!skip_x) launch(0);
     } else {
         if (!skip_x) launch(0);
-        if (!fft_yz(h, true, ngrids, twz)) {
-            launch(1);
-            launch(2);
-        }
+        launch(1);
+        launch(2);
     }
 }
 
@@ -452,71 +339,10 @@ void mobility_set_gridk(fsd_handle* h) {
     count_launch();
     k_gridk<<<(G + 255) / 256, 256, 0, h->stream>>>(h->w.gridk, h->g.Nx, h->g.Ny, h->g.Nz, h->box, h->p.xi, h->g.eta,
                                                     two_pi);
+    if (h->w.spec) wave_set_table(h);
 }
 
 // ---------------------------------------------------------------- Green step
-// Spectra order: X Y Z XX XY XZ YX YY YZ ZX ZY (force then couplet / velocity
-// then velocity gradient), as Mobility_WaveSpace_Green_kernel (Mobility.cu:315).
-// sgn = +1 applies the operator at wave vector tk; sgn = -1 applies the
-// operator with its imaginary-unit couplings conjugated (used to average with
-// the mirror point on Nyquist planes).
-__device__ __forceinline__ void green_apply(const float4 tk, const float2* f, float2* o, float sgn) {
-    const float2 fX = f[0], fY = f[1], fZ = f[2];
-    const float2 cXX = f[3], cXY = f[4], cXZ = f[5], cYX = f[6], cYY = f[7], cYZ = f[8], cZX = f[9], cZY = f[10];
-    const float2 cZZ = make_float2(-(cXX.x + cYY.x), -(cXX.y + cYY.y));
-    const float ksq = tk.x * tk.x + tk.y * tk.y + tk.z * tk.z;
-    const float k = sqrtf(ksq);
-    const float2 kdF = make_float2((tk.x * fX.x + tk.y * fY.x + tk.z * fZ.x) / ksq,
-                                   (tk.x * fX.y + tk.y * fY.y + tk.z * fZ.y) / ksq);
-    const float2 Cdkx = make_float2(cXX.x * tk.x + cXY.x * tk.y + cXZ.x * tk.z, cXX.y * tk.x + cXY.y * tk.y + cXZ.y * tk.z);
-    const float2 Cdky = make_float2(cYX.x * tk.x + cYY.x * tk.y + cYZ.x * tk.z, cYX.y * tk.x + cYY.y * tk.y + cYZ.y * tk.z);
-    const float2 Cdkz = make_float2(cZX.x * tk.x + cZY.x * tk.y + cZZ.x * tk.z, cZX.y * tk.x + cZY.y * tk.y + cZZ.y * tk.z);
-    const float2 kdcdk = make_float2((Cdkx.x * tk.x + Cdky.x * tk.y + Cdkz.x * tk.z) / ksq,
-                                     (Cdkx.y * tk.x + Cdky.y * tk.y + Cdkz.y * tk.z) / ksq);
-    const float sk = sinf(k), ck = cosf(k);
-    const float j0 = sk / k;
-    const float j1k = (sk - k * ck) / (ksq * k);
-    // UF: (I - kk) F, real scale.
-    const float Buf = tk.w * j0 * j0;
-    o[0] = make_float2((fX.x - tk.x * kdF.x) * Buf, (fX.y - tk.x * kdF.y) * Buf);
-    o[1] = make_float2((fY.x - tk.y * kdF.x) * Buf, (fY.y - tk.y * kdF.y) * Buf);
-    o[2] = make_float2((fZ.x - tk.z * kdF.x) * Buf, (fZ.y - tk.z * kdF.y) * Buf);
-    // UC: imaginary scale.
-    const float Buc = sgn * (float)((double)(-tk.w * j0) * (3.0 * (double)(sk - k * ck) / (double)(ksq * k)));
-    o[0].x += -(Cdkx.y - tk.x * kdcdk.y) * Buc;
-    o[1].x += -(Cdky.y - tk.y * kdcdk.y) * Buc;
-    o[2].x += -(Cdkz.y - tk.z * kdcdk.y) * Buc;
-    o[0].y += (Cdkx.x - tk.x * kdcdk.x) * Buc;
-    o[1].y += (Cdky.x - tk.y * kdcdk.x) * Buc;
-    o[2].y += (Cdkz.x - tk.z * kdcdk.x) * Buc;
-    // DF: imaginary scale, D_ab = i B (F_a k_b - k_a k_b k.F/k^2).
-    const float Bdf = sgn * (float)((double)(tk.w * j0) * (3.0 * (double)(sk - k * ck) / (double)(ksq * k)));
-    const float fa[3][2] = {{fX.x, fX.y}, {fY.x, fY.y}, {fZ.x, fZ.y}};
-    const float kv[3] = {tk.x, tk.y, tk.z};
-    const int ia[8] = {0, 0, 0, 1, 1, 1, 2, 2};
-    const int ib[8] = {0, 1, 2, 0, 1, 2, 0, 1};
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-        const float kk = kv[ia[c]] * kv[ib[c]];
-        const float Fkr = fa[ia[c]][0] * kv[ib[c]], Fki = fa[ia[c]][1] * kv[ib[c]];
-        o[3 + c] = make_float2(-(Fki - kk * kdF.y) * Bdf, (Fkr - kk * kdF.x) * Bdf);
-    }
-    // DC: real scale.
-    const float Bdc = (float)((double)tk.w * (-1.0) * (-9.0) * (double)j1k * (double)j1k);
-    const float2 Cdk[3] = {Cdkx, Cdky, Cdkz};
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-        const float kk = kv[ia[c]] * kv[ib[c]];
-        o[3 + c].x += (Cdk[ia[c]].x * kv[ib[c]] - kk * kdcdk.x) * Bdc;
-        o[3 + c].y += (Cdk[ia[c]].y * kv[ib[c]] - kk * kdcdk.y) * Bdc;
-    }
-}
-
-// Packed pair p holds spectra (packA(p), packB(p)); compile-time so that the
-// unrolled loops keep the spectra in registers.
-__host__ __device__ constexpr int packA(int p) { return p == 0 ? 0 : p == 1 ? 3 : p == 2 ? 5 : p == 3 ? 7 : p == 4 ? 9 : 2; }
-__host__ __device__ constexpr int packB(int p) { return p == 0 ? 1 : p == 1 ? 4 : p == 2 ? 6 : p == 3 ? 8 : p == 4 ? 10 : -1; }
-
 // Forward x-pass, Green's function and inverse x-pass in one kernel.  A block
 // holds, for all 6 packed grids, a set of x-lines closed under the mirror map
 // (y, z) -> (-y, -z), so both points of every mirror pair {k, -k} are in
@@ -678,104 +504,6 @@ __global__ void __launch_bounds__(256, 3) k_fft_x_green(float2* __restrict__ gri
     }
 }
 
-// Length-N1*N2 transforms of nlines rows (row stride ls) in place: forward
-// leaves coefficient k = k2 + N2 k1 at slot k1 + N1 k2; the inverse runs the
-// adjoint stages in reverse order, from that order back to natural order.
-template <int N1, int N2>
-__device__ __forceinline__ void rows_fwd(float2* buf, int nlines, int ls, const float2* tw) {
-    for (int t = threadIdx.x; t < nlines * N1; t += blockDim.x) {
-        const int l = t % nlines, n1 = t / nlines;
-        float2* L = buf + l * ls + n1;
-        float2 y[N2];
-#pragma unroll
-        for (int q = 0; q < N2; ++q) y[q] = L[q * N1];
-        small_dft<N2>(y, false);
-#pragma unroll
-        for (int q = 0; q < N2; ++q) L[q * N1] = q == 0 ? y[0] : cmul(y[q], tw[n1 * q]);
-    }
-    __syncthreads();
-    for (int t = threadIdx.x; t < nlines * N2; t += blockDim.x) {
-        const int l = t % nlines, k2 = t / nlines;
-        float2* L = buf + l * ls + k2 * N1;
-        float2 y[N1];
-#pragma unroll
-        for (int q = 0; q < N1; ++q) y[q] = L[q];
-        small_dft<N1>(y, false);
-#pragma unroll
-        for (int q = 0; q < N1; ++q) L[q] = y[q];
-    }
-    __syncthreads();
-}
-
-template <int N1, int N2>
-__device__ __forceinline__ void rows_inv(float2* buf, int nlines, int ls, const float2* tw) {
-    for (int t = threadIdx.x; t < nlines * N2; t += blockDim.x) {
-        const int l = t % nlines, k2 = t / nlines;
-        float2* L = buf + l * ls + k2 * N1;
-        float2 y[N1];
-#pragma unroll
-        for (int q = 0; q < N1; ++q) y[q] = L[q];
-        small_dft<N1>(y, true);
-#pragma unroll
-        for (int q = 0; q < N1; ++q) L[q] = y[q];
-    }
-    __syncthreads();
-    for (int t = threadIdx.x; t < nlines * N1; t += blockDim.x) {
-        const int l = t % nlines, n1 = t / nlines;
-        float2* L = buf + l * ls + n1;
-        float2 y[N2];
-#pragma unroll
-        for (int q = 0; q < N2; ++q) y[q] = q == 0 ? L[0] : cmul(L[q * N1], conjf2(tw[n1 * q]));
-        small_dft<N2>(y, true);
-#pragma unroll
-        for (int q = 0; q < N2; ++q) L[q * N1] = y[q];
-    }
-    __syncthreads();
-}
-
-template <int N1, int N2>
-struct DigitSlot {
-    __device__ int operator()(int x) const { return x / N2 + N1 * (x % N2); }
-};
-
-// The fused x-pass for Nx = N1 * N2: one shared buffer, rows padded to N + 1.
-template <int N1, int N2>
-__global__ void __launch_bounds__(256, 3) k_fft_x_green_t(float2* __restrict__ grid, const float4* __restrict__ gridk,
-                                                          int Ny, int Nz, int B, int nzc,
-                                                          const float2* __restrict__ tw_global) {
-    constexpr int n = N1 * N2, LS = n + 1;
-    extern __shared__ float2 smem[];
-    __shared__ int ly[64], lz[64], lmir[64];
-    __shared__ int s_nl, s_np;
-    float2* tw = smem;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) tw[i] = tw_global[i];
-    const size_t G = (size_t)n * Ny * Nz;
-    if (threadIdx.x == 0) {
-        const int2 c = x_green_lines(blockIdx.x, Ny, Nz, B, nzc, ly, lz, lmir);
-        s_nl = c.x;
-        s_np = c.y;
-    }
-    __syncthreads();
-    const int nl = s_nl, np = s_np;
-    const int L6 = 6 * nl;
-    float2* a = smem + n;
-    for (int i = threadIdx.x; i < L6 * n; i += blockDim.x) {
-        const int x = i / L6, q = i - x * L6;
-        const int g = q / nl, l = q - g * nl;
-        a[(size_t)q * LS + x] = grid[(size_t)g * G + ((size_t)x * Ny + ly[l]) * Nz + lz[l]];
-    }
-    __syncthreads();
-    rows_fwd<N1, N2>(a, L6, LS, tw);
-    x_green_pairs(a, nl, np, LS, DigitSlot<N1, N2>(), ly, lz, lmir, gridk, n, Ny, Nz);
-    __syncthreads();
-    rows_inv<N1, N2>(a, L6, LS, tw);
-    for (int i = threadIdx.x; i < L6 * n; i += blockDim.x) {
-        const int x = i / L6, q = i - x * L6;
-        const int g = q / nl, l = q - g * nl;
-        grid[(size_t)g * G + ((size_t)x * Ny + ly[l]) * Nz + lz[l]] = a[(size_t)q * LS + x];
-    }
-}
-
 // Launch of the fused x-pass: z-runs of B (4 unless tuned), fewer when the
 // lines would not fit in shared memory.
 static void fft_x_green(fsd_handle* h) {
@@ -789,19 +517,6 @@ static void fft_x_green(fsd_handle* h) {
     const int nplanes = (Nz % 2 == 0) ? 2 : 1;
     const int nblocks = Ny * nzc + nplanes * (Ny / 2 + 1);
     const size_t shm = sizeof(float2) * ((size_t)Nx + 2 * 12 * (size_t)B * Nx);
-    // Specialised line lengths keep one padded buffer (rows of Nx + 1).
-    const size_t shm_t = sizeof(float2) * ((size_t)Nx + 12 * (size_t)B * (Nx + 1));
-    auto go = [&](auto kern) {
-        if (!smem_limit_ok((const void*)kern, shm_t, "k_fft_x_green_t shared memory")) return;
-        count_launch();
-        kern<<<nblocks, 256, shm_t, h->stream>>>(h->w.grid, h->w.gridk, Ny, Nz, B, nzc, h->w.twiddle);
-    };
-    switch (Nx) {
-        case 72: go(k_fft_x_green_t<8, 9>); return;
-        case 36: go(k_fft_x_green_t<4, 9>); return;
-        case 27: go(k_fft_x_green_t<3, 9>); return;
-        default: break;
-    }
     if (!smem_limit_ok((const void*)k_fft_x_green, shm, "k_fft_x_green shared memory")) return;
     count_launch();
     k_fft_x_green<<<nblocks, 256, shm, h->stream>>>(h->w.grid, h->w.gridk, Nx, Ny, Nz, B, nzc, px, h->w.twiddle);
@@ -1464,7 +1179,12 @@ static void contract(fsd_handle* h, const float4* pos) {
 void mobility_wave_from_spectrum(fsd_handle* h, const float4* pos) {
     {
         ProfRegion pr(h, R_FFT);
-        fft3d(h, true, 6);
+        if (h->w.spec) {
+            wave_inverse_x(h);
+            wave_inverse_yz(h);
+        } else {
+            fft3d(h, true, 6);
+        }
     }
     ProfRegion pr(h, R_CONTRACT);
     contract(h, pos);
@@ -1562,6 +1282,13 @@ static int autotune(fsd_handle* h, const float4* pos) {
                         best.spread_rows = rows;
                     }
                 }
+    if (h->w.spec) {  // the specialised transforms have no launch shape to choose
+        h->tune = best;
+        FSD_CHECK_CUDA(cudaGetLastError());
+        std::lock_guard<std::mutex> lock(g_tune_mu);
+        g_tune_cache.emplace(key, best);
+        return FSD_OK;
+    }
     std::vector<int> bxy, bz;
     for (int d = 8; d <= 32; ++d)
         if (g.Nz % d == 0) bxy.push_back(d);
@@ -1623,15 +1350,18 @@ int mobility_apply(fsd_handle* h, const float4* pos, const float* genF, float* g
         }
         {
             ProfRegion pr(h, R_FFT);
-            fft3d(h, false, 6, true);  // z and y passes
+            if (h->w.spec) wave_forward_yz(h);
+            else fft3d(h, false, 6, true);  // z and y passes
         }
         {
             ProfRegion pr(h, R_GREEN);  // x pass, Green's function, inverse x pass
-            fft_x_green(h);
+            if (h->w.spec) wave_x_green(h);
+            else fft_x_green(h);
         }
         {
             ProfRegion pr(h, R_FFT);
-            fft3d(h, true, 6, true);  // y and z passes
+            if (h->w.spec) wave_inverse_yz(h);
+            else fft3d(h, true, 6, true);  // y and z passes
         }
         {
             ProfRegion pr(h, R_CONTRACT);
