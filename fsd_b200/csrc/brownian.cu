@@ -413,7 +413,8 @@ int brownian_farfield(fsd_handle* h, const float4* pos, uint32_t step, float* ou
     else
         k_noise_spectrum<<<(G + 255) / 256, 256, 0, h->stream>>>(w.grid, w.gridk, g.Nx, g.Ny, g.Nz, fac,
                                                                  h->seed_hashed, step, kStreamFFWave);
-    mobility_wave_from_spectrum(h, pos);
+    const int e = mobility_wave_from_spectrum(h, pos);
+    if (e != FSD_OK) return e;
     // Combine into generalized layout (wave part only): needs f4/c4 unused.
     mobility_combine(h, pos, nullptr, w.lz_c, true, false, nullptr);
     }

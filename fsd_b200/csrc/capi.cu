@@ -70,8 +70,7 @@ static int allocate(fsd_handle* h) {
     // Cell capacity for the untilted box (tilting only removes cells).
     const int3 nc = cell_dims(Box{h->box.Lx, h->box.Ly, h->box.Lz, 0.0f}, rlist);
     w.ncell_cap = (nc.x >= 3 && nc.y >= 3 && nc.z >= 3) ? (size_t)nc.x * nc.y * nc.z : 0;
-    const size_t nbins = std::max(w.ncell_cap, G);
-    FSD_TRY(dalloc(&w.scan_scratch, scan_scratch_elems((int)nbins + 1)));
+    FSD_TRY(dalloc(&w.scan_scratch, scan_scratch_elems((int)w.ncell_cap + 1)));
     FSD_TRY(dalloc(&w.part_cell, N));
     FSD_TRY(dalloc(&w.cell_count, w.ncell_cap + 1));
     FSD_TRY(dalloc(&w.cell_start, w.ncell_cap + 1));
@@ -80,12 +79,18 @@ static int allocate(fsd_handle* h) {
     FSD_TRY(dalloc(&w.order, N));
     FSD_TRY(dalloc(&w.lub_n, N));
     FSD_TRY(init_particle_order(h));
-    FSD_TRY(dalloc(&w.part_origin_key, N));
-    FSD_TRY(dalloc(&w.part_origin, 3 * (size_t)N));
-    FSD_TRY(dalloc(&w.bin_count, G + 1));
+    const size_t ncol = (size_t)h->g.Nx * h->g.Ny;
+    FSD_TRY(dalloc(&w.bin_key, 2 * (size_t)N));
+    FSD_TRY(dalloc(&w.bin_items, N));
+    FSD_TRY(dalloc(&w.col_count, ncol));
+    FSD_TRY(dalloc(&w.col_start, ncol + 1));
+    FSD_TRY(dalloc(&w.bin_ticket, 1));
+    FSD_CHECK_CUDA(cudaMemsetAsync(w.col_count, 0, sizeof(unsigned) * ncol, h->stream));
+    FSD_CHECK_CUDA(cudaMemsetAsync(w.bin_ticket, 0, sizeof(unsigned), h->stream));
     FSD_TRY(dalloc(&w.bin_start, G + 1));
-    FSD_TRY(dalloc(&w.bin_fill, G + 1));
     FSD_TRY(dalloc(&w.bin_parts, N));
+    FSD_TRY(dalloc(&w.bin_pos, N));
+    FSD_TRY(dalloc(&w.bin_force, 3 * (size_t)N));
     FSD_TRY(dalloc(&w.grid, 6 * G));
     FSD_TRY(dalloc(&w.gridk, G));
     FSD_TRY(dalloc(&w.twiddle, (size_t)h->g.Nx + h->g.Ny + h->g.Nz));
@@ -142,8 +147,8 @@ static int allocate(fsd_handle* h) {
 static void release(fsd_handle* h) {
     Workspace& w = h->w;
     void* dev[] = {w.nneigh, w.nlist, w.nl_overflow, w.scan_scratch, w.part_cell, w.cell_count, w.cell_start,
-                   w.cell_fill, w.cell_parts, w.order, w.lub_n, w.lub_list, w.part_origin_key, w.part_origin, w.bin_count, w.bin_start, w.bin_fill,
-                   w.bin_parts, w.grid, w.gridk, w.twiddle, w.spec, w.green_table, w.f4, w.c4, w.uwave, w.sx, w.sy, w.sz, w.V, w.Z, w.dred,
+                   w.cell_fill, w.cell_parts, w.order, w.lub_n, w.lub_list, w.bin_key, w.bin_items, w.col_count,
+                   w.col_start, w.bin_ticket, w.bin_start, w.bin_parts, w.bin_pos, w.bin_force, w.grid, w.gridk, w.twiddle, w.spec, w.green_table, w.f4, w.c4, w.uwave, w.sx, w.sy, w.sz, w.V, w.Z, w.dred,
                    w.hcol, w.hcol2, w.ticket, w.gmres_state, w.pc_t, w.pc_y, w.rhs, w.sol, w.rfd_rhs, w.rfd_sol, w.psi,
                    w.pos_prime, w.vel, w.force, w.lanczos_V, w.lz_a, w.lz_b, w.lz_c, w.lz_dot, h->d_ewald,
                    h->d_res_dist, h->d_res_vals, w.rk_pos, w.rk_posw, w.rk_ori, w.rk_vel, w.rk_u1, w.rk_noise};

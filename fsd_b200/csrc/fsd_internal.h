@@ -86,12 +86,15 @@ struct Workspace {
     unsigned* lub_n = nullptr;
     unsigned* lub_list = nullptr;
     // particles binned by spreading-stencil origin (one bin per grid node)
-    unsigned* part_origin_key = nullptr;
-    int* part_origin = nullptr;
-    unsigned* bin_count = nullptr;
-    unsigned* bin_start = nullptr;
-    unsigned* bin_fill = nullptr;
-    unsigned* bin_parts = nullptr;
+    uint2* bin_key = nullptr;      // (column, slot) and (z, -) of each particle's stencil origin
+    uint2* bin_items = nullptr;    // (z, particle) by column, unsorted within it
+    unsigned* col_count = nullptr; // per (x, y) column, zero between calls
+    unsigned* col_start = nullptr;
+    unsigned* bin_ticket = nullptr;
+    unsigned* bin_start = nullptr; // first member of each node's bin
+    unsigned* bin_parts = nullptr; // particles by bin, index order within a bin
+    float4* bin_pos = nullptr;     // their positions in that order, w = origin's z (bits)
+    float4* bin_force = nullptr;   // their force and couplet in that order, 3 float4 each
     // wave space
     float2* grid = nullptr;        // 6 packed complex grids of G points
     float4* gridk = nullptr;       // wave vector and Green's scale per grid point
