@@ -1512,7 +1512,7 @@ static void spread(fsd_handle* h) {
         // tile-relative and the tiles, four warps each, fill the chip four
         // times over (with fewer warps in flight each tile's serial walk over
         // its particles shows: 34 us against 17.8 with one node per lane at
-        // N = 8000, phi = 0.2; 47 against 52 at N = 32768, 72^3).  Else one node per
+        // N = 8000, phi = 0.45; 47 against 52 at N = 32768, 72^3).  Else one node per
         // lane on smaller tiles, which stage each particle more often but are
         // more, and keep separations tile-relative in a smaller box.
         const int shapes[4][5] = {{8, 8, 8, 4, 4 * 148}, {4, 8, 8, 1, 2 * 148}, {4, 4, 8, 1, 2 * 148}, {4, 4, 4, 1, 0}};

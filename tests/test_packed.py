@@ -1,0 +1,58 @@
+"""Clusters of close-packed spheres at the sizes where rows, sets and groups of lanes begin and end, against
+the FP64 oracle."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+import torch
+
+from conftest import ewald_golden
+from fsd_b200.core import FSD
+from oracle import fsd_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+EDGE = 40.0
+L = (EDGE, EDGE, EDGE)
+
+
+def packed(N, spacing, seed, jitter=0.004):
+    """The N sites of a face-centred cubic lattice nearest the box corner, jittered and wrapped."""
+    k = np.arange(-9, 10)
+    g = np.array(np.meshgrid(k, k, k)).reshape(3, -1).T
+    g = g[g.sum(1) % 2 == 0] * (spacing / np.sqrt(2.0))
+    rng = np.random.default_rng(seed)
+    x = g[np.argsort((g ** 2).sum(1), kind="stable")[:N]]
+    x = x + jitter * (2.0 * rng.random(x.shape) - 1.0) + EDGE / 2
+    pos = np.zeros((N, 4), np.float32)
+    pos[rng.permutation(N), :3] = x - EDGE * np.floor(x / EDGE + 0.5)
+    return pos
+
+
+def dev(x):
+    return torch.as_tensor(np.ascontiguousarray(x, np.float32)).cuda().view(-1)
+
+
+def rel(a, b):
+    a, b = np.asarray(a, np.float64), np.asarray(b, np.float64)
+    return float(np.linalg.norm(a - b) / max(np.linalg.norm(b), 1e-300))
+
+
+def solver(pos, xy=0.0, **kw):
+    s = FSD(len(pos), (*L, xy), **kw)
+    p = dev(pos)
+    s.build_neighbor_list(p)
+    return s, p
+
+
+@pytest.mark.parametrize("N", [1, 2, 3, 13, 20, 40, 151])
+def test_approximate_inverse_of_every_set_size(cuda, N):
+    """Sets from one member to the cap of 32.  FP64 normal equations, blocks stored in FP32: 1e-7 expected."""
+    pos = packed(N, 2.03, N)
+    s, p = solver(pos, precond="learned", learned_inner=0)
+    s.precond_build(p)
+    A = O.pruned_rfu_sparse(pos, L, 0.0, *O.resistance_table()).tocsr()
+    G = O.spai2(A, N)
+    b = np.random.default_rng(N).standard_normal(17 * N)
+    assert rel(s.precond_apply(dev(b)).cpu().numpy(), O.saddle_precond(b, G, N)) < 1e-5
+    s.close()
