@@ -415,8 +415,8 @@ int brownian_farfield(fsd_handle* h, const float4* pos, uint32_t step, float* ou
                                                                  h->seed_hashed, step, kStreamFFWave);
     const int e = mobility_wave_from_spectrum(h, pos);
     if (e != FSD_OK) return e;
-    // Combine into generalized layout (wave part only): needs f4/c4 unused.
-    mobility_combine(h, pos, nullptr, w.lz_c, true, false, nullptr);
+    // Combine into generalized layout (wave part only).
+    mobility_combine(h, w.lz_c, true, false, nullptr);
     }
     // Real space: Lanczos square root of M_real on an 11N normal vector.
     float* psi = w.lz_a;

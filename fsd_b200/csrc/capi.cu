@@ -98,8 +98,8 @@ static int allocate(fsd_handle* h) {
         FSD_TRY(dalloc(&w.spec, wave_spec_elems(h->g)));
         FSD_TRY(dalloc(&w.green_table, wave_table_elems(h->g)));
     }
-    FSD_TRY(dalloc(&w.f4, N));
-    FSD_TRY(dalloc(&w.c4, 2 * (size_t)N));
+    FSD_TRY(dalloc(&w.rec, 16 * (size_t)N));
+    FSD_TRY(dalloc(&w.u8, 8 * (size_t)N));
     FSD_TRY(dalloc(&w.uwave, 11 * (size_t)N));
     const size_t n17 = 17 * (size_t)N;
     FSD_TRY(dalloc(&w.sx, n17));
@@ -148,10 +148,10 @@ static void release(fsd_handle* h) {
     Workspace& w = h->w;
     void* dev[] = {w.nneigh, w.nlist, w.nl_overflow, w.scan_scratch, w.part_cell, w.cell_count, w.cell_start,
                    w.cell_fill, w.cell_parts, w.order, w.lub_n, w.lub_list, w.bin_key, w.bin_items, w.col_count,
-                   w.col_start, w.bin_ticket, w.bin_start, w.bin_parts, w.bin_pos, w.bin_force, w.grid, w.gridk, w.twiddle, w.spec, w.green_table, w.f4, w.c4, w.uwave, w.sx, w.sy, w.sz, w.V, w.Z, w.dred,
+                   w.col_start, w.bin_ticket, w.bin_start, w.bin_parts, w.bin_pos, w.bin_force, w.grid, w.gridk, w.twiddle, w.spec, w.green_table, w.rec, w.u8, w.uwave, w.sx, w.sy, w.sz, w.V, w.Z, w.dred,
                    w.hcol, w.hcol2, w.ticket, w.gmres_state, w.pc_t, w.pc_y, w.rhs, w.sol, w.rfd_rhs, w.rfd_sol, w.psi,
                    w.pos_prime, w.vel, w.force, w.lanczos_V, w.lz_a, w.lz_b, w.lz_c, w.lz_dot, h->d_ewald,
-                   h->d_res_dist, h->d_res_vals, w.rk_pos, w.rk_posw, w.rk_ori, w.rk_vel, w.rk_u1, w.rk_noise};
+                   h->d_res_dist, h->d_res_vals, h->d_res_rfu, h->d_res_g, h->d_res_m, w.rk_pos, w.rk_posw, w.rk_ori, w.rk_vel, w.rk_u1, w.rk_noise};
     for (void* p : dev)
         if (p) cudaFree(p);
     if (w.host_flag) cudaFreeHost(w.host_flag);
@@ -334,7 +334,10 @@ int fsd_create(const fsd_params* p, void* stream, fsd_handle** out) {
     if (st == FSD_OK) {
         const size_t tb = h->ewald_host.size() * sizeof(float);
         if (cudaMalloc(&h->d_ewald, tb) != cudaSuccess || cudaMalloc(&h->d_res_dist, sizeof(float) * kResRows) ||
-            cudaMalloc(&h->d_res_vals, sizeof(float) * kResRows * kResFuncs)) {
+            cudaMalloc(&h->d_res_vals, sizeof(float) * kResRows * kResFuncs) ||
+            cudaMalloc(&h->d_res_rfu, sizeof(float) * kResRows * 16) ||
+            cudaMalloc(&h->d_res_g, sizeof(float) * kResRows * 8) ||
+            cudaMalloc(&h->d_res_m, sizeof(float) * kResRows * 8)) {
             st = FSD_ERR_ALLOC;
         } else {
             cudaMemcpyAsync(h->d_ewald, h->ewald_host.data(), tb, cudaMemcpyHostToDevice, h->stream);
@@ -343,6 +346,20 @@ int fsd_create(const fsd_params* p, void* stream, fsd_handle** out) {
             cudaMemcpyAsync(h->d_res_dist, tdist.data(), sizeof(float) * kResRows, cudaMemcpyHostToDevice, h->stream);
             cudaMemcpyAsync(h->d_res_vals, tvals.data(), sizeof(float) * kResRows * kResFuncs, cudaMemcpyHostToDevice,
                             h->stream);
+            // the same functions in the rows the lubrication kernels read
+            std::vector<float> rows[3];
+            const int first[3] = {0, 10, 16}, count[3] = {10, 6, 6}, rs[3] = {16, 8, 8};
+            float* const dst[3] = {h->d_res_rfu, h->d_res_g, h->d_res_m};
+            for (int t = 0; t < 3; ++t) {
+                rows[t].assign((size_t)kResRows * rs[t], 0.f);
+                for (int i = 0; i < kResRows; ++i) {
+                    float* o = rows[t].data() + (size_t)i * rs[t];
+                    for (int c = 0; c < count[t]; ++c) o[c] = tvals[(size_t)i * kResFuncs + first[t] + c];
+                    o[count[t]] = tdist[i];
+                }
+                cudaMemcpyAsync(dst[t], rows[t].data(), sizeof(float) * rows[t].size(), cudaMemcpyHostToDevice,
+                                h->stream);
+            }
             fill_twiddles(h);
             mobility_set_gridk(h);
             if (cudaStreamSynchronize(h->stream) != cudaSuccess) st = FSD_ERR_CUDA;

@@ -57,6 +57,15 @@ __device__ __forceinline__ void wrap_position(float3& w, int3& img, const Box& b
     else if (w.z < -b.Lz / 2) { w.z += b.Lz; img.z--; }
 }
 
+// 32 bytes in one load (32-byte aligned, read-only for the kernel).  A gather
+// costs the L1 one tag lookup per lane and instruction, so records of 32 bytes
+// take half the lookups of two float4.
+__device__ __forceinline__ void load8(const float* p, float* v) {
+    asm volatile("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+                 : "l"(p));
+}
+
 // Interpolated near-field resistance scalars [first, first+count) of the table
 // row bracketing distance r.  Pairs at r <= 2.001 use the regularised row 232
 // (Lubrication.cu:172-186).  Beyond the last tabulated gap the index reaches

@@ -102,8 +102,8 @@ struct Workspace {
     float2* spec = nullptr;        // half spectra of the 11 real grids (specialised transforms only)
     float4* green_table = nullptr; // wave vector and Green factors per half-spectrum point, 2 float4 each
     // particle work arrays
-    float4* f4 = nullptr;          // force per particle
-    float4* c4 = nullptr;          // couplet, two float4 per particle
+    float* rec = nullptr;          // position, force and couplet, 16 floats per particle
+    float* u8 = nullptr;           // U and W of a saddle vector, 8 floats per particle
     float* uwave = nullptr;        // 11 per particle: wave-space u and velocity gradient
     // Krylov
     float* sx = nullptr;           // 17N work vectors
@@ -196,6 +196,9 @@ struct fsd_handle {
     float4* d_ewald = nullptr;
     float* d_res_dist = nullptr;
     float* d_res_vals = nullptr;
+    float* d_res_rfu = nullptr;  // functions 0-9 and distance, rows of 16
+    float* d_res_g = nullptr;    // functions 10-15 and distance, rows of 8
+    float* d_res_m = nullptr;    // functions 16-21 and distance, rows of 8
     fsd::Workspace w;
     fsd_solve_info info{};
     bool nlist_valid = false;

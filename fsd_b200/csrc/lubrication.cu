@@ -4,8 +4,16 @@
 // are needed; a group of 8 lanes splits a particle's neighbours and reduces
 // with shuffles.  The list is the neighbour list cut at rlub plus the list
 // buffer (same order, so the same sums), and particles are visited in cell
-// order so that a block's gathers overlap.  The resistance scalars are interpolated from the tabulated
-// Jeffrey-Onishi functions exactly as the reference does (res_interp).
+// order so that a block's gathers overlap.  The resistance scalars are
+// interpolated from the tabulated Jeffrey-Onishi functions as the reference
+// does.
+//
+// Bound by the L1 tag rate (one lookup per lane and gather): the table's rows
+// read value by value (20 loads for R_FU) and U component by component made 30
+// gathers per pair, 38 us per R_FU product at N = 32768, phi = 0.4 (30 to 55 us
+// for the others).  Each product's functions now sit in rows of 8 or 16 floats
+// with the row's distance, read in 32-byte loads, and a saddle product takes U
+// from packed records of 8: 27 us per R_FU product.
 #include "fsd_device.cuh"
 #include "fsd_kernels.cuh"
 #include "fsd_profile.h"
@@ -20,11 +28,66 @@ struct LubArgs {
     const unsigned* nneigh;
     const unsigned* nlist;
     int stride;
-    ResTable tab;
+    const float* tab;       // the product's function rows (kResRows of 8 or 16 floats)
     Box box;
     int N;
     float rlub2;
 };
+
+// The COUNT interpolated functions of a table of rows of RS floats (functions
+// first, the row's distance in slot COUNT) at distance r; false past the last
+// row, where they are zero.  Pairs at r <= 2.001 use the regularised row 232
+// (Lubrication.cu:172-186).
+template <int COUNT, int RS>
+__device__ __forceinline__ bool lub_interp(const float* __restrict__ tab, float r, float* out) {
+    constexpr int L = COUNT + 1 <= 8 ? 8 : 12;
+    const bool near = (double)r <= 2.001;
+    int ind = 232;
+    if (!near) {
+        const float s = (float)(((double)r - 2.0) * (1.0 / (double)kResMin));
+        ind = (int)(log10f(s) / kResDr);
+    }
+    if (ind >= kResRows - 1) return false;
+    float lo[L], hi[L];
+    const float* p = tab + (size_t)ind * RS;
+    load8(p, lo);
+    load8(p + RS, hi);
+    if constexpr (L > 8) {
+        const float4 a = __ldg(reinterpret_cast<const float4*>(p + 8)), b = __ldg(reinterpret_cast<const float4*>(p + RS + 8));
+        lo[8] = a.x;
+        lo[9] = a.y;
+        lo[10] = a.z;
+        hi[8] = b.x;
+        hi[9] = b.y;
+        hi[10] = b.z;
+    }
+    const float fac = near ? 0.f : (r - lo[COUNT]) / (hi[COUNT] - lo[COUNT]);
+#pragma unroll
+    for (int c = 0; c < COUNT; ++c) out[c] = lo[c] + (hi[c] - lo[c]) * fac;
+    return true;
+}
+
+// U and W of particle j: PACKED from records of 8, else from the 6N vector.
+template <bool PACKED>
+__device__ __forceinline__ void load_uw(const float* __restrict__ U, unsigned j, float3& u, float3& w) {
+    if constexpr (PACKED) {
+        float v[8];
+        load8(U + 8 * (size_t)j, v);
+        u = make_float3(v[0], v[1], v[2]);
+        w = make_float3(v[3], v[4], v[5]);
+    } else {
+        const float* p = U + 6 * (size_t)j;
+        if ((reinterpret_cast<uintptr_t>(U) & 7) == 0) {  // 6-vectors start on 8 bytes
+            const float2* q = reinterpret_cast<const float2*>(p);
+            const float2 a = __ldg(q), b = __ldg(q + 1), c = __ldg(q + 2);
+            u = make_float3(a.x, a.y, b.x);
+            w = make_float3(b.y, c.x, c.y);
+        } else {
+            u = make_float3(p[0], p[1], p[2]);
+            w = make_float3(p[3], p[4], p[5]);
+        }
+    }
+}
 
 // Imposed + active rate of strain of one particle as a symmetric 3x3
 // (Lubrication.cu:380-410): E = (xx-zz, 2xy, 2xz, 2yz, yy-zz) -> tensor.
@@ -57,6 +120,7 @@ __device__ __forceinline__ float3 eps_dot(float3 r, float3 v) {
 
 // F = R_FU U (Lubrication_RFU_kernel, Lubrication.cu:69-309).  With saddle_x,
 // writes saddle_x[6i + c] - F instead (Saddle.cu:141-148).
+template <bool PACKED>
 __global__ void __launch_bounds__(128) k_rfu(LubArgs a, const float* __restrict__ U, float* __restrict__ out,
                                              const float* __restrict__ saddle_x) {
     const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / kLubGroup;
@@ -64,8 +128,8 @@ __global__ void __launch_bounds__(128) k_rfu(LubArgs a, const float* __restrict_
     const bool valid = gid < a.N;
     const int i = (int)a.order[valid ? gid : a.N - 1];
     const float4 pi = a.pos[i];
-    const float3 ui = make_float3(U[6 * i], U[6 * i + 1], U[6 * i + 2]);
-    const float3 wi = make_float3(U[6 * i + 3], U[6 * i + 4], U[6 * i + 5]);
+    float3 ui, wi;
+    load_uw<PACKED>(U, i, ui, wi);
     float f[6] = {0, 0, 0, 0, 0, 0};
     const unsigned nn = valid ? a.nneigh[i] : 0u;
     const unsigned* row = a.nlist + (size_t)i * a.stride;
@@ -77,11 +141,11 @@ __global__ void __launch_bounds__(128) k_rfu(LubArgs a, const float* __restrict_
         if (!(d2 < a.rlub2 && d2 > 0.f)) continue;
         const float dist = sqrtf(d2);
         float c[10];
-        res_interp<10>(a.tab, dist, 0, c);
+        if (!lub_interp<10, 16>(a.tab, dist, c)) continue;
         const float XA11 = c[0], XA12 = c[1], YA11 = c[2], YA12 = c[3], YB11 = c[4], YB12 = c[5];
         const float XC11 = c[6], XC12 = c[7], YC11 = c[8], YC12 = c[9];
-        const float3 uj = make_float3(U[6 * j], U[6 * j + 1], U[6 * j + 2]);
-        const float3 wj = make_float3(U[6 * j + 3], U[6 * j + 4], U[6 * j + 5]);
+        float3 uj, wj;
+        load_uw<PACKED>(U, j, uj, wj);
         const float3 r = make_float3(R.x / dist, R.y / dist, R.z / dist);
         const float rdui = r.x * ui.x + r.y * ui.y + r.z * ui.z;
         const float rduj = r.x * uj.x + r.y * uj.y + r.z * uj.z;
@@ -135,7 +199,7 @@ __global__ void __launch_bounds__(128) k_rfe(LubArgs a, float shear_rate, const 
         if (!(d2 < a.rlub2)) continue;
         const float dist = sqrtf(d2);
         float c[6];
-        res_interp<6>(a.tab, dist, 10, c);
+        if (!lub_interp<6, 8>(a.tab, dist, c)) continue;
         const float XG11 = c[0], XG12 = c[1], YG11 = c[2], YG12 = c[3], YH11 = c[4], YH12 = c[5];
         strain_block(shear_rate, ori, b2mask, B2, j, Ej);
         const float3 r = make_float3(R.x / dist, R.y / dist, R.z / dist);
@@ -167,8 +231,8 @@ __global__ void __launch_bounds__(128) k_rfe(LubArgs a, float shear_rate, const 
 }
 
 // Components (xx, xy, xz, yz, yy) of the stresslet.
-__constant__ int kSa[5] = {0, 0, 0, 1, 1};
-__constant__ int kSb[5] = {0, 1, 2, 2, 1};
+__host__ __device__ constexpr int sa_of(int k) { return k < 3 ? 0 : 1; }
+__host__ __device__ constexpr int sb_of(int k) { return k < 3 ? k : 5 - k; }
 
 __device__ __forceinline__ float comp(float3 v, int k) { return k == 0 ? v.x : (k == 1 ? v.y : v.z); }
 
@@ -179,8 +243,8 @@ __global__ void __launch_bounds__(128) k_rsu(LubArgs a, const float* __restrict_
     const bool valid = gid < a.N;
     const int i = (int)a.order[valid ? gid : a.N - 1];
     const float4 pi = a.pos[i];
-    const float3 ui = make_float3(U[6 * i], U[6 * i + 1], U[6 * i + 2]);
-    const float3 wi = make_float3(U[6 * i + 3], U[6 * i + 4], U[6 * i + 5]);
+    float3 ui, wi;
+    load_uw<false>(U, i, ui, wi);
     float s[5] = {0, 0, 0, 0, 0};
     const unsigned nn = valid ? a.nneigh[i] : 0u;
     const unsigned* row = a.nlist + (size_t)i * a.stride;
@@ -192,17 +256,17 @@ __global__ void __launch_bounds__(128) k_rsu(LubArgs a, const float* __restrict_
         if (!(d2 < a.rlub2)) continue;
         const float dist = sqrtf(d2);
         float c[6];
-        res_interp<6>(a.tab, dist, 10, c);
+        if (!lub_interp<6, 8>(a.tab, dist, c)) continue;
         const float XG11 = c[0], XG12 = c[1], YG11 = c[2], YG12 = c[3], YH11 = c[4], YH12 = c[5];
-        const float3 uj = make_float3(U[6 * j], U[6 * j + 1], U[6 * j + 2]);
-        const float3 wj = make_float3(U[6 * j + 3], U[6 * j + 4], U[6 * j + 5]);
+        float3 uj, wj;
+        load_uw<false>(U, j, uj, wj);
         const float3 r = make_float3(R.x / dist, R.y / dist, R.z / dist);
         const float rdui = r.x * ui.x + r.y * ui.y + r.z * ui.z;
         const float rduj = r.x * uj.x + r.y * uj.y + r.z * uj.z;
         const float3 ewi = eps_dot(r, wi), ewj = eps_dot(r, wj);
 #pragma unroll
         for (int k = 0; k < 5; ++k) {
-            const int A = kSa[k], B = kSb[k];
+            const int A = sa_of(k), B = sb_of(k);
             const float ra = comp(r, A), rb = comp(r, B);
             const float P = ra * rb - (A == B ? 1.0f / 3.0f : 0.0f);
             s[k] += XG11 * P * rdui + XG12 * P * rduj + YG11 * (comp(ui, A) * rb + ra * comp(ui, B) - 2.0f * ra * rb * rdui) +
@@ -239,7 +303,7 @@ __global__ void __launch_bounds__(128) k_rse(LubArgs a, float shear_rate, const 
         if (!(d2 < 16.0f)) continue;
         const float dist = sqrtf(d2);
         float c[6];
-        res_interp<6>(a.tab, dist, 16, c);
+        if (!lub_interp<6, 8>(a.tab, dist, c)) continue;
         const float XM11 = c[0], XM12 = c[1], YM11 = c[2], YM12 = c[3], ZM11 = c[4], ZM12 = c[5];
         strain_block(shear_rate, ori, b2mask, B2, j, Ej);
         const float3 r = make_float3(R.x / dist, R.y / dist, R.z / dist);
@@ -253,7 +317,7 @@ __global__ void __launch_bounds__(128) k_rse(LubArgs a, float shear_rate, const 
         const float rdEdrj = r.x * Edrj.x + r.y * Edrj.y + r.z * Edrj.z;
 #pragma unroll
         for (int k = 0; k < 5; ++k) {
-            const int A = kSa[k], B = kSb[k];
+            const int A = sa_of(k), B = sb_of(k);
             const float ra = comp(r, A), rb = comp(r, B);
             const float dab = (A == B) ? 1.0f : 0.0f;
             const float P = ra * rb - dab / 3.0f;
@@ -273,15 +337,14 @@ __global__ void __launch_bounds__(128) k_rse(LubArgs a, float shear_rate, const 
     for (int c = 0; c < 5; ++c) S[5 * i + c] += s[c];
 }
 
-static LubArgs lub_args(fsd_handle* h, const float4* pos) {
+static LubArgs lub_args(fsd_handle* h, const float4* pos, const float* rows) {
     LubArgs a;
     a.pos = pos;
     a.order = h->w.order;
     a.nneigh = h->w.lub_n;
     a.nlist = h->w.lub_list;
     a.stride = h->w.nl_stride;
-    a.tab.dist = h->d_res_dist;
-    a.tab.vals = h->d_res_vals;
+    a.tab = rows;
     a.box = h->box;
     a.N = h->p.N;
     a.rlub2 = h->p.rlub * h->p.rlub;
@@ -293,24 +356,29 @@ static int lub_blocks(int N) { return (N * kLubGroup + 127) / 128; }
 void lub_rfu(fsd_handle* h, const float4* pos, const float* U, float* F, const float* saddle_x) {
     ProfRegion pr(h, R_RFU);
     count_launch();
-    k_rfu<<<lub_blocks(h->p.N), 128, 0, h->stream>>>(lub_args(h, pos), U, F, saddle_x);
+    k_rfu<false><<<lub_blocks(h->p.N), 128, 0, h->stream>>>(lub_args(h, pos, h->d_res_rfu), U, F, saddle_x);
+}
+void lub_rfu_packed(fsd_handle* h, const float4* pos, float* F, const float* saddle_x) {
+    ProfRegion pr(h, R_RFU);
+    count_launch();
+    k_rfu<true><<<lub_blocks(h->p.N), 128, 0, h->stream>>>(lub_args(h, pos, h->d_res_rfu), h->w.u8, F, saddle_x);
 }
 void lub_rfe(fsd_handle* h, const float4* pos, float shear_rate, const float3* ori, const float* b2mask, float B2,
              float* F) {
     ProfRegion pr(h, R_LUB_OTHER);
     count_launch();
-    k_rfe<<<lub_blocks(h->p.N), 128, 0, h->stream>>>(lub_args(h, pos), shear_rate, ori, b2mask, B2, F);
+    k_rfe<<<lub_blocks(h->p.N), 128, 0, h->stream>>>(lub_args(h, pos, h->d_res_g), shear_rate, ori, b2mask, B2, F);
 }
 void lub_rsu(fsd_handle* h, const float4* pos, const float* U, float* S) {
     ProfRegion pr(h, R_LUB_OTHER);
     count_launch();
-    k_rsu<<<lub_blocks(h->p.N), 128, 0, h->stream>>>(lub_args(h, pos), U, S);
+    k_rsu<<<lub_blocks(h->p.N), 128, 0, h->stream>>>(lub_args(h, pos, h->d_res_g), U, S);
 }
 void lub_rse(fsd_handle* h, const float4* pos, float shear_rate, const float3* ori, const float* b2mask, float B2,
              float* S) {
     ProfRegion pr(h, R_LUB_OTHER);
     count_launch();
-    k_rse<<<lub_blocks(h->p.N), 128, 0, h->stream>>>(lub_args(h, pos), shear_rate, ori, b2mask, B2, S);
+    k_rse<<<lub_blocks(h->p.N), 128, 0, h->stream>>>(lub_args(h, pos, h->d_res_m), shear_rate, ori, b2mask, B2, S);
 }
 
 }  // namespace fsd

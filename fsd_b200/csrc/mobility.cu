@@ -526,11 +526,15 @@ static void fft_x_green(fsd_handle* h) {
 // Split the generalized force and map torque + stresslet to the couplet
 // (Saddle_SplitGeneralizedF_kernel, Helper_Saddle.cu:108; Mobility_TS2C_kernel,
 // Helper_Mobility.cu:294-336, including its torque sign flip).
-// With `parts` (particles in bin order) a second copy in that order is written
-// as the spreading kernel's packed pairs:
-// (Fx,Fy,Cxx,Cxy) (Cxz,Cyx,Cyy,Cyz) (Czx,Czy,Fz,0).
-__global__ void k_prep(const float* __restrict__ genF, int N, float4* f4, float4* c4,
-                       const unsigned* __restrict__ parts, float4* __restrict__ sorted) {
+// Per particle, as the kernels that gather them want them:
+//   rec     16 floats (with `real`): position, force, couplet
+//           (x y z Fx Fy Fz Cxx Cxy | Cxz Cyz Cyy Cyx Czx Czy - -);
+//   sorted  12 floats in bin order (with `parts`): the spreading kernel's pairs
+//           (Fx,Fy,Cxx,Cxy) (Cxz,Cyx,Cyy,Cyz) (Czx,Czy,Fz,0);
+//   u8      8 floats (with `saddle_x`): the saddle vector's U and W.
+__global__ void k_prep(const float* __restrict__ genF, const float4* __restrict__ pos, int N, float* __restrict__ rec,
+                       const unsigned* __restrict__ parts, float4* __restrict__ sorted,
+                       const float* __restrict__ saddle_x, float* __restrict__ u8) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= N) return;
     const int i = parts ? (int)parts[q] : q;
@@ -541,9 +545,20 @@ __global__ void k_prep(const float* __restrict__ genF, int N, float4* f4, float4
     const float Sxx = s[0], Sxy = s[1], Sxz = s[2], Syz = s[3], Syy = s[4];
     const float4 c0 = make_float4(Sxx, Sxy + 0.5f * Lz, Sxz - 0.5f * Ly, Syz + 0.5f * Lx);
     const float4 c1 = make_float4(Syy, Sxy - 0.5f * Lz, Sxz + 0.5f * Ly, Syz - 0.5f * Lx);
-    f4[i] = make_float4(fx, fy, fz, 0.0f);
-    c4[2 * i] = c0;
-    c4[2 * i + 1] = c1;
+    if (rec) {
+        const float4 p = pos[i];
+        float4* o = reinterpret_cast<float4*>(rec + 16 * (size_t)i);
+        o[0] = make_float4(p.x, p.y, p.z, fx);
+        o[1] = make_float4(fy, fz, c0.x, c0.y);
+        o[2] = make_float4(c0.z, c0.w, c1.x, c1.y);
+        o[3] = make_float4(c1.z, c1.w, 0.f, 0.f);
+    }
+    if (saddle_x) {
+        const float* u = saddle_x + 11 * (size_t)N + 6 * (size_t)i;
+        float4* o = reinterpret_cast<float4*>(u8 + 8 * (size_t)i);
+        o[0] = make_float4(u[0], u[1], u[2], u[3]);
+        o[1] = make_float4(u[4], u[5], 0.f, 0.f);
+    }
     if (!parts) return;
     sorted[3 * q] = make_float4(fx, fy, c0.x, c0.y);
     sorted[3 * q + 1] = make_float4(c0.z, c1.y, c1.x, c0.w);
@@ -1307,23 +1322,26 @@ __global__ void __launch_bounds__(256) k_contract(const float4* __restrict__ pos
 }
 
 // ------------------------------------------- real space, self and combine
-// Group of 8 lanes per particle: real-space Ewald pair sum with linear table
+// Group of GROUP lanes per particle: real-space Ewald pair sum with linear table
 // interpolation (Mobility_RealSpace_kernel, Mobility.cu:1046-1226), the self
 // term, the optional wave-space part, then velocity gradient -> (W, E)
 // (Mobility_D2WE_kernel) and generalized packing
 // (Saddle_MakeGeneralizedU_kernel).
+//
+// Bound by the L1 tag rate: every gather instruction takes one lookup per
+// lane.  Position, force and couplet in three arrays and the table's two rows
+// as float4 were eight gathers per pair, 53 us per call at N = 32768,
+// phi = 0.4; packed records and rows in 32-byte loads are four, 43 us.
 struct RealArgs {
-    const float4* pos;
+    const float* rec;       // 16 floats per particle (k_prep)
     const unsigned* order;  // particles in cell order
-    const float4* f4;
-    const float4* c4;
     const float* uwave;     // may be null
     const unsigned* nneigh;
     const unsigned* nlist;
     int stride;
-    const float4* table;
+    const float* table;     // 8 floats per row
     float self_x, self_y;
-    float ewald_cut, ewald_dr;
+    float ewald_cut, ewald_dr, inv_dr, row_scale;
     int ewald_n;
     Box box;
     int N;
@@ -1332,43 +1350,56 @@ struct RealArgs {
     float* genU;
 };
 
-constexpr int kRealGroup = 8;
+constexpr size_t kRealWarpThreads = 148 * 896;  // seven blocks of 128 per SM
 
+template <int GROUP>
 __global__ void __launch_bounds__(128) k_real_combine(RealArgs a) {
-    const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / kRealGroup;
-    const int gl = threadIdx.x % kRealGroup;
+    const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / GROUP;
+    const int gl = threadIdx.x % GROUP;
     const int N = a.N;
     const bool valid = gid < N;
     const int i = (int)a.order[valid ? gid : N - 1];
     float u[3] = {0, 0, 0}, D[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     if (a.real) {
-        const float4 pi = a.pos[i];
+        const float4 pi = *reinterpret_cast<const float4*>(a.rec + 16 * (size_t)i);
         const float mindistSq = a.ewald_dr * a.ewald_dr, maxdistSq = a.ewald_cut * a.ewald_cut;
         const unsigned nn = valid ? a.nneigh[i] : 0u;
         const unsigned* row = a.nlist + (size_t)i * a.stride;
-        for (unsigned q = gl; q < nn; q += kRealGroup) {
-            const unsigned j = row[q];
-            const float4 pj = a.pos[j];
-            const float3 r = min_image(make_float3(pi.x - pj.x, pi.y - pj.y, pi.z - pj.z), a.box);
+        // the next neighbour's index and first half record are loaded a step ahead
+        unsigned j = gl < nn ? row[gl] : (unsigned)i, jn;
+        float pn[8];
+        load8(a.rec + 16 * (size_t)j, pn);
+        jn = gl + GROUP < nn ? row[gl + GROUP] : (unsigned)i;
+        for (unsigned q = gl; q < nn; q += GROUP) {
+            float p0[8], p1[8];
+#pragma unroll
+            for (int c = 0; c < 8; ++c) p0[c] = pn[c];
+            const unsigned jc = j;
+            j = jn;
+            load8(a.rec + 16 * (size_t)j, pn);
+            jn = q + 2 * GROUP < nn ? row[q + 2 * GROUP] : (unsigned)i;
+            const float3 r = min_image(make_float3(pi.x - p0[0], pi.y - p0[1], pi.z - p0[2]), a.box);
             const float distSqr = r.x * r.x + r.y * r.y + r.z * r.z;
             if (!(distSqr < maxdistSq && distSqr >= mindistSq)) continue;
+            load8(a.rec + 16 * (size_t)jc + 8, p1);
             const float dist = sqrtf(distSqr);
-            const float4 Fj = a.f4[j];
-            const float4 C0 = a.c4[2 * j], C1 = a.c4[2 * j + 1];
+            const float3 Fj = make_float3(p0[3], p0[4], p0[5]);
+            const float4 C0 = make_float4(p0[6], p0[7], p1[0], p1[1]), C1 = make_float4(p1[2], p1[3], p1[4], p1[5]);
             // Clamped so that a distance rounding up to the cutoff stays inside the table.
-            const int r_ind = min(max(__float2int_rd(a.ewald_n * (dist - a.ewald_dr) / (a.ewald_cut - a.ewald_dr)), 0),
-                                  a.ewald_n - 1);
-            const float4 t1m = __ldg(a.table + 2 * r_ind), t2m = __ldg(a.table + 2 * r_ind + 1);
-            const float4 t1p = __ldg(a.table + 2 * r_ind + 2), t2p = __ldg(a.table + 2 * r_ind + 3);
-            const float fac = dist / a.ewald_dr - r_ind - 1.0f;
-            const float f1 = t1m.x + (t1p.x - t1m.x) * fac;
-            const float f2 = t1m.y + (t1p.y - t1m.y) * fac;
-            const float g1 = -(t1m.z + (t1p.z - t1m.z) * fac);
-            const float g2 = -(t1m.w + (t1p.w - t1m.w) * fac);
-            const float h1 = t2m.x + (t2p.x - t2m.x) * fac;
-            const float h2 = t2m.y + (t2p.y - t2m.y) * fac;
-            const float h3 = t2m.z + (t2p.z - t2m.z) * fac;
-            const float Rx = r.x / dist, Ry = r.y / dist, Rz = r.z / dist;
+            const int r_ind = min(max(__float2int_rd(a.row_scale * (dist - a.ewald_dr)), 0), a.ewald_n - 1);
+            float lo[8], hi[8];
+            load8(a.table + 8 * (size_t)r_ind, lo);
+            load8(a.table + 8 * (size_t)r_ind + 8, hi);
+            const float fac = fmaf(-(float)(r_ind + 1), a.ewald_dr, dist) * a.inv_dr;
+            const float f1 = lo[0] + (hi[0] - lo[0]) * fac;
+            const float f2 = lo[1] + (hi[1] - lo[1]) * fac;
+            const float g1 = -(lo[2] + (hi[2] - lo[2]) * fac);
+            const float g2 = -(lo[3] + (hi[3] - lo[3]) * fac);
+            const float h1 = lo[4] + (hi[4] - lo[4]) * fac;
+            const float h2 = lo[5] + (hi[5] - lo[5]) * fac;
+            const float h3 = lo[6] + (hi[6] - lo[6]) * fac;
+            const float idist = 1.0f / dist;
+            const float Rx = r.x * idist, Ry = r.y * idist, Rz = r.z * idist;
             const float rdotf = Rx * Fj.x + Ry * Fj.y + Rz * Fj.z;
             const float Czz = -(C0.x + C1.x);
             // C.r and r.C with C = [[XX XY XZ][YX YY YZ][ZX ZY ZZ]] = [[c0x c0y c0z][c1y c1x c0w][c1z c1w Czz]]
@@ -1413,13 +1444,17 @@ __global__ void __launch_bounds__(128) k_real_combine(RealArgs a) {
                     h3 * (Cr_z * Ry + Rz * rC_y + rC_z * Ry - 6.f * rCr * Rz * Ry - C0.w);
         }
 #pragma unroll
-        for (int c = 0; c < 3; ++c) u[c] = group_sum<kRealGroup>(u[c]);
+        for (int c = 0; c < 3; ++c) u[c] = group_sum<GROUP>(u[c]);
 #pragma unroll
-        for (int c = 0; c < 8; ++c) D[c] = group_sum<kRealGroup>(D[c]);
+        for (int c = 0; c < 8; ++c) D[c] = group_sum<GROUP>(D[c]);
     }
     if (!valid || gl != 0) return;
     if (a.real) {
-        const float4 F = a.f4[i], C0 = a.c4[2 * i], C1 = a.c4[2 * i + 1];
+        float p0[8], p1[8];
+        load8(a.rec + 16 * (size_t)i, p0);
+        load8(a.rec + 16 * (size_t)i + 8, p1);
+        const float3 F = make_float3(p0[3], p0[4], p0[5]);
+        const float4 C0 = make_float4(p0[6], p0[7], p1[0], p1[1]), C1 = make_float4(p1[2], p1[3], p1[4], p1[5]);
         u[0] += a.self_x * F.x;
         u[1] += a.self_x * F.y;
         u[2] += a.self_x * F.z;
@@ -1591,23 +1626,22 @@ int mobility_wave_from_spectrum(fsd_handle* h, const float4* pos) {
     return FSD_OK;
 }
 
-void mobility_combine(fsd_handle* h, const float4* pos, const float* genF, float* genU, bool wave, bool real,
+void mobility_combine(fsd_handle* h, float* genU, bool wave, bool real,
                       const float* saddle_x) {
-    (void)genF;
     RealArgs r;
-    r.pos = pos;
+    r.rec = h->w.rec;
     r.order = h->w.order;
-    r.f4 = h->w.f4;
-    r.c4 = h->w.c4;
     r.uwave = wave ? h->w.uwave : nullptr;
     r.nneigh = h->w.nneigh;
     r.nlist = h->w.nlist;
     r.stride = h->w.nl_stride;
-    r.table = h->d_ewald;
+    r.table = reinterpret_cast<const float*>(h->d_ewald);
     r.self_x = h->self_x;
     r.self_y = h->self_y;
     r.ewald_cut = h->ewald_cut;
     r.ewald_dr = h->ewald_dr;
+    r.inv_dr = 1.0f / h->ewald_dr;
+    r.row_scale = (float)((double)h->ewald_n / ((double)h->ewald_cut - (double)h->ewald_dr));
     r.ewald_n = h->ewald_n;
     r.box = h->box;
     r.N = h->p.N;
@@ -1616,7 +1650,13 @@ void mobility_combine(fsd_handle* h, const float4* pos, const float* genF, float
     r.genU = genU;
     const int N = h->p.N;
     count_launch();
-    k_real_combine<<<(N * kRealGroup + 127) / 128, 128, 0, h->stream>>>(r);
+    // Eight lanes per particle keep every lane busy on rows of 40 to 100
+    // neighbours; a small suspension does not fill the chip that way and is
+    // bound by the chain of gathers per lane, which a whole warp shortens.
+    if ((size_t)N * 32 <= kRealWarpThreads)
+        k_real_combine<32><<<(N + 3) / 4, 128, 0, h->stream>>>(r);
+    else
+        k_real_combine<8><<<(N + 15) / 16, 128, 0, h->stream>>>(r);
 }
 
 // ---------------------------------------------------------------- autotuner
@@ -1743,8 +1783,9 @@ int mobility_apply(fsd_handle* h, const float4* pos, const float* genF, float* g
         if (st != FSD_OK) return st;
     }
     count_launch();
-    k_prep<<<(N + 255) / 256, 256, 0, h->stream>>>(genF, N, h->w.f4, h->w.c4, wave ? h->w.bin_parts : nullptr,
-                                                   h->w.bin_force);
+    k_prep<<<(N + 255) / 256, 256, 0, h->stream>>>(genF, pos, N, real ? h->w.rec : nullptr,
+                                                   wave ? h->w.bin_parts : nullptr, h->w.bin_force, saddle_x,
+                                                   h->w.u8);
     if (wave) {
         {
             ProfRegion pr(h, R_SPREAD);
@@ -1775,7 +1816,7 @@ int mobility_apply(fsd_handle* h, const float4* pos, const float* genF, float* g
         }
     }
     ProfRegion pr(h, R_REAL);
-    mobility_combine(h, pos, genF, genU, wave, real, saddle_x);
+    mobility_combine(h, genU, wave, real, saddle_x);
     FSD_CHECK_CUDA(cudaGetLastError());
     return FSD_OK;
 }

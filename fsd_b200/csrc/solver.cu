@@ -29,7 +29,7 @@ int saddle_multiply(fsd_handle* h, const float4* pos, const float* x, float* b, 
     const int N = h->p.N;
     int st = mobility_apply(h, pos, x, b, 3, x, rebin);
     if (st != FSD_OK) return st;
-    lub_rfu(h, pos, x + 11 * N, b + 11 * N, x);
+    lub_rfu_packed(h, pos, b + 11 * N, x);
     FSD_CHECK_CUDA(cudaGetLastError());
     return FSD_OK;
 }

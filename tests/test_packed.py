@@ -56,3 +56,28 @@ def test_approximate_inverse_of_every_set_size(cuda, N):
     b = np.random.default_rng(N).standard_normal(17 * N)
     assert rel(s.precond_apply(dev(b)).cpu().numpy(), O.saddle_precond(b, G, N)) < 1e-5
     s.close()
+
+
+@pytest.mark.parametrize("N", [1, 2, 5, 31, 33, 257, 700])
+@pytest.mark.parametrize("xy", [0.0, -0.5])
+def test_pair_sums_of_small_and_odd_sizes(cuda, N, xy):
+    """Real-space mobility and the four lubrication products; the velocity also from an address that is a
+    multiple of four bytes only.  FP32 pair sums: 1e-6 expected, 1e-5 allowed."""
+    pos = packed(N, 2.03, N)
+    s, p = solver(pos, xy)
+    pr = O.Problem(pos, L, xy, table=ewald_golden())
+    rng = np.random.default_rng(N + 1)
+    F, U = rng.standard_normal(11 * N).astype(np.float32), rng.standard_normal(6 * N).astype(np.float32)
+    assert rel(s.mobility(p, dev(F), parts=2).cpu(), pr.mobility(F, parts=2)) < 1e-5
+    got = s.rfu(p, dev(U))
+    if N == 1:
+        assert not got.any()
+    else:
+        assert rel(got.cpu(), pr.rfu(U)) < 1e-5
+    odd = torch.zeros(6 * N + 1, device="cuda")
+    odd[1:] = dev(U)
+    assert torch.equal(s.rfu(p, odd[1:]), got)
+    sl = s.rsu(p, dev(U)).cpu().numpy()
+    assert torch.equal(s.rsu(p, odd[1:]).cpu(), torch.as_tensor(sl))
+    assert np.isfinite(sl).all() and np.isfinite(s.rfe(p, 0.7).cpu().numpy()).all()
+    s.close()
