@@ -70,22 +70,25 @@ static int allocate(fsd_handle* h) {
     // Cell capacity for the untilted box (tilting only removes cells).
     const int3 nc = cell_dims(Box{h->box.Lx, h->box.Ly, h->box.Lz, 0.0f}, rlist);
     w.ncell_cap = (nc.x >= 3 && nc.y >= 3 && nc.z >= 3) ? (size_t)nc.x * nc.y * nc.z : 0;
-    FSD_TRY(dalloc(&w.scan_scratch, scan_scratch_elems((int)w.ncell_cap + 1)));
+    w.ncell_pad = ((w.ncell_cap + 15) & ~(size_t)15) + 16;
     FSD_TRY(dalloc(&w.part_cell, N));
-    FSD_TRY(dalloc(&w.cell_count, w.ncell_cap + 1));
+    FSD_TRY(dalloc(&w.part_slot, N));
+    FSD_TRY(dalloc(&w.cell_count, w.ncell_pad));
     FSD_TRY(dalloc(&w.cell_start, w.ncell_cap + 1));
-    FSD_TRY(dalloc(&w.cell_fill, w.ncell_cap + 1));
+    FSD_TRY(dalloc(&w.cell_items, N));
     FSD_TRY(dalloc(&w.cell_parts, N));
+    FSD_TRY(dalloc(&w.cell_pos, N));
     FSD_TRY(dalloc(&w.order, N));
     FSD_TRY(dalloc(&w.lub_n, N));
     FSD_TRY(init_particle_order(h));
     const size_t ncol = (size_t)h->g.Nx * h->g.Ny;
     FSD_TRY(dalloc(&w.bin_key, 2 * (size_t)N));
     FSD_TRY(dalloc(&w.bin_items, N));
-    FSD_TRY(dalloc(&w.col_count, ncol));
+    const size_t ncol_pad = (ncol + 15) & ~(size_t)15;  // scanned in runs of 16
+    FSD_TRY(dalloc(&w.col_count, ncol_pad));
     FSD_TRY(dalloc(&w.col_start, ncol + 1));
     FSD_TRY(dalloc(&w.bin_ticket, 1));
-    FSD_CHECK_CUDA(cudaMemsetAsync(w.col_count, 0, sizeof(unsigned) * ncol, h->stream));
+    FSD_CHECK_CUDA(cudaMemsetAsync(w.col_count, 0, sizeof(unsigned) * ncol_pad, h->stream));
     FSD_CHECK_CUDA(cudaMemsetAsync(w.bin_ticket, 0, sizeof(unsigned), h->stream));
     FSD_TRY(dalloc(&w.bin_start, G + 1));
     FSD_TRY(dalloc(&w.bin_parts, N));
@@ -146,8 +149,8 @@ static int allocate(fsd_handle* h) {
 
 static void release(fsd_handle* h) {
     Workspace& w = h->w;
-    void* dev[] = {w.nneigh, w.nlist, w.nl_overflow, w.scan_scratch, w.part_cell, w.cell_count, w.cell_start,
-                   w.cell_fill, w.cell_parts, w.order, w.lub_n, w.lub_list, w.bin_key, w.bin_items, w.col_count,
+    void* dev[] = {w.nneigh, w.nlist, w.nl_overflow, w.part_cell, w.part_slot, w.cell_count, w.cell_start,
+                   w.cell_items, w.cell_parts, w.cell_pos, w.order, w.lub_n, w.lub_list, w.bin_key, w.bin_items, w.col_count,
                    w.col_start, w.bin_ticket, w.bin_start, w.bin_parts, w.bin_pos, w.bin_force, w.grid, w.gridk, w.twiddle, w.spec, w.green_table, w.rec, w.u8, w.uwave, w.sx, w.sy, w.sz, w.V, w.Z, w.dred,
                    w.hcol, w.hcol2, w.ticket, w.gmres_state, w.pc_t, w.pc_y, w.rhs, w.sol, w.rfd_rhs, w.rfd_sol, w.psi,
                    w.pos_prime, w.vel, w.force, w.lanczos_V, w.lz_a, w.lz_b, w.lz_c, w.lz_dot, h->d_ewald,
@@ -495,7 +498,6 @@ int fsd_build_neighbor_list(fsd_handle* h, const float* d_pos) {
         FSD_TRY(build_neighbor_list(h, (const float4*)d_pos, &maxc));
         h->info.nlist_max = maxc;
         if (maxc <= h->w.nl_stride) {
-            FSD_TRY(build_lub_list(h, (const float4*)d_pos));
             h->nlist_valid = true;
             h->pc_valid = false;
             return FSD_OK;

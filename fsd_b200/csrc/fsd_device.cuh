@@ -147,4 +147,49 @@ __device__ __forceinline__ void block_partial(double v, double* part) {
     }
 }
 
+// Exclusive scan of count[0:n] into start[0:n] (start[n] = total) by one block
+// of up to 1024 threads; count is padded to a multiple of 16 and read past the
+// L1 (other blocks' atomics).
+__device__ __forceinline__ void block_scan_counts(const unsigned* count, unsigned* start, int n) {
+    __shared__ unsigned sh[32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    unsigned carry = 0;
+    for (int base = 0; base < n; base += 16 * blockDim.x) {
+        const int c0 = base + 16 * threadIdx.x;
+        unsigned v[16], sum = 0;
+#pragma unroll
+        for (int k = 0; k < 16; k += 4) {
+            const uint4 q = c0 + k < n ? __ldcg(reinterpret_cast<const uint4*>(count + c0 + k))
+                                       : make_uint4(0u, 0u, 0u, 0u);
+            v[k] = q.x;
+            v[k + 1] = q.y;
+            v[k + 2] = q.z;
+            v[k + 3] = q.w;
+            sum += q.x + q.y + q.z + q.w;
+        }
+        unsigned x = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) sh[wid] = x;
+        __syncthreads();
+        unsigned before = 0, all = 0;
+        for (int k = 0; k < nw; ++k) {
+            if (k < wid) before += sh[k];
+            all += sh[k];
+        }
+        unsigned off = carry + before + x - sum;
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+            if (c0 + k < n) start[c0 + k] = off;
+            off += v[k];
+        }
+        carry += all;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) start[n] = carry;
+}
+
 }  // namespace fsd

@@ -70,13 +70,15 @@ struct Workspace {
     int nl_stride = 0;
     int* nl_overflow = nullptr;    // device: largest count seen
     int* host_flag = nullptr;      // pinned host mirror of small flags
-    unsigned* scan_scratch = nullptr;
     // cell list
     unsigned* part_cell = nullptr;
-    unsigned* cell_count = nullptr;
+    unsigned* part_slot = nullptr;
+    unsigned* cell_count = nullptr;  // ncell_pad entries, the last a block ticket
     unsigned* cell_start = nullptr;
-    unsigned* cell_fill = nullptr;
-    unsigned* cell_parts = nullptr;
+    unsigned* cell_items = nullptr;  // particles by cell, unsorted within it
+    unsigned* cell_parts = nullptr;  // and sorted
+    float4* cell_pos = nullptr;      // their positions in that order, w = index (bits)
+    size_t ncell_pad = 0;
     size_t ncell_cap = 0;
     // particles in cell order (a permutation of 0..N-1, identity until the
     // first cell-list build): the order in which per-particle pair kernels

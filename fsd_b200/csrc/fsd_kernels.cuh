@@ -8,11 +8,8 @@ namespace fsd {
 // nlist.cu
 size_t scan_scratch_elems(int n);
 void exclusive_scan(const unsigned* in, unsigned* out, int n, unsigned* scratch, cudaStream_t st);
-void counting_sort(const unsigned* key, int n, int nbins, unsigned* count, unsigned* start, unsigned* fill,
-                   unsigned* items, unsigned* scan_scratch, cudaStream_t st);
 int3 cell_dims(const Box& b, float rlist);
 int build_neighbor_list(fsd_handle* h, const float4* pos, int* max_count_host);
-int build_lub_list(fsd_handle* h, const float4* pos);
 int init_particle_order(fsd_handle* h);
 
 // mobility.cu

@@ -604,49 +604,8 @@ __global__ void __launch_bounds__(1024) k_col_count(const float4* __restrict__ p
     }
     __threadfence();
     if (!last_block(ticket)) return;
-    __shared__ unsigned sh[32];
-    const int ncol = Nx * Ny;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    unsigned carry = 0;
-    for (int base = 0; base < ncol; base += 4 * blockDim.x) {
-        const int c0 = base + 4 * threadIdx.x;
-        unsigned v[4], sum = 0;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            v[k] = c0 + k < ncol ? __ldcg(col_count + c0 + k) : 0u;
-            sum += v[k];
-        }
-        unsigned x = sum;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += y;
-        }
-        if (lane == 31) sh[wid] = x;
-        __syncthreads();
-        if (wid == 0) {
-            unsigned y = lane < (int)(blockDim.x >> 5) ? sh[lane] : 0u;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const unsigned z = __shfl_up_sync(0xffffffffu, y, o);
-                if (lane >= o) y += z;
-            }
-            sh[lane] = y;
-        }
-        __syncthreads();
-        unsigned off = carry + (wid ? sh[wid - 1] : 0u) + x - sum;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            if (c0 + k < ncol) col_start[c0 + k] = off;
-            off += v[k];
-        }
-        carry += sh[(blockDim.x >> 5) - 1];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        col_start[ncol] = carry;
-        *ticket = 0;
-    }
+    block_scan_counts(col_count, col_start, Nx * Ny);
+    if (threadIdx.x == 0) *ticket = 0;
 }
 
 // Particles into their columns (in the order the atomics gave; ranked below),

@@ -711,7 +711,9 @@ int precond_build(fsd_handle* h, const float4* pos) {
     ProfRegion pr(h, R_PRECOND_BUILD);
     FSD_CHECK_CUDA(cudaMemsetAsync(ic->p_over, 0, sizeof(int), st));
     count_launch();
-    k_prune<<<(N + 127) / 128, 128, 0, st>>>(pos, N, h->box, h->w.nneigh, h->w.nlist, h->w.nl_stride,
+    const bool near = h->p.rp <= h->p.rlub;  // the lubrication sub-list holds every pair within rp
+    k_prune<<<(N + 127) / 128, 128, 0, st>>>(pos, N, h->box, near ? h->w.lub_n : h->w.nneigh,
+                                             near ? h->w.lub_list : h->w.nlist, h->w.nl_stride,
                                              h->p.rp * h->p.rp, ic->pn, ic->plist, ic->p_over);
     ic->h_pn.resize(N);
     ic->h_plist.resize((size_t)N * kPrunedCap);
@@ -847,7 +849,9 @@ int precond_assemble_pruned(fsd_handle* h, const float4* pos, float relaxer, con
     cudaStream_t st = h->stream;
     FSD_CHECK_CUDA(cudaMemsetAsync(ic->p_over, 0, sizeof(int), st));
     count_launch();
-    k_prune<<<(N + 127) / 128, 128, 0, st>>>(pos, N, h->box, h->w.nneigh, h->w.nlist, h->w.nl_stride,
+    const bool near = h->p.rp <= h->p.rlub;  // the lubrication sub-list holds every pair within rp
+    k_prune<<<(N + 127) / 128, 128, 0, st>>>(pos, N, h->box, near ? h->w.lub_n : h->w.nneigh,
+                                             near ? h->w.lub_list : h->w.nlist, h->w.nl_stride,
                                              h->p.rp * h->p.rp, ic->pn, ic->plist, ic->p_over);
     count_launch();
     k_assemble<<<(N + 127) / 128, 128, 0, st>>>(pos, N, h->box, ic->pn, ic->plist,

@@ -81,3 +81,24 @@ def test_pair_sums_of_small_and_odd_sizes(cuda, N, xy):
     assert torch.equal(s.rsu(p, odd[1:]).cpu(), torch.as_tensor(sl))
     assert np.isfinite(sl).all() and np.isfinite(s.rfe(p, 0.7).cpu().numpy()).all()
     s.close()
+
+
+@pytest.mark.parametrize("N,edge,xy", [(1, 13.0, 0.0), (2, 14.0, 0.5), (33, 15.0, -0.5), (300, 16.0, 0.31),
+                                       (1025, 27.0, 0.49), (700, 40.0, 0.0)])
+def test_neighbor_rows_at_few_cells(cuda, N, edge, xy):
+    """Rows against all pairs where the box has two, three or four cells per axis, and the sheared image of a
+    cell reaches the next; pairs within rounding of the list radius are left out of the comparison."""
+    rng = np.random.default_rng(N)
+    pos = np.zeros((N, 4), np.float32)
+    pos[:, :3] = (rng.random((N, 3)) - 0.5) * edge
+    pos[:, 0] += xy * pos[:, 1]
+    box = (edge,) * 3
+    s = FSD(N, (*box, xy))
+    s.build_neighbor_list(dev(pos))
+    r = s.pse_info().ewald_cut + 0.4
+    rows = s.neighbor_list()
+    lo, hi = O.neighbor_list(pos, box, xy, r - 1e-5), O.neighbor_list(pos, box, xy, r + 1e-5)
+    for got, a, b in zip(rows, lo, hi):
+        assert len(np.unique(got)) == len(got)
+        assert set(a) <= set(got) <= set(b)
+    s.close()
