@@ -116,7 +116,6 @@ static int allocate(fsd_handle* h) {
     FSD_TRY(dalloc(&w.hcol, 2 * (kMaxRestart + 2)));
     FSD_TRY(dalloc(&w.ticket, 1));
     FSD_CHECK_CUDA(cudaMemsetAsync(w.ticket, 0, sizeof(unsigned), h->stream));
-    FSD_TRY(dalloc(&w.hcol2, kMaxRestart + 2));
     FSD_TRY(gmres_alloc(h));
     FSD_TRY(dalloc(&w.pc_t, 6 * (size_t)N));
     FSD_TRY(dalloc(&w.pc_y, 6 * (size_t)N));
@@ -152,7 +151,7 @@ static void release(fsd_handle* h) {
     void* dev[] = {w.nneigh, w.nlist, w.nl_overflow, w.part_cell, w.part_slot, w.cell_count, w.cell_start,
                    w.cell_items, w.cell_parts, w.cell_pos, w.order, w.lub_n, w.lub_list, w.bin_key, w.bin_items, w.col_count,
                    w.col_start, w.bin_ticket, w.bin_start, w.bin_parts, w.bin_pos, w.bin_force, w.grid, w.gridk, w.twiddle, w.spec, w.green_table, w.rec, w.u8, w.uwave, w.sx, w.sy, w.sz, w.V, w.Z, w.dred,
-                   w.hcol, w.hcol2, w.ticket, w.gmres_state, w.pc_t, w.pc_y, w.rhs, w.sol, w.rfd_rhs, w.rfd_sol, w.psi,
+                   w.hcol, w.ticket, w.gmres_state, w.pc_t, w.pc_y, w.rhs, w.sol, w.rfd_rhs, w.rfd_sol, w.psi,
                    w.pos_prime, w.vel, w.force, w.lanczos_V, w.lz_a, w.lz_b, w.lz_c, w.lz_dot, h->d_ewald,
                    h->d_res_dist, h->d_res_vals, h->d_res_rfu, h->d_res_g, h->d_res_m, w.rk_pos, w.rk_posw, w.rk_ori, w.rk_vel, w.rk_u1, w.rk_noise};
     for (void* p : dev)

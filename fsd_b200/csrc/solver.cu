@@ -102,34 +102,6 @@ __global__ void __launch_bounds__(kRedThreads) k_multidot(const float* __restric
     }
 }
 
-// Same partial dots for the Gram-Schmidt passes, where nv is large: the
-// block's slice of w is staged in shared memory once and each warp takes
-// whole vectors, so no block-wide reduction is needed per vector.  Slices are
-// `chunk` long (the launch's dynamic shared memory is chunk floats).
-__global__ void __launch_bounds__(kRedThreads) k_multidot_ws(const float* __restrict__ V, size_t ld, int nv,
-                                                             const float* __restrict__ w, size_t n, size_t chunk,
-                                                             double* part, const int* done) {
-    if (done && *done) return;
-    extern __shared__ float ws[];
-    const size_t b0 = (size_t)blockIdx.x * chunk;
-    const size_t len = b0 < n ? min(chunk, n - b0) : 0;
-    for (size_t k = threadIdx.x; k < len; k += blockDim.x) ws[k] = w[b0 + k];
-    __syncthreads();
-    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (int i = threadIdx.x >> 5; i < nv; i += nw) {
-        const float* vi = V + (size_t)i * ld + b0;
-        double s = 0.0;
-        size_t k = lane;
-        for (; k + 96 < len; k += 128) {
-            const float a0 = vi[k], a1 = vi[k + 32], a2 = vi[k + 64], a3 = vi[k + 96];
-            s += (double)a0 * ws[k] + (double)a1 * ws[k + 32] + (double)a2 * ws[k + 64] + (double)a3 * ws[k + 96];
-        }
-        for (; k < len; k += 32) s += (double)vi[k] * ws[k];
-        s = group_sum_d<32>(s);
-        if (lane == 0) part[(size_t)i * gridDim.x + blockIdx.x] = s;
-    }
-}
-
 // out[i] (+)= sum_b part[i * nb + b], one warp per i.
 __global__ void k_finish_dots(const double* part, int nb, int nv, double* out, bool accumulate, const int* done) {
     if (done && *done) return;
@@ -140,20 +112,6 @@ __global__ void k_finish_dots(const double* part, int nb, int nv, double* out, b
     for (int b = lane; b < nb; b += 32) s += part[(size_t)i * nb + b];
     s = group_sum_d<32>(s);
     if (lane == 0) out[i] = accumulate ? out[i] + s : s;
-}
-
-// w -= sum_i c[i] V_i.
-__global__ void k_multiaxpy(const float* __restrict__ V, size_t ld, int nv, const double* __restrict__ c, float* w,
-                            size_t n, const int* done) {
-    if (done && *done) return;
-    __shared__ float cs[kMaxRestart + 1];
-    for (int i = threadIdx.x; i < nv; i += blockDim.x) cs[i] = (float)c[i];
-    __syncthreads();
-    for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x) {
-        float acc = w[k];
-        for (int i = 0; i < nv; ++i) acc -= cs[i] * V[(size_t)i * ld + k];
-        w[k] = acc;
-    }
 }
 
 // y = sum_i c[i] V_i.
@@ -186,11 +144,6 @@ __global__ void k_residual(const float* __restrict__ b, const float* __restrict_
 __global__ void k_axpy(float* __restrict__ x, const float* __restrict__ u, size_t n) {
     for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
         x[k] += u[k];
-}
-
-__global__ void k_add_dots(double* a, const double* b, int n, const int* done) {
-    if (done && *done) return;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) a[i] += b[i];
 }
 
 // --------------------------------------------------------- Arnoldi control
@@ -240,52 +193,34 @@ __global__ void k_cycle_start(GmresState* s, const double* dots, double tol, int
     s->done = (s->resid <= tol || beta2 == 0.0 || !(beta2 == beta2)) ? 1 : 0;
 }
 
-// After orthogonalising column j: h[0..j] in hcol, ||w||^2 in hcol[j+1].
-__global__ void k_arnoldi_update(GmresState* s, const double* hcol, int m) {
-    if (s->done) return;
-    const int j = s->j;
-    for (int i = 0; i <= j; ++i) s->H[i][j] = hcol[i];
-    const double hn2 = hcol[j + 1];
-    double hj1 = sqrt(hn2 > 0.0 ? hn2 : 0.0);
-    s->H[j + 1][j] = hj1;
-    for (int i = 0; i < j; ++i) {
-        const double a = s->H[i][j], b = s->H[i + 1][j];
-        s->H[i][j] = s->cs[i] * a + s->sn[i] * b;
-        s->H[i + 1][j] = -s->sn[i] * a + s->cs[i] * b;
-    }
-    const double a = s->H[j][j], b = s->H[j + 1][j];
-    const double r = hypot(a, b);
-    const double c = r > 0.0 ? a / r : 1.0, sv = r > 0.0 ? b / r : 0.0;
-    s->cs[j] = c;
-    s->sn[j] = sv;
-    s->H[j][j] = r;
-    s->H[j + 1][j] = 0.0;
-    s->g[j + 1] = -sv * s->g[j];
-    s->g[j] = c * s->g[j];
-    s->j = j + 1;
-    s->total += 1;
-    const double bn = s->bnorm2 > 0.0 ? sqrt(s->bnorm2) : 1.0;
-    s->resid = fabs(s->g[j + 1]) / bn;
-    if (!(hj1 > 1e-300) || !(s->resid == s->resid)) s->breakdown = (hj1 > 1e-300) ? 2 : 1;
-    if (s->resid <= s->tol || s->j >= m || s->breakdown) s->done = 1;
-}
-
 // Least-squares solve H y = g (upper triangular, size j).  With apply_t the
 // coefficients are mapped from the preconditioned vectors to the final basis:
-// sum_c y_c v~_c = sum_i (T y)_i V_i.
-__global__ void k_lsq(GmresState* s, int apply_t) {
-    const int j = s->j;
-    for (int i = j - 1; i >= 0; --i) {
-        double v = s->g[i];
-        for (int k = i + 1; k < j; ++k) v -= s->H[i][k] * s->y[k];
-        s->y[i] = (s->H[i][i] != 0.0) ? v / s->H[i][i] : 0.0;
+// sum_c y_c v~_c = sum_i (T y)_i V_i.  One block, thread i owns row i: each
+// solved y_k leaves all rows at once (one thread walking the triangle took
+// 40 us for 25 iterations and 122 us for 60).
+constexpr int kLsqThreads = (kMaxRestart + 31) / 32 * 32;
+
+__global__ void __launch_bounds__(kLsqThreads) k_lsq(GmresState* s, int apply_t) {
+    __shared__ double y[kMaxRestart];
+    const int j = s->j, i = threadIdx.x;
+    double g = i < j ? s->g[i] : 0.0;
+    const double d = i < j ? s->H[i][i] : 0.0;
+    double h = i < j - 1 ? s->H[i][j - 1] : 0.0;  // column k of this row, loaded a step ahead
+    for (int k = j - 1; k >= 0; --k) {
+        const double hn = i < k - 1 ? s->H[i][k - 1] : 0.0;
+        if (i == k) y[k] = d != 0.0 ? g / d : 0.0;
+        __syncthreads();
+        if (i < k) g -= h * y[k];
+        h = hn;
     }
-    if (!apply_t) return;
-    for (int i = 0; i < j; ++i) {
-        double v = 0.0;
-        for (int c = i; c < j; ++c) v += s->Tc[c][i] * s->y[c];
-        s->y[i] = v;  // y[c] for c > i is still unmapped; y[i] is not read again
+    if (i >= j) return;
+    double v = y[i];
+    if (apply_t) {
+        v = 0.0;
+#pragma unroll 4
+        for (int c = i; c < j; ++c) v += s->Tc[c][i] * y[c];
     }
+    s->y[i] = v;
 }
 
 struct GmresHost {
@@ -319,56 +254,94 @@ __global__ void k_export(const GmresState* s, GmresHost* o) {
 // or the cycle is full.
 
 // part[(2i) nb + b] = V_i . V_j and part[(2i+1) nb + b] = V_i . w over block
-// b's slice, i <= j; both slices of V_j and w are staged in shared memory.
-// Slices are `chunk` long, a multiple of 4, and the basis vectors start on
-// 16-byte boundaries, so the basis is read as float4.
-__global__ void __launch_bounds__(kRedThreads) k_dots_pair(const float* __restrict__ V, size_t ld, int j,
-                                                           const float* __restrict__ w, size_t n, size_t chunk,
-                                                           double* part, const int* done) {
+// b's slices, i <= j; with `out` the last block also sums them into
+// out[0:2(j+1)] (few blocks; otherwise k_finish_dots).
+//
+// A warp holds its slice of V_j and w (32 float4) in registers as FP64 and
+// reads 16 basis vectors against it, so a basis value is converted once (it
+// was the conversions, three per value, that bound the previous form: 30.6 us
+// at N = 32768 and 33 vectors, 12 us of memory time).  The 32 sums are reduced
+// by halving exchanges, which leaves sum l in lane l.
+constexpr int kPairVecs = 16;
+constexpr int kPairSlice = 32;  // float4 per warp and slice
+
+__global__ void __launch_bounds__(kRedThreads, 2) k_dots_pair(const float* __restrict__ V, size_t ld, int j,
+                                                              const float* __restrict__ w, size_t n, double* part,
+                                                              const int* done, double* out, unsigned* ticket) {
     if (*done) return;
-    extern __shared__ float4 sm4[];
-    float4* sv = sm4;
-    float4* sw = sm4 + chunk / 4;
-    const size_t b0 = (size_t)blockIdx.x * chunk;
-    const size_t len = b0 < n ? min(chunk, n - b0) : 0;
-    const size_t len4 = len / 4;
-    const float* vj = V + (size_t)j * ld + b0;
-    for (size_t k = threadIdx.x; k < len4; k += blockDim.x) {
-        sv[k] = reinterpret_cast<const float4*>(vj)[k];
-        sw[k] = make_float4(w[b0 + 4 * k], w[b0 + 4 * k + 1], w[b0 + 4 * k + 2], w[b0 + 4 * k + 3]);
+    __shared__ double red[kRedThreads / 32][32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const size_t n4 = n / 4, ld4 = ld / 4;
+    const size_t nslice = (n4 + kPairSlice - 1) / kPairSlice;
+    const size_t gw = (size_t)blockIdx.x * (kRedThreads / 32) + wid, nw = (size_t)gridDim.x * (kRedThreads / 32);
+    const float4* V4 = reinterpret_cast<const float4*>(V);
+    const float4* vj = V4 + (size_t)j * ld4;
+    const float4* w4 = reinterpret_cast<const float4*>(w);
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int g0 = 0; g0 <= j; g0 += kPairVecs) {
+        double acc[2 * kPairVecs];
+#pragma unroll
+        for (int k = 0; k < 2 * kPairVecs; ++k) acc[k] = 0.0;
+        for (size_t s = gw; s < nslice; s += nw) {
+            const size_t f = s * kPairSlice + lane;
+            const bool in = f < n4;
+            const float4 p = in ? vj[f] : zero, q = in ? w4[f] : zero;
+            const double pd[4] = {p.x, p.y, p.z, p.w}, qd[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+            for (int u = 0; u < kPairVecs; u += 8) {
+                float4 a[8];  // vectors past j repeat it (their sums are dropped)
+#pragma unroll
+                for (int t = 0; t < 8; ++t) a[t] = in ? V4[(size_t)min(g0 + u + t, j) * ld4 + f] : zero;
+#pragma unroll
+                for (int t = 0; t < 8; ++t) {
+                    const double ad[4] = {a[t].x, a[t].y, a[t].z, a[t].w};
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        acc[2 * (u + t)] += ad[c] * pd[c];
+                        acc[2 * (u + t) + 1] += ad[c] * qd[c];
+                    }
+                }
+            }
+        }
+        // the ragged end (n not a multiple of 4)
+        if (gw == nw - 1 && 4 * n4 + lane < n) {
+            const size_t t = 4 * n4 + lane;
+            const double p = V[(size_t)j * ld + t], q = w[t];
+#pragma unroll
+            for (int u = 0; u < kPairVecs; ++u)
+                if (g0 + u <= j) {
+                    const double a = V[(size_t)(g0 + u) * ld + t];
+                    acc[2 * u] += a * p;
+                    acc[2 * u + 1] += a * q;
+                }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const bool up = lane & o;
+#pragma unroll
+            for (int k = 0; k < o; ++k) {
+                const double keep = up ? acc[o + k] : acc[k], send = up ? acc[k] : acc[o + k];
+                acc[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+            }
+        }
+        red[wid][lane] = acc[0];
+        __syncthreads();
+        if (wid == 0 && g0 + lane / 2 <= j) {
+            double t = 0.0;
+#pragma unroll
+            for (int k = 0; k < kRedThreads / 32; ++k) t += red[k][lane];
+            part[(size_t)(2 * g0 + lane) * gridDim.x + blockIdx.x] = t;
+        }
+        __syncthreads();
     }
-    __syncthreads();
-    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (int i = threadIdx.x >> 5; i <= j; i += nw) {
-        const float4* vi = reinterpret_cast<const float4*>(V + (size_t)i * ld + b0);
-        double s1 = 0.0, s2 = 0.0;
-        size_t k = lane;
-        for (; k + 32 < len4; k += 64) {
-            const float4 a = vi[k], c = vi[k + 32];
-            const float4 p = sv[k], q = sw[k], p2 = sv[k + 32], q2 = sw[k + 32];
-            s1 += (double)a.x * p.x + (double)a.y * p.y + (double)a.z * p.z + (double)a.w * p.w +
-                  (double)c.x * p2.x + (double)c.y * p2.y + (double)c.z * p2.z + (double)c.w * p2.w;
-            s2 += (double)a.x * q.x + (double)a.y * q.y + (double)a.z * q.z + (double)a.w * q.w +
-                  (double)c.x * q2.x + (double)c.y * q2.y + (double)c.z * q2.z + (double)c.w * q2.w;
-        }
-        for (; k < len4; k += 32) {
-            const float4 a = vi[k], p = sv[k], q = sw[k];
-            s1 += (double)a.x * p.x + (double)a.y * p.y + (double)a.z * p.z + (double)a.w * p.w;
-            s2 += (double)a.x * q.x + (double)a.y * q.y + (double)a.z * q.z + (double)a.w * q.w;
-        }
-        // the ragged end of the last slice
-        const float* vs = V + (size_t)i * ld + b0;
-        for (size_t t = 4 * len4 + lane; t < len; t += 32) {
-            s1 += (double)vs[t] * vj[t];
-            s2 += (double)vs[t] * w[b0 + t];
-        }
-        s1 = group_sum_d<32>(s1);
-        s2 = group_sum_d<32>(s2);
-        if (lane == 0) {
-            part[(size_t)(2 * i) * gridDim.x + blockIdx.x] = s1;
-            part[(size_t)(2 * i + 1) * gridDim.x + blockIdx.x] = s2;
-        }
+    if (!out) return;
+    if (wid == 0) __threadfence();
+    if (!last_block(ticket)) return;
+    for (int q = wid; q < 2 * (j + 1); q += kRedThreads / 32) {
+        const double t = warp_sum_parts(part + (size_t)q * gridDim.x, gridDim.x);
+        if (lane == 0) out[q] = t;
     }
+    if (threadIdx.x == 0) *ticket = 0;
 }
 
 // Givens rotations 0..c-1 applied to column col (rows 0..c, in shared
@@ -601,21 +574,10 @@ int saddle_solve(fsd_handle* h, const float4* pos, const float* b, float* x, flo
     // applications: the preconditioned basis Z is kept and x += Z y.
     const bool flexible = precond_is_flexible(h);
     if (flexible && !w.Z) return FSD_ERR_BAD_PARAMS;
-    const size_t chunk = (n + nbl - 1) / nbl;
-    const bool staged = chunk * sizeof(float) <= 48 * 1024;
-    // Delayed re-orthogonalisation stages two slices per block, each a
-    // multiple of 4 floats long.
-    const size_t chunk4 = (chunk + 3) & ~(size_t)3;
-    const size_t pair_smem = 2 * chunk4 * sizeof(float);
-    const bool delayed = pair_smem <= 200 * 1024;
-    if (delayed && pair_smem > 48 * 1024)
-        FSD_CHECK_CUDA(ensure_smem_limit((const void*)k_dots_pair, pair_smem));
-    auto multidot = [&](const float* Vb, size_t ldv, int nv, const float* wv, size_t nn, double* pt, const int* dn) {
-        if (staged)
-            k_multidot_ws<<<nbl, kRedThreads, chunk * sizeof(float), st>>>(Vb, ldv, nv, wv, nn, chunk, pt, dn);
-        else
-            k_multidot<<<nbl, kRedThreads, 0, st>>>(Vb, ldv, nv, wv, nn, pt, dn);
-    };
+    // Blocks of the paired dots: up to two per SM, one slice per warp.
+    const int pbl = (int)std::min<size_t>(nbl, (n / 4 / kPairSlice + kRedThreads / 32) / (kRedThreads / 32));
+    const bool pfinish = pbl <= 64;
+    const int ubl = (int)std::min<size_t>(2 * 148, (n / 4 + kRedThreads) / kRedThreads);
     int total = 0;
     bool first = true;
     int status = FSD_OK;
@@ -659,45 +621,15 @@ int saddle_solve(fsd_handle* h, const float4* pos, const float* b, float* x, flo
                 e = saddle_multiply(h, pos, zj, Ax, false);
                 if (e != FSD_OK) return e;
                 ProfRegion pk(h, R_KRYLOV);
-                if (delayed) {
+                count_launch();
+                k_dots_pair<<<pbl, kRedThreads, 0, st>>>(V, ld, j, Ax, n, part, &gs->done, pfinish ? dots : nullptr,
+                                                         w.ticket);
+                if (!pfinish) {
                     count_launch();
-                    k_dots_pair<<<nbl, kRedThreads, pair_smem, st>>>(V, ld, j, Ax, n, chunk4, part, &gs->done);
-                    count_launch();
-                    k_finish_dots<<<(2 * (j + 1) + 7) / 8, 256, 0, st>>>(part, nbl, 2 * (j + 1), dots, false,
-                                                                         &gs->done);
-                    count_launch();
-                    k_dcgs_update<<<2 * 148, kRedThreads, 0, st>>>(V, ld, j, Ax, n, dots, gs, m, part, w.ticket);
-                    if ((j % 4) == 3 || j == m - 1) {
-                        count_launch();
-                        k_export<<<1, 1, 0, st>>>(gs, gh);
-                        FSD_CHECK_CUDA(cudaStreamSynchronize(st));
-                        if (gh->done) break;
-                    }
-                    continue;
+                    k_finish_dots<<<(2 * (j + 1) + 7) / 8, 256, 0, st>>>(part, pbl, 2 * (j + 1), dots, false, &gs->done);
                 }
-                // CGS2 against V_0..V_j.
                 count_launch();
-                multidot(V, ld, j + 1, Ax, n, part, &gs->done);
-                count_launch();
-                k_finish_dots<<<(j + 1 + 7) / 8, 256, 0, st>>>(part, nbl, j + 1, dots, false, &gs->done);
-                count_launch();
-                k_multiaxpy<<<vblocks, vthreads, 0, st>>>(V, ld, j + 1, dots, Ax, n, &gs->done);
-                count_launch();
-                multidot(V, ld, j + 1, Ax, n, part, &gs->done);
-                count_launch();
-                k_finish_dots<<<(j + 1 + 7) / 8, 256, 0, st>>>(part, nbl, j + 1, w.hcol2, false, &gs->done);
-                count_launch();
-                k_multiaxpy<<<vblocks, vthreads, 0, st>>>(V, ld, j + 1, w.hcol2, Ax, n, &gs->done);
-                count_launch();
-                k_add_dots<<<1, 128, 0, st>>>(dots, w.hcol2, j + 1, &gs->done);
-                count_launch();
-                k_multidot<<<nbl, kRedThreads, 0, st>>>(Ax, n, 1, Ax, n, part, &gs->done);
-                count_launch();
-                k_finish_dots<<<1, 32, 0, st>>>(part, nbl, 1, dots + j + 1, false, &gs->done);
-                count_launch();
-                k_arnoldi_update<<<1, 1, 0, st>>>(gs, dots, m);
-                count_launch();
-                k_scale_copy<<<vblocks, vthreads, 0, st>>>(Ax, V + (size_t)(j + 1) * ld, n, dots + j + 1, &gs->done);
+                k_dcgs_update<<<ubl, kRedThreads, 0, st>>>(V, ld, j, Ax, n, dots, gs, m, part, w.ticket);
                 if ((j % 4) == 3 || j == m - 1) {
                     count_launch();
                     k_export<<<1, 1, 0, st>>>(gs, gh);
@@ -715,7 +647,7 @@ int saddle_solve(fsd_handle* h, const float4* pos, const float* b, float* x, flo
             total = gh->total;
             if (jc > 0) {
                 count_launch();
-                k_lsq<<<1, 1, 0, st>>>(gs, delayed && !flexible ? 1 : 0);
+                k_lsq<<<1, kLsqThreads, 0, st>>>(gs, flexible ? 0 : 1);
                 if (flexible) {  // x += Z y
                     count_launch();
                     k_combine<<<vblocks, vthreads, 0, st>>>(w.Z, ld, jc, gs_y(gs), z, n);

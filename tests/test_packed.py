@@ -102,3 +102,19 @@ def test_neighbor_rows_at_few_cells(cuda, N, edge, xy):
         assert len(np.unique(got)) == len(got)
         assert set(a) <= set(got) <= set(b)
     s.close()
+
+
+@pytest.mark.parametrize("precond,inner", [("none", 0), ("learned", 0), ("learned", 4)])
+@pytest.mark.parametrize("N", [1, 2, 3, 6, 31])
+def test_solve_of_unaligned_lengths(cuda, N, precond, inner):
+    """17 N of every remainder by four (rows of the Krylov basis that begin off a 16-byte boundary), and systems
+    smaller than the number of iterations allowed."""
+    pos = packed(N, 2.3, N)
+    s, p = solver(pos, precond=precond, solver_tol=1e-6, gmres_restart=60, learned_inner=inner)
+    s.precond_build(p)
+    pr = O.Problem(pos, L, 0.0, table=ewald_golden())
+    rhs = np.random.default_rng(N).standard_normal(17 * N)
+    x, it, res, st = s.saddle_solve(p, dev(rhs))
+    assert res < 1e-5
+    assert rel(x.cpu().numpy(), pr.solve(rhs)) < 1e-4
+    s.close()
