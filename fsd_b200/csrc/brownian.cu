@@ -206,14 +206,9 @@ void dot_device(fsd_handle* h, const float* a, const float* b, size_t n, double*
     k_sum_parts<<<1, 32, 0, h->stream>>>(h->w.dred, kDotBlocks, out);
 }
 
-// Lanczos three-term step: w <- (w - beta v_prev - alpha v) and alpha = v.w
-__global__ void k_axpby(float* __restrict__ y, const float* __restrict__ x, float a, size_t n) {
+__global__ void k_sum2(float* __restrict__ y, const float* __restrict__ a, const float* __restrict__ b, size_t n) {
     for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
-        y[k] += a * x[k];
-}
-__global__ void k_scale(float* __restrict__ y, const float* __restrict__ x, float a, size_t n) {
-    for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
-        y[k] = a * x[k];
+        y[k] = a[k] + b[k];
 }
 __global__ void k_lincomb(const float* __restrict__ V, size_t ld, int m, const double* __restrict__ c,
                           float* __restrict__ y, size_t n, float scale) {
@@ -298,6 +293,76 @@ static bool sqrt_T_e1(int m, const std::vector<double>& alpha, const std::vector
 }
 
 // --------------------------------------------------------------- Lanczos
+// The coefficients stay on the device, so a step is the operator and three
+// launches, and the host waits only where it tests convergence; the arithmetic
+// is that of the plain recurrence, operation for operation.  (Separate axpy,
+// dot, sum and scale launches with two host waits per step left the GPU idle
+// for half of a Brownian sample.)
+
+constexpr double kLzInvariant = 1e-8;  // a smaller beta ends the recurrence (Brownian_FarField.cu:571-579)
+
+// Sum of s over the grid (kDotBlocks blocks of 256, in the order of dot_device);
+// true in thread 0 of the last block.
+__device__ __forceinline__ bool grid_sum(double& s, double* part, unsigned* ticket) {
+    block_partial(s, part);
+    if (!last_block(ticket)) return false;
+    if (threadIdx.x >= 32) return false;
+    s = warp_sum_parts(part, gridDim.x);
+    if (threadIdx.x != 0) return false;
+    *ticket = 0;
+    return true;
+}
+
+// norm[0] = |x|.
+__global__ void __launch_bounds__(256) k_lz_norm(const float* __restrict__ x, size_t n, double* part, unsigned* ticket,
+                                                 double* norm) {
+    double s = 0.0;
+    for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
+        s += (double)x[k] * (double)x[k];
+    if (grid_sum(s, part, ticket)) norm[0] = sqrt(s);
+}
+
+// w -= beta_j v_{j-1}; alpha_j = v_j . w.
+__global__ void __launch_bounds__(256) k_lz_alpha(float* __restrict__ w, const float* __restrict__ v,
+                                                  const float* __restrict__ vprev, size_t n, int j, double* part,
+                                                  unsigned* ticket, double* alpha, const double* __restrict__ beta) {
+    const float nb = j > 0 ? (float)(-beta[j]) : 0.f;
+    double s = 0.0;
+    for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x) {
+        float t = w[k];
+        if (j > 0) {
+            t += nb * vprev[k];
+            w[k] = t;
+        }
+        s += (double)v[k] * (double)t;
+    }
+    if (grid_sum(s, part, ticket)) alpha[j] = s;
+}
+
+// w -= alpha_j v_j; beta_{j+1} = |w|.
+__global__ void __launch_bounds__(256) k_lz_beta(float* __restrict__ w, const float* __restrict__ v, size_t n, int j,
+                                                 double* part, unsigned* ticket, const double* __restrict__ alpha,
+                                                 double* beta) {
+    const float na = (float)(-alpha[j]);
+    double s = 0.0;
+    for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x) {
+        float t = w[k];
+        t += na * v[k];
+        w[k] = t;
+        s += (double)t * (double)t;
+    }
+    if (grid_sum(s, part, ticket)) beta[j + 1] = sqrt(s > 0.0 ? s : 0.0);
+}
+
+// y = x / *norm (zero past an invariant subspace; first: past a zero vector).
+__global__ void k_lz_scale(float* __restrict__ y, const float* __restrict__ x, size_t n, const double* __restrict__ norm,
+                           int first) {
+    const double b = *norm;
+    const float a = (first ? b > 0.0 : b >= kLzInvariant) ? (float)(1.0 / b) : 0.f;
+    for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
+        y[k] = a * x[k];
+}
+
 // y = ||x|| V_m sqrt(T_m) e1 ~ A^1/2 x for the operator `apply` (n = 11N or
 // 6N), starting from the carried iteration count *m_io, adding one
 // iteration at a time until the relative change of y drops below tol
@@ -312,68 +377,69 @@ int lanczos_sqrt(fsd_handle* h, size_t n, const float* x, float* y, int* m_io, f
     float* V = w.lanczos_V;
     int nb;
     vblocks(n, &nb);
-    double* hd = w.lz_host;
+    double* d_alpha = w.lz_dot;
+    double* d_beta = w.lz_dot + (mmax + 2);
+    const double* alpha = w.lz_host;
+    const double* beta = w.lz_host + (mmax + 2);  // beta[0] = |x|
     // v_1 = x / ||x||
-    dot_device(h, x, x, n, w.lz_dot);
-    FSD_CHECK_CUDA(cudaMemcpyAsync(hd, w.lz_dot, sizeof(double), cudaMemcpyDeviceToHost, st));
-    FSD_CHECK_CUDA(cudaStreamSynchronize(st));
-    const double xnorm = sqrt(hd[0]);
+    count_launch();
+    k_lz_norm<<<kDotBlocks, 256, 0, st>>>(x, n, w.dred, w.ticket, d_beta);
+    count_launch();
+    k_lz_scale<<<nb, 256, 0, st>>>(V, x, n, d_beta, 1);
+    int done = 0;  // steps enqueued
+    auto steps_to = [&](int k) -> int {
+        for (; done < k; ++done) {
+            float* v = V + (size_t)done * n;
+            float* next = v + n;
+            const int e = apply(v, next);
+            if (e != FSD_OK) return e;
+            ProfRegion pl(h, R_LANCZOS);
+            count_launch();
+            k_lz_alpha<<<kDotBlocks, 256, 0, st>>>(next, v, done > 0 ? v - n : nullptr, n, done, w.dred, w.ticket,
+                                                   d_alpha, d_beta);
+            count_launch();
+            k_lz_beta<<<kDotBlocks, 256, 0, st>>>(next, v, n, done, w.dred, w.ticket, d_alpha, d_beta);
+            count_launch();
+            k_lz_scale<<<nb, 256, 0, st>>>(next, next, n, d_beta + done + 1, 0);
+        }
+        FSD_CHECK_CUDA(cudaMemcpyAsync(w.lz_host, w.lz_dot, sizeof(double) * 2 * (mmax + 2), cudaMemcpyDeviceToHost, st));
+        FSD_CHECK_CUDA(cudaStreamSynchronize(st));
+        return FSD_OK;
+    };
+    // z = sqrt(T_k) e1 from the first k coefficients
+    auto coords = [&](int k, std::vector<double>& z) {
+        return sqrt_T_e1(k, std::vector<double>(alpha, alpha + k), std::vector<double>(beta, beta + k + 1), z);
+    };
+    // the first k of the steps so far before an invariant subspace
+    auto usable = [&](int k, bool* stop) {
+        for (int j = 0; j < k; ++j)
+            if (beta[j + 1] < kLzInvariant) {
+                *stop = true;
+                return j + 1;
+            }
+        return k;
+    };
+    const int m = std::max(1, std::min(*m_io, mmax - 2));
+    int e = steps_to(m + 1);  // the first test needs two sizes
+    if (e != FSD_OK) return e;
+    const double xnorm = beta[0];
     if (!(xnorm > 0.0)) {
         FSD_CHECK_CUDA(cudaMemsetAsync(y, 0, sizeof(float) * n, st));
         if (iters) *iters = 0;
         if (err_out) *err_out = 0.f;
         return FSD_OK;
     }
-    count_launch();
-    k_scale<<<nb, 256, 0, st>>>(V, x, (float)(1.0 / xnorm), n);
-    std::vector<double> alpha, beta(1, 0.0), z, zprev;
-    int m = std::max(1, std::min(*m_io, mmax - 2));
-    double err = 1.0;
     bool stop = false;
-    int k = 0;
-    auto step = [&](int j) -> int {
-        // w = A v_j - beta_j v_{j-1}; alpha_j = v_j.w; w -= alpha_j v_j; beta_{j+1} = ||w||
-        float* vj = V + (size_t)j * n;
-        float* wv = V + (size_t)(j + 1) * n;
-        int e = apply(vj, wv);
-        if (e != FSD_OK) return e;
-        ProfRegion pl(h, R_LANCZOS);
-        if (j > 0) {
-            count_launch();
-            count_launch();
-            k_axpby<<<nb, 256, 0, st>>>(wv, V + (size_t)(j - 1) * n, (float)(-beta[j]), n);
-        }
-        dot_device(h, vj, wv, n, w.lz_dot);
-        FSD_CHECK_CUDA(cudaMemcpyAsync(hd, w.lz_dot, sizeof(double), cudaMemcpyDeviceToHost, st));
-        FSD_CHECK_CUDA(cudaStreamSynchronize(st));
-        const double a = hd[0];
-        alpha.push_back(a);
-        count_launch();
-        k_axpby<<<nb, 256, 0, st>>>(wv, vj, (float)(-a), n);
-        dot_device(h, wv, wv, n, w.lz_dot);
-        FSD_CHECK_CUDA(cudaMemcpyAsync(hd, w.lz_dot, sizeof(double), cudaMemcpyDeviceToHost, st));
-        FSD_CHECK_CUDA(cudaStreamSynchronize(st));
-        const double b = sqrt(std::max(hd[0], 0.0));
-        beta.push_back(b);
-        if (b < 1e-8) {
-            stop = true;  // invariant subspace (Brownian_FarField.cu:571-579)
-        } else {
-            count_launch();
-            k_scale<<<nb, 256, 0, st>>>(wv, wv, (float)(1.0 / b), n);
-        }
-        return FSD_OK;
-    };
-    for (k = 0; k < m && !stop; ++k) {
-        int e = step(k);
-        if (e != FSD_OK) return e;
-    }
-    if (!sqrt_T_e1(k, alpha, beta, zprev)) return FSD_ERR_BREAKDOWN;
+    int k = usable(m, &stop);
+    std::vector<double> z, zprev;
+    if (!coords(k, zprev)) return FSD_ERR_BREAKDOWN;
     z = zprev;
+    double err = 1.0;
     while (!stop && err > tol && k < mmax - 1) {
-        int e = step(k);
+        e = steps_to(k + 1);
         if (e != FSD_OK) return e;
-        ++k;
-        if (!sqrt_T_e1(k, alpha, beta, z)) return FSD_ERR_BREAKDOWN;
+        k = usable(k + 1, &stop);
+        if (!coords(k, z)) return FSD_ERR_BREAKDOWN;
         double dn = 0.0, yn = 0.0;
         for (int i = 0; i < k; ++i) {
             const double d = z[i] - (i < (int)zprev.size() ? zprev[i] : 0.0);
@@ -431,9 +497,7 @@ int brownian_farfield(fsd_handle* h, const float4* pos, uint32_t step, float* ou
     if (st != FSD_OK && st != FSD_ERR_LANCZOS_MAXIT) return st;
     // out = wave + real
     count_launch();
-    k_scale<<<(int)std::min<size_t>(4 * 148, (n + 255) / 256), 256, 0, h->stream>>>(out11, w.lz_c, 1.0f, n);
-    count_launch();
-    k_axpby<<<(int)std::min<size_t>(4 * 148, (n + 255) / 256), 256, 0, h->stream>>>(out11, w.lz_b, 1.0f, n);
+    k_sum2<<<(int)std::min<size_t>(4 * 148, (n + 255) / 256), 256, 0, h->stream>>>(out11, w.lz_c, w.lz_b, n);
     FSD_CHECK_CUDA(cudaGetLastError());
     return st;
 }

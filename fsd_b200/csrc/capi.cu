@@ -131,8 +131,9 @@ static int allocate(fsd_handle* h) {
     FSD_TRY(dalloc(&w.lz_a, 11 * (size_t)N));
     FSD_TRY(dalloc(&w.lz_b, 11 * (size_t)N));
     FSD_TRY(dalloc(&w.lz_c, 11 * (size_t)N));
-    FSD_TRY(dalloc(&w.lz_dot, 4096));
-    FSD_CHECK_CUDA(cudaMallocHost(&w.lz_host, sizeof(double) * 4096));
+    const size_t nlz = 2 * ((size_t)h->p.lanczos_max + 2);
+    FSD_TRY(dalloc(&w.lz_dot, nlz));
+    FSD_CHECK_CUDA(cudaMallocHost(&w.lz_host, sizeof(double) * nlz));
     FSD_CHECK_CUDA(cudaMemsetAsync(w.sol, 0, sizeof(float) * n17, h->stream));
     if (h->p.integrator == 1) {
         FSD_TRY(dalloc(&w.rk_pos, N));

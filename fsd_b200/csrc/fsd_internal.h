@@ -135,8 +135,8 @@ struct Workspace {
     float* lz_a = nullptr;         // 11N work vectors
     float* lz_b = nullptr;
     float* lz_c = nullptr;
-    double* lz_dot = nullptr;      // device dot results
-    double* lz_host = nullptr;     // pinned host copies
+    double* lz_dot = nullptr;      // Lanczos coefficients: alpha, then the basis norms
+    double* lz_host = nullptr;     // pinned host copy
     // two-stage Runge-Kutta (integrator = 1 only)
     float4* rk_pos = nullptr;      // predictor positions, unwrapped
     float4* rk_posw = nullptr;     // predictor positions wrapped into the box (velocity evaluation)
