@@ -1,0 +1,146 @@
+// Products of the learned preconditioner's inner polynomial (and of the
+// approximate inverse applied once), each fused with the step around it, and
+// the copies of G and A that all row products read (fsd_bsr.cuh).
+#include "fsd_bsr.cuh"
+#include "fsd_device.cuh"
+#include "fsd_kernels.cuh"
+#include "fsd_learned.h"
+#include "fsd_solver.h"
+
+namespace fsd {
+
+// Row i of the blocks at src (block CSR, or padded rows of kPrunedCap blocks
+// when pn is given) by components at the same offset of dst.
+__global__ void __launch_bounds__(256) k_bsr_layout(const int* __restrict__ rowptr, const unsigned* __restrict__ pn, int N,
+                                                    const float* __restrict__ src, float* __restrict__ dst) {
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (i >= N) return;
+    const size_t e0 = pn ? (size_t)i * kPrunedCap : (size_t)rowptr[i];
+    const int n = pn ? (int)pn[i] : rowptr[i + 1] - rowptr[i];
+    src += 36 * e0;
+    dst += 36 * e0;
+    for (int t = threadIdx.x & 31; t < 36 * n; t += 32) {
+        const int r = t / (6 * n), k = t - r * 6 * n, e = k / 6, c = k - 6 * e;
+        dst[t] = src[36 * e + 6 * r + c];
+    }
+}
+
+// Brings the copies up to date with G and A.
+int bsr_sync(fsd_handle* h) {
+    LearnedState* s = learned(h);
+    const int N = h->p.N, grid = (N + 7) / 8;
+    if (s->g_dirty) {
+        if (!s->g_comp) FSD_CHECK_CUDA(cudaMalloc(&s->g_comp, sizeof(float) * 36 * (size_t)s->g_cap));
+        count_launch();
+        k_bsr_layout<<<grid, 256, 0, h->stream>>>(s->g_rowptr, nullptr, N, s->g_val, s->g_comp);
+        s->g_dirty = false;
+    }
+    if (s->a_dirty && s->a_blocks) {
+        if (!s->a_comp) FSD_CHECK_CUDA(cudaMalloc(&s->a_comp, sizeof(float) * 36 * (size_t)N * kPrunedCap));
+        count_launch();
+        k_bsr_layout<<<grid, 256, 0, h->stream>>>(nullptr, s->a_pn, N, s->a_blocks, s->a_comp);
+        s->a_dirty = false;
+    }
+    FSD_CHECK_CUDA(cudaGetLastError());
+    return FSD_OK;
+}
+
+// Modes: kBsrFirst = first product of the Clenshaw recurrence (operand
+// t = b[0:6N] - b[11N:17N], writes T = t, B = c_{k-1} t, out = c_{k-1} G t);
+// kBsrPlain = plain product out = M x; kBsrLast = last product y = G v with
+// the saddle post step into xs; kBsrStep = Clenshaw step
+// out = c_m T + f ((2/lambda) A u - B1) - B2; kBsrOnce = y = G t with the
+// saddle pre and post steps (xs must not overlap b).
+template <int MODE>
+__global__ void __launch_bounds__(256) k_bsr_rows(BsrArgs a) {
+    const int N = a.N;
+    const int q = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kBsrRows + bsr_sub();
+    const bool have = q < N;
+    const int i = have ? q : 0;
+    const size_t offU = 11 * (size_t)N;
+    const int r = have ? bsr_component() : -1;
+    const size_t i6 = 6 * (size_t)i + (r < 0 ? 0 : r);
+    // the row's epilogue operands, loaded before the product
+    float e_a = 0.f, e_b = 0.f, e_c = 0.f;
+    if (r >= 0) {
+        if (MODE == kBsrFirst) {
+            e_a = a.x[i6];
+            e_b = a.x[offU + i6];
+        } else if (MODE == kBsrLast || MODE == kBsrOnce) {
+            e_a = a.b[i6];
+        } else if (MODE == kBsrStep) {
+            e_a = a.T[i6];
+            e_b = a.B1[i6];
+            e_c = a.B2 ? a.B2[i6] : 0.f;
+        }
+    }
+    const float* row;
+    const int* cols;
+    int n;
+    if (MODE == kBsrStep) {  // A: padded rows of the pruned list
+        row = a.val + 36 * (size_t)i * kPrunedCap;
+        cols = a.col + (size_t)i * kPrunedCap;
+        n = have ? (int)a.pn[i] : 0;
+    } else {
+        const int q0 = a.rowptr[i];
+        row = a.val + 36 * (size_t)q0;
+        cols = a.col + q0;
+        n = have ? a.rowptr[i + 1] - q0 : 0;
+    }
+    float acc;
+    if constexpr (MODE == kBsrFirst || MODE == kBsrOnce)
+        acc = bsr_row(row, cols, n, BsrSaddle{MODE == kBsrFirst ? a.x : a.b, offU});
+    else
+        acc = bsr_row(row, cols, n, BsrPlain{a.x});
+    if (MODE == kBsrLast || MODE == kBsrOnce) {
+        if (r >= 0 && r < 5) {
+            const size_t q5 = 6 * (size_t)N + 5 * (size_t)i + r;
+            a.xs[q5] = a.b[q5];
+        }
+    }
+    if (r < 0) return;
+    if (MODE == kBsrFirst) {
+        const float c = a.pc[a.k - 1];
+        const float tv = e_a - e_b;
+        a.T[i6] = tv;
+        a.B[i6] = c * tv;
+        a.out[i6] = c * acc;
+    } else if (MODE == kBsrPlain) {
+        a.out[i6] = acc;
+    } else if (MODE == kBsrLast || MODE == kBsrOnce) {
+        a.xs[i6] = e_a - acc;
+        a.xs[offU + i6] = acc;
+    } else {
+        const float s2 = 2.0f / a.pc[kMaxPoly];
+        const float f = a.m >= 1 ? 2.0f : 1.0f;
+        float v = fmaf(a.pc[a.m], e_a, f * fmaf(s2, acc, -e_b));
+        if (a.B2) v -= e_c;
+        a.out[i6] = v;
+    }
+}
+
+// Kernel entry of a mode (for launches and graph-node updates).
+const void* bsr_kernel(int mode) {
+    switch (mode) {
+        case kBsrFirst: return (const void*)k_bsr_rows<kBsrFirst>;
+        case kBsrPlain: return (const void*)k_bsr_rows<kBsrPlain>;
+        case kBsrLast: return (const void*)k_bsr_rows<kBsrLast>;
+        case kBsrStep: return (const void*)k_bsr_rows<kBsrStep>;
+        default: return (const void*)k_bsr_rows<kBsrOnce>;
+    }
+}
+
+int bsr_blocks(int N) { return (N + 8 * kBsrRows - 1) / (8 * kBsrRows); }
+
+void bsr_launch(int mode, const BsrArgs& a, cudaStream_t st) {
+    const int grid = bsr_blocks(a.N);
+    switch (mode) {
+        case kBsrFirst: k_bsr_rows<kBsrFirst><<<grid, 256, 0, st>>>(a); break;
+        case kBsrPlain: k_bsr_rows<kBsrPlain><<<grid, 256, 0, st>>>(a); break;
+        case kBsrLast: k_bsr_rows<kBsrLast><<<grid, 256, 0, st>>>(a); break;
+        case kBsrStep: k_bsr_rows<kBsrStep><<<grid, 256, 0, st>>>(a); break;
+        default: k_bsr_rows<kBsrOnce><<<grid, 256, 0, st>>>(a); break;
+    }
+}
+
+}  // namespace fsd

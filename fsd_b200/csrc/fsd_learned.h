@@ -7,20 +7,19 @@
 
 namespace fsd {
 
-// Block-CSR products with the matrix tile streamed by bulk copies (bsr_tma.cu).
-constexpr int kTileBlocks = 104;  // blocks (and rows) of a tile of the block-sparse products
-constexpr int kBsrThreads = 128;  // threads per tile
-struct BsrTmaArgs {
+// Fused block-sparse products (bsr_rows.cu) on the copies of G (block
+// CSR, rowptr) and A (padded pruned-list rows, pn) that fsd_bsr.cuh lays out.
+enum { kBsrFirst = 0, kBsrPlain = 1, kBsrLast = 2, kBsrStep = 3, kBsrOnce = 4 };
+struct BsrArgs {
     const int* rowptr;
+    const unsigned* pn;
     const int* col;
     const float* val;
-    const int* tile_row;  // ntiles + 1 row boundaries
-    const int* ntiles;    // device count (launches cover the capacity)
     int N;
-    const float* x;       // operand (mode 0: the saddle vector b)
-    const float* b;       // mode 2: saddle input for the post step
+    const float* x;       // operand (kBsrFirst: the saddle vector b)
+    const float* b;       // kBsrLast, kBsrOnce: saddle input
     float* out;
-    float* xs;            // mode 2: saddle output
+    float* xs;            // kBsrLast, kBsrOnce: saddle output
     float* T;
     float* B;
     const float* B1;
@@ -28,15 +27,10 @@ struct BsrTmaArgs {
     const float* pc;      // coefficients, spectral bound at kMaxPoly
     int m, k;
 };
-size_t bsr_tma_smem();
-const void* bsr_tma_kernel(int mode);
-int bsr_tma_prepare();
-void bsr_tma_launch(int mode, const BsrTmaArgs& a, int grid, cudaStream_t st);
-int bsr_tma_error();
-int bsr_make_tiles(const std::vector<int>& rowptr, int N, std::vector<int>& tiles);
-__global__ void k_compact_pruned(const unsigned* __restrict__ pn, const unsigned* __restrict__ plist,
-                                 const float* __restrict__ A, const int* __restrict__ rowptr, int N, int* col,
-                                 float* val);
+const void* bsr_kernel(int mode);
+int bsr_blocks(int N);
+void bsr_launch(int mode, const BsrArgs& a, cudaStream_t st);
+int bsr_sync(fsd_handle* h);
 
 struct LearnedState {
     // G in block-CSR over particles (original order), 6x6 row-major fp32 blocks
@@ -49,6 +43,11 @@ struct LearnedState {
     const unsigned* a_pn = nullptr;
     const unsigned* a_plist = nullptr;
     const float* a_blocks = nullptr;
+    // copies for the row products (fsd_bsr.cuh), rewritten before the next
+    // application after G or A changed
+    float* g_comp = nullptr;
+    float* a_comp = nullptr;
+    bool g_dirty = true, a_dirty = true;
     // inner GMRES work space
     int inner_cap = -1;
     float* Vi = nullptr;      // (kMaxInner + 1) x 6N basis, unnormalised
@@ -94,14 +93,6 @@ struct LearnedState {
     cudaGraphNode_t pnode_first = nullptr, pnode_last = nullptr;
     const void* pkey[10] = {};
     int pkey_k = -1;
-    // block-CSR copy of A and the row tiles of A and G for the streamed products
-    int* a_rowptr = nullptr;
-    int* a_col = nullptr;
-    float* a_val = nullptr;
-    size_t a_cap = 0;
-    int* g_tiles = nullptr;   // tile_cap + 1 row boundaries, then the count at [tile_cap + 1]
-    int* a_tiles = nullptr;
-    int tile_cap = 0;
 };
 
 LearnedState* learned(fsd_handle* h);
@@ -124,7 +115,6 @@ int poly_set_coefficients(fsd_handle* h, const float* host_c, int k);
 int poly_get_coefficients(fsd_handle* h, float* host_c, int n);
 void poly_interval_coefficients(double rho, double lambda, int k, float* c);
 int poly_set_interval(fsd_handle* h, double rho);
-int poly_prepare_products(fsd_handle* h);
 
 // mpnn.cu
 void mpnn_free(fsd_handle* h);

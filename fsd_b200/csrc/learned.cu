@@ -15,6 +15,7 @@
 #include <cstring>
 #include <vector>
 
+#include "fsd_bsr.cuh"
 #include "fsd_device.cuh"
 #include "fsd_kernels.cuh"
 #include "fsd_learned.h"
@@ -32,7 +33,7 @@ void learned_free(fsd_handle* h) {
     LearnedState* s = (LearnedState*)h->learned;
     if (!s) return;
     mpnn_free(h);
-    void* ptrs[] = {s->g_rowptr, s->g_col,   s->g_val,     s->Vi,        s->Zi,        s->part,   s->H,
+    void* ptrs[] = {s->g_comp, s->a_comp, s->g_rowptr, s->g_col,   s->g_val,     s->Vi,        s->Zi,        s->part,   s->H,
                     s->nrm,      s->ticket,  s->sp_sets,   s->sp_size,   s->sp_rowptr, s->sp_scan, s->sp_bucket,
                     s->sp_cnt};
     for (void* p : ptrs)
@@ -51,11 +52,13 @@ int learned_reserve(fsd_handle* h, int nnzb) {
     LearnedState* s = learned(h);
     const int N = h->p.N;
     if (!s->g_rowptr) FSD_CHECK_CUDA(cudaMalloc(&s->g_rowptr, sizeof(int) * (N + 1)));
-    if (nnzb + 8 > s->g_cap) {  // headroom: the streamed products read column indices up to three past the end
+    if (nnzb + 8 > s->g_cap) {
         if (s->g_col) cudaFree(s->g_col);
         if (s->g_val) cudaFree(s->g_val);
+        if (s->g_comp) cudaFree(s->g_comp);
         s->g_col = nullptr;
         s->g_val = nullptr;
+        s->g_comp = nullptr;
         s->g_cap = 0;
         // headroom, so that pattern growth from step to step rarely reallocates
         const int cap = nnzb + nnzb / 8 + 1024;
@@ -93,38 +96,9 @@ int learned_set_blocks(fsd_handle* h, int nnzb, const int* d_rowptr, const int* 
                                        h->stream));
     }
     s->g_nnzb = nnzb;
+    s->g_dirty = true;
     s->g_user = true;
     return FSD_OK;
-}
-
-// x = P^-1 b with y = G t, t_i = b[6i:6i+6] - b[11N+6i:11N+6i+6]:
-// x[6i:6i+6] = b[6i:6i+6] - y_i, x[6N:11N] = b[6N:11N], x[11N+6i:...] = y_i.
-// Eight lanes per particle row; lane r < 6 owns output component r.
-__global__ void __launch_bounds__(256) k_pc_bsr(const int* __restrict__ rowptr, const int* __restrict__ col,
-                                                const float* __restrict__ G, const float* __restrict__ b,
-                                                float* __restrict__ x, int N) {
-    const int gid = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = gid >> 3;
-    const int r = threadIdx.x & 7;
-    if (i >= N) return;  // whole groups of eight leave together
-    const unsigned gmask = 0xffu << (threadIdx.x & 24);
-    const float* bU = b + 11 * (size_t)N;
-    float acc = 0.f;
-    for (int e = rowptr[i]; e < rowptr[i + 1]; ++e) {
-        const int j = col[e];
-        const float tj = (r < 6) ? b[6 * j + r] - bU[6 * j + r] : 0.f;
-        const float* Ge = G + (size_t)e * 36 + (r < 6 ? r : 0) * 6;
-#pragma unroll
-        for (int c = 0; c < 6; ++c) {
-            const float tc = __shfl_sync(gmask, tj, c, 8);
-            if (r < 6) acc += Ge[c] * tc;
-        }
-    }
-    if (r < 6) {
-        x[6 * i + r] = b[6 * i + r] - acc;
-        x[11 * (size_t)N + 6 * i + r] = acc;
-    }
-    if (r < 5) x[6 * (size_t)N + 5 * i + r] = b[6 * (size_t)N + 5 * i + r];
 }
 
 // ----------------------------------------------------------- inner solve
@@ -523,13 +497,23 @@ int precond_apply_learned(fsd_handle* h, const float* b, float* x) {
     cudaStream_t st = h->stream;
     if (poly_active(h)) return poly_apply(h, b, x);
     const int k = h->p.learned_inner;
+    int e;
     if (k == 0) {
+        e = bsr_sync(h);  // after user-set blocks; built ones are in place
+        if (e != FSD_OK) return e;
+        BsrArgs a{};
+        a.rowptr = s->g_rowptr;
+        a.col = s->g_col;
+        a.val = s->g_comp;
+        a.N = N;
+        a.b = b;
+        a.xs = x;
         count_launch();
-        k_pc_bsr<<<(8 * N + 255) / 256, 256, 0, st>>>(s->g_rowptr, s->g_col, s->g_val, b, x, N);
+        bsr_launch(kBsrOnce, a, st);
         FSD_CHECK_CUDA(cudaGetLastError());
         return FSD_OK;
     }
-    int e = inner_graph(h, b, x);
+    e = inner_graph(h, b, x);
     if (e != FSD_OK) return e;
     e = inner_bind(h, b, x);
     if (e != FSD_OK) return e;
@@ -562,8 +546,6 @@ int precond_build_learned(fsd_handle* h, const float4* pos) {
         }
     }
     if (poly) {
-        e = poly_prepare_products(h);
-        if (e != FSD_OK) return e;
         e = poly_lambda(h);
         if (e != FSD_OK) return e;
         // Coefficients: the caller's; else the Chebyshev interval whose lower
@@ -594,6 +576,10 @@ int precond_build_learned(fsd_handle* h, const float4* pos) {
             e = mpnn_poly_calibrate(h, h->p.learned_poly, ++s->poly_builds);
             if (e != FSD_OK) return e;
         }
+    }
+    if (!poly && h->p.learned_inner == 0) {
+        e = bsr_sync(h);
+        if (e != FSD_OK) return e;
     }
     h->pc_valid = true;
     return FSD_OK;

@@ -895,6 +895,7 @@ static int mp_head(fsd_handle* h) {
     const int N = s->N;
     count_launch();
     k_head_blocks<<<(N + 127) / 128, 128, 0, h->stream>>>(s->cnt, s->rhat, s->oe, s->on, s->J, N, ls->g_val);
+    ls->g_dirty = true;
     FSD_CHECK_CUDA(cudaGetLastError());
     return FSD_OK;
 }

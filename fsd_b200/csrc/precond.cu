@@ -862,6 +862,7 @@ int precond_assemble_pruned(fsd_handle* h, const float4* pos, float relaxer, con
     *pn = ic->pn;
     *plist = ic->plist;
     *blocks = ic->blocks;
+    learned(h)->a_dirty = true;
     return FSD_OK;
 }
 

@@ -432,6 +432,7 @@ int spai_build(fsd_handle* h) {
     if (es != FSD_OK) return es;
     FSD_CHECK_CUDA(cudaGetLastError());
     s->g_nnzb = nnzb;
+    s->g_dirty = true;
     return FSD_OK;
 }
 

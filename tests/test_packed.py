@@ -134,3 +134,27 @@ def test_nearfield_sample_is_the_square_root(cuda, N):
     ref = np.sqrt(2.0) * (V @ (np.sqrt(np.maximum(w, 0.0)) * (V.T @ psi)))
     assert rel(s.brownian_nearfield(p, 4).cpu().numpy(), ref) < 1e-3
     s.close()
+
+
+@pytest.mark.parametrize("N", [1, 2, 15, 17, 33])
+def test_products_with_user_blocks_of_any_row_length(cuda, N):
+    """G once, on rows of no block to N blocks (N > 16 lanes of operand pairs, N > 32 of blocks).  FP32 rows of at
+    most 6 N terms: 1e-6 expected."""
+    s, p = solver(packed(N, 2.3, N), precond="learned", learned_inner=0)
+    rng = np.random.default_rng(N)
+    n = np.minimum(N, np.arange(N) * 2)
+    n[-1] = N
+    rowptr = np.concatenate([[0], np.cumsum(n)]).astype(np.int32)
+    col = np.concatenate([rng.permutation(N)[:k] for k in n]).astype(np.int32)
+    blocks = rng.standard_normal((len(col), 6, 6)).astype(np.float32)
+    s.precond_set_blocks(torch.as_tensor(rowptr).cuda(), torch.as_tensor(col).cuda(), torch.as_tensor(blocks).cuda())
+    G = np.zeros((6 * N, 6 * N))
+    for i in range(N):
+        for e in range(rowptr[i], rowptr[i + 1]):
+            G[6 * i:6 * i + 6, 6 * col[e]:6 * col[e] + 6] += blocks[e]
+    b = rng.standard_normal(17 * N)
+    s.precond_build(p)
+    x = dev(b)
+    got = s.precond_apply(x).cpu().numpy()
+    assert rel(got, O.saddle_precond(b.astype(np.float32).astype(np.float64), G, N)) < 1e-5
+    s.close()
