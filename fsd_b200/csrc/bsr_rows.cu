@@ -25,8 +25,8 @@ __global__ void __launch_bounds__(256) k_bsr_layout(const int* __restrict__ rowp
     }
 }
 
-// Brings the copies up to date with G and A.
-int bsr_sync(fsd_handle* h) {
+// Brings the copies up to date with G, and with A for the polynomial.
+int bsr_sync(fsd_handle* h, bool with_a) {
     LearnedState* s = learned(h);
     const int N = h->p.N, grid = (N + 7) / 8;
     if (s->g_dirty) {
@@ -35,7 +35,7 @@ int bsr_sync(fsd_handle* h) {
         k_bsr_layout<<<grid, 256, 0, h->stream>>>(s->g_rowptr, nullptr, N, s->g_val, s->g_comp);
         s->g_dirty = false;
     }
-    if (s->a_dirty && s->a_blocks) {
+    if (with_a && s->a_dirty && s->a_blocks) {
         if (!s->a_comp) FSD_CHECK_CUDA(cudaMalloc(&s->a_comp, sizeof(float) * 36 * (size_t)N * kPrunedCap));
         count_launch();
         k_bsr_layout<<<grid, 256, 0, h->stream>>>(nullptr, s->a_pn, N, s->a_blocks, s->a_comp);

@@ -1,6 +1,5 @@
 // Block-sparse row products for the learned preconditioner (6x6 fp32 blocks):
-// two rows per warp, sixteen lanes each, on a copy of the matrix laid out by
-// components.
+// 16 or 32 lanes per row, on a copy of the matrix laid out by components.
 //
 // Row i with n blocks is 36 n contiguous floats; component r of the row's
 // result is the dot product of 6 n consecutive floats (r 6n + 6 e + c for block
@@ -12,9 +11,10 @@
 // Latency- and L2-bound: products with G and A take 5.4 and 3.2 us at N = 8000,
 // phi = 0.45.  Eight lanes per row on tiles streamed into shared memory by bulk
 // copies took 7.2 and 4.2 us (each block's lines were looked up three times), a
-// whole warp per row on this layout 5.7 and 4.2 (half its lanes idle), rows
-// padded to whole chunks of 16 pairs 5.3 and 3.4 but 32 instead of 25 us at
-// N = 32768, where the padding no longer stays in L2.
+// whole warp per row on this layout 5.7 and 4.2 (half its lanes idle).  Where
+// the matrices no longer stay in L2 the whole warp is the faster form (the
+// inner GMRES, N = 32768: 21.3 against 26.5 us with G).  Rows padded to whole
+// chunks of 16 pairs cost 32 us there.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -23,22 +23,23 @@ namespace fsd {
 
 constexpr int kBsrRows = 2;  // rows per warp
 __device__ __forceinline__ int bsr_sub() { return (threadIdx.x >> 4) & 1; }
-// Component that a row's lane returns (six of the sixteen lanes; else -1).
+// Component that a row's lane returns (six of its W lanes; else -1).
+template <int W = 16>
 __device__ __forceinline__ int bsr_component() {
-    const int l = threadIdx.x & 15;
-    return ((l & 1) == 0 && (l & 6) != 6) ? 3 * (l >> 3) + ((l >> 1) & 3) : -1;
+    const int l = threadIdx.x & (W - 1), q = l / (W / 8);
+    return l % (W / 8) == 0 && (q & 3) != 3 ? 3 * (q >> 2) + (q & 3) : -1;
 }
 
 // sum over the row's n blocks (0 for lanes without a row) of block * x_col in
-// the component lanes; row = its chunks, ld(j, k) loads operand pair k
+// the component lanes; row = its 36 n floats, ld(j, k) loads operand pair k
 // (components 2k, 2k + 1) of particle j.  All lanes of the warp take part.
-template <class LD>
+template <int W = 16, class LD>
 __device__ __forceinline__ float bsr_row(const float* __restrict__ row, const int* __restrict__ cols, int n, LD ld) {
-    const int l = threadIdx.x & 15;
+    const int l = threadIdx.x & (W - 1);
     const int np = 3 * n;  // pairs per component
     unsigned long long acc[6] = {0, 0, 0, 0, 0, 0};
     const unsigned long long* m = reinterpret_cast<const unsigned long long*>(row) + l;
-    for (int p = l; p < np; p += 16, m += 16) {
+    for (int p = l; p < np; p += W, m += W) {
         unsigned long long g[6];
 #pragma unroll
         for (int r = 0; r < 6; ++r) g[r] = __ldg(m + r * np);
@@ -58,21 +59,23 @@ __device__ __forceinline__ float bsr_row(const float* __restrict__ row, const in
         v[r] = t.x + t.y;
     }
     // halving exchanges: components 0-2 and 3-5, then {0, 1} and {2}, then 0 and 1
-    const bool h8 = l & 8, h4 = l & 4, h2 = l & 2;
+    const bool h8 = l & (W / 2), h4 = l & (W / 4), h2 = l & (W / 8);
     float a[3], b[2];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         const float keep = h8 ? v[3 + k] : v[k], send = h8 ? v[k] : v[3 + k];
-        a[k] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
+        a[k] = keep + __shfl_xor_sync(0xffffffffu, send, W / 2);
     }
     {
         const float keep = h4 ? a[2] : a[0], send = h4 ? a[0] : a[2];
-        b[0] = keep + __shfl_xor_sync(0xffffffffu, send, 4);
-        b[1] = a[1] + __shfl_xor_sync(0xffffffffu, a[1], 4);  // wanted by the lower half
+        b[0] = keep + __shfl_xor_sync(0xffffffffu, send, W / 4);
+        b[1] = a[1] + __shfl_xor_sync(0xffffffffu, a[1], W / 4);  // wanted by the lower half
     }
     const float keep = (h2 && !h4) ? b[1] : b[0], send = (h2 || h4) ? b[0] : b[1];
-    const float s = keep + __shfl_xor_sync(0xffffffffu, send, 2);
-    return s + __shfl_xor_sync(0xffffffffu, s, 1);
+    float s = keep + __shfl_xor_sync(0xffffffffu, send, W / 8);
+#pragma unroll
+    for (int o = W / 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
 }
 
 // Operand pairs of a plain 6N vector (8-byte aligned), and of the saddle

@@ -127,7 +127,13 @@ __device__ __forceinline__ bool last_block(unsigned* ticket) {
 // Sum of part[0:n] in a fixed order by one warp (same result every run).
 __device__ __forceinline__ double warp_sum_parts(const double* part, int n) {
     double s = 0.0;
-    for (int b = threadIdx.x & 31; b < n; b += 32) s += __ldcg(part + b);
+    for (int b = threadIdx.x & 31; b < n; b += 256) {  // eight loads in flight, added in the same order
+        double v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = b + 32 * k < n ? __ldcg(part + b + 32 * k) : 0.0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) s += v[k];
+    }
     return group_sum_d<32>(s);
 }
 

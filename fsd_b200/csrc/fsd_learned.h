@@ -30,7 +30,7 @@ struct BsrArgs {
 const void* bsr_kernel(int mode);
 int bsr_blocks(int N);
 void bsr_launch(int mode, const BsrArgs& a, cudaStream_t st);
-int bsr_sync(fsd_handle* h);
+int bsr_sync(fsd_handle* h, bool with_a);
 
 struct LearnedState {
     // G in block-CSR over particles (original order), 6x6 row-major fp32 blocks
@@ -50,11 +50,11 @@ struct LearnedState {
     bool g_dirty = true, a_dirty = true;
     // inner GMRES work space
     int inner_cap = -1;
-    float* Vi = nullptr;      // (kMaxInner + 1) x 6N basis, unnormalised
-    float* Zi = nullptr;      // kMaxInner x 6N, Z_j = G V_j / |V_j|
+    float* Vi = nullptr;      // kMaxInner x 6N basis U_j, unnormalised, then A z of the current step
+    float* Zi = nullptr;      // kMaxInner x 6N, Z_j = G U_j
     double* part = nullptr;   // (kMaxInner + 1) x blocks partial sums
     double* H = nullptr;      // (kMaxInner + 1) x kMaxInner Hessenberg, column-major by step, beta, y
-    double* nrm = nullptr;    // kMaxInner + 1 basis norms
+    double* nrm = nullptr;    // kMaxInner basis norms
     unsigned* ticket = nullptr;  // last-block counter, zero between kernels
     void* mp = nullptr;      // message-passing network state (mpnn.cu)
     // two-hop sparse approximate inverse (spai.cu)

@@ -106,6 +106,25 @@ int learned_set_blocks(fsd_handle* h, int nnzb, const int* d_rowptr, const int* 
 // to 1e-3), and fp16 copies, even scaled per block, raised the outer
 // iteration counts by a quarter.
 
+// k steps of GMRES on A, right-preconditioned by G.  The basis U_j is kept
+// unnormalised with |U_j| in nrm[j], and Z_j = G U_j:
+//   k_inner_g (step j): Z_j, and |U_j| by the last block; the first step forms
+//       U_0 from the right-hand side in its gathers;
+//   k_inner_a: w = A Z_j / |U_j| and its dots with U_0..U_j;
+//   k_inner_orth: U_{j+1} = w less its parts along U_0..U_j, or at the last
+//   step k_inner_last: only the norm of that, and the least-squares solution.
+// Launch- and latency-bound below some thousand particles; G and A (78 MB
+// between them) do not both stay in L2 at N = 32768.  Taking the norm beside
+// the product instead of at the end of the orthogonalisation leaves that a map
+// without a reduction, 7.0 -> 2.9 us at N = 32768, and the first right-hand
+// side needs no kernel.  Eight lanes per row suit the plain rows of A (15.9 us;
+// 18.3 with a warp per row by components).
+//
+// Slower or less accurate: the orthogonalisation inside the product (by
+// linearity, Z_j = G w - sum c_q Z_q; the application's error against 64 bits
+// grew by a quarter); every second product over the rows in descending order,
+// so as to meet what L2 still holds (25 -> 38 us).
+
 // Row r of a 6x6 fp32 block times x, summed over a group of eight lanes
 // (lane c < 6 holds x_c in xj).
 __device__ __forceinline__ float block_row(const float* blk, int rr, float xj, unsigned gmask) {
@@ -120,68 +139,51 @@ __device__ __forceinline__ float block_row(const float* blk, int rr, float xj, u
     return sum;
 }
 
-// z = G (u / |u|) in block CSR, |u| read from the device (zero gives zero).
-// Eight lanes per particle row; lane r < 6 owns output component r.
-__global__ void __launch_bounds__(256) k_bsr_spmv_n(const int* __restrict__ rowptr, const int* __restrict__ col,
-                                                    const float* __restrict__ G, const float* __restrict__ u,
-                                                    const double* __restrict__ unrm, float* __restrict__ z, int N) {
-    const int gid = blockIdx.x * blockDim.x + threadIdx.x;
-    const int r = threadIdx.x & 7;
-    const int i = gid >> 3;  // rows in storage order: the kernel streams G
-    if (i >= N) return;      // whole groups of eight leave together
-    const unsigned gmask = 0xffu << (threadIdx.x & 24);
-    const int rr = r < 6 ? r : 0;
-    float acc = 0.f;
-    const int e1 = rowptr[i + 1];
-    int e = rowptr[i];
-    for (; e + 3 < e1; e += 4) {  // four blocks in flight per lane
-        const int j0 = col[e], j1 = col[e + 1], j2 = col[e + 2], j3 = col[e + 3];
-        const float x0 = (r < 6) ? u[6 * j0 + r] : 0.f, x1 = (r < 6) ? u[6 * j1 + r] : 0.f;
-        const float x2 = (r < 6) ? u[6 * j2 + r] : 0.f, x3 = (r < 6) ? u[6 * j3 + r] : 0.f;
-        const float* Ge = G + (size_t)e * 36;
-        acc += block_row(Ge, rr, x0, gmask);
-        acc += block_row(Ge + 36, rr, x1, gmask);
-        acc += block_row(Ge + 72, rr, x2, gmask);
-        acc += block_row(Ge + 108, rr, x3, gmask);
-    }
-    for (; e < e1; ++e) {
-        const int j = col[e];
-        const float xj = (r < 6) ? u[6 * j + r] : 0.f;
-        acc += block_row(G + (size_t)e * 36, rr, xj, gmask);
-    }
-    const double nv = *unrm;
-    const float f = nv > 0.0 ? (float)(1.0 / nv) : 0.f;
-    if (r < 6) z[6 * i + r] = f * acc;
-}
-
 constexpr int kInnerBlocks = 296;
+constexpr int kInnerRowBlocks = 4 * 148;  // at most: every block resident, its rows strided over the warps
 constexpr int kInnerThreads = 256;
+constexpr int kBetaSlot = (kMaxInner + 1) * kMaxInner;  // in H: beta, then the k coefficients
 
-// u0 = b[0:6N] - b[11N:17N]; |u0| goes to nrm[0] and to H's beta slot.
-__global__ void __launch_bounds__(kInnerThreads) k_inner_rhs(const float* __restrict__ b, float* __restrict__ u0,
-                                                             int N, double* part, unsigned* ticket, double* H,
-                                                             double* nrm) {
+// Z_j = G U_j, a warp per row on G's copy by components, and |U_j|; FIRST:
+// U_0 = b[0:6N] - b[11N:17N], taken from b in the gathers too.
+template <bool FIRST>
+__global__ void __launch_bounds__(kInnerThreads, 4) k_inner_g(const int* __restrict__ rowptr, const int* __restrict__ col,
+                                                              const float* __restrict__ G, const float* __restrict__ b,
+                                                              float* U, float* __restrict__ z, int N, double* beta,
+                                                              double* nrm, double* part, unsigned* ticket) {
+    const int r = bsr_component<32>();
+    const size_t offU = 11 * (size_t)N;
     double s = 0.0;
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < 6 * N; k += gridDim.x * blockDim.x) {
-        const float v = b[k] - b[11 * (size_t)N + k];
-        u0[k] = v;
-        s += (double)v * v;
+    for (int i = (blockIdx.x * kInnerThreads + threadIdx.x) >> 5; i < N; i += (gridDim.x * kInnerThreads) >> 5) {
+        const int q0 = rowptr[i], n = rowptr[i + 1] - q0;
+        const size_t i6 = 6 * (size_t)i + (r < 0 ? 0 : r);
+        float u = 0.f, acc;
+        if (r >= 0) u = FIRST ? b[i6] - b[offU + i6] : U[i6];
+        if constexpr (FIRST)
+            acc = bsr_row<32>(G + 36 * (size_t)q0, col + q0, n, BsrSaddle{b, offU});
+        else
+            acc = bsr_row<32>(G + 36 * (size_t)q0, col + q0, n, BsrPlain{U});
+        if (r >= 0) {
+            if (FIRST) U[i6] = u;
+            z[i6] = acc;
+            s += (double)u * u;
+        }
     }
     block_partial(s, part);
     if (!last_block(ticket)) return;
     if (threadIdx.x < 32) {
         const double t = sqrt(warp_sum_parts(part, gridDim.x));
         if (threadIdx.x == 0) {
-            nrm[0] = t;
-            H[(kMaxInner + 1) * kMaxInner] = t;
+            *nrm = t;
+            *beta = t;  // H's beta slot, or the subdiagonal of the previous column
             *ticket = 0;
         }
     }
 }
 
-// w = A z over the pruned list (self included), written to the basis slot
-// U_nv, fused with the dots H[j][q] = (U_q . w) / |U_q| for q < nv = j + 1.
-__global__ void __launch_bounds__(256) k_pruned_spmv_dots(const unsigned* __restrict__ pn,
+// w = A z / |U_j| over the pruned list (self included), written to the basis
+// slot U_nv, fused with the dots H[j][q] = (U_q . w) / |U_q| for q < nv = j + 1.
+__global__ void __launch_bounds__(256) k_inner_a(const unsigned* __restrict__ pn,
                                                           const unsigned* __restrict__ plist,
                                                           const float* __restrict__ A,
                                                           const float* __restrict__ z, float* U, size_t ld, int nv,
@@ -216,6 +218,8 @@ __global__ void __launch_bounds__(256) k_pruned_spmv_dots(const unsigned* __rest
             const float xj = (r < 6) ? z[6 * jj + r] : 0.f;
             acc += block_row(A + e * 36, rr, xj, gmask);
         }
+        const double nj = nrm[j];
+        acc *= nj > 0.0 ? (float)(1.0 / nj) : 0.f;
         if (act) U[(size_t)nv * ld + 6 * i + r] = acc;
     }
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -239,101 +243,106 @@ __global__ void __launch_bounds__(256) k_pruned_spmv_dots(const unsigned* __rest
     if (threadIdx.x == 0) *ticket = 0;
 }
 
-// Least squares min || beta e1 - H y || by Givens rotations in FP64 (one
-// thread; k <= kMaxInner).  Columns after a breakdown (zero subdiagonal or
-// zero pivot) are dropped.  y is written after H's beta slot.
-__device__ void inner_lsq(double* H, int k) {
-    double R[kMaxInner + 1][kMaxInner];
-    double g[kMaxInner + 1];
-    const double beta = H[(kMaxInner + 1) * kMaxInner];
-    for (int c = 0; c < k; ++c)
-        for (int r = 0; r <= k; ++r) R[r][c] = H[(size_t)c * (kMaxInner + 1) + r];
-    for (int r = 0; r <= k; ++r) g[r] = 0.0;
+// The factors of U_q in w's orthogonalisation against nv vectors.
+__device__ __forceinline__ void inner_factors(float* cs, const double* hj, const double* nrm, int nv) {
+    if ((int)threadIdx.x < nv)
+        cs[threadIdx.x] = nrm[threadIdx.x] > 0.0 ? (float)(hj[threadIdx.x] / nrm[threadIdx.x]) : 0.f;
+    __syncthreads();
+}
+__device__ __forceinline__ float2 inner_pair(const float* U, size_t ld, int nv, const float* cs, size_t k) {
+    float2 u = *reinterpret_cast<const float2*>(U + nv * ld + k);
+#pragma unroll 6
+    for (int q = 0; q < nv; ++q) {
+        const float2 v = *reinterpret_cast<const float2*>(U + q * ld + k);
+        u.x = fmaf(-cs[q], v.x, u.x);
+        u.y = fmaf(-cs[q], v.y, u.y);
+    }
+    return u;
+}
+
+// U_nv -= sum_{q<nv} (H[j][q] / |U_q|) U_q, by pairs (ld = 6N is even).
+__global__ void __launch_bounds__(kInnerThreads) k_inner_orth(float* U, size_t ld, int nv, const double* __restrict__ hj,
+                                                              const double* __restrict__ nrm) {
+    __shared__ float cs[kMaxInner];
+    inner_factors(cs, hj, nrm, nv);
+    const size_t k = 2 * (blockIdx.x * (size_t)kInnerThreads + threadIdx.x);
+    if (k < ld) *reinterpret_cast<float2*>(U + nv * ld + k) = inner_pair(U, ld, nv, cs, k);
+}
+
+// Least squares min || beta e1 - H y || by Givens rotations in FP64, one warp:
+// lane q holds column q, every lane the rotated right-hand side.  Columns after
+// a breakdown (zero subdiagonal or zero pivot) are dropped.  The coefficients of
+// Z_q = G U_q, y_q / |U_q|, are written after H's beta slot.  (One thread on
+// arrays in local memory took 10 us.)
+template <int K>
+__device__ __forceinline__ void inner_lsq(double* H, const double* nrm) {
+    const int lane = threadIdx.x & 31;
+    double R[K + 1], g[K + 1];
+#pragma unroll
+    for (int r = 0; r <= K; ++r) {
+        R[r] = lane < K && r <= lane + 1 ? H[(size_t)lane * (kMaxInner + 1) + r] : 0.0;
+        g[r] = 0.0;
+    }
+    const double beta = H[kBetaSlot];
     g[0] = beta;
-    int used = k;
-    for (int c = 0; c < k; ++c) {
-        const double a = R[c][c], bb = R[c + 1][c];
-        const double rr = sqrt(a * a + bb * bb);
+    int used = K;
+#pragma unroll
+    for (int c = 0; c < K; ++c) {
+        if (used < K) continue;
+        const double a = __shfl_sync(0xffffffffu, R[c], c), b = __shfl_sync(0xffffffffu, R[c + 1], c);
+        const double rr = sqrt(a * a + b * b);
         if (!(rr > 1e-300 * (beta > 0 ? beta : 1.0))) {
             used = c;
-            break;
+            continue;
         }
-        const double cs = a / rr, sn = bb / rr;
-        for (int q = c; q < k; ++q) {
-            const double x0 = R[c][q], x1 = R[c + 1][q];
-            R[c][q] = cs * x0 + sn * x1;
-            R[c + 1][q] = -sn * x0 + cs * x1;
-        }
+        const double cs = a / rr, sn = b / rr;
+        const double x0 = R[c], x1 = R[c + 1];
+        R[c] = cs * x0 + sn * x1;
+        R[c + 1] = -sn * x0 + cs * x1;
         const double g0 = g[c], g1 = g[c + 1];
         g[c] = cs * g0 + sn * g1;
         g[c + 1] = -sn * g0 + cs * g1;
-        if (!(R[c + 1][c] == R[c + 1][c])) {
-            used = c;
-            break;
-        }
     }
-    double y[kMaxInner];
-    for (int c = used - 1; c >= 0; --c) {
-        double v = g[c];
-        for (int q = c + 1; q < used; ++q) v -= R[c][q] * y[q];
-        y[c] = v / R[c][c];
+    double y = 0.0;  // lane q: y_q
+#pragma unroll
+    for (int c = K - 1; c >= 0; --c) {
+        if (c >= used) continue;
+        const double yc = g[c] / __shfl_sync(0xffffffffu, R[c], c);
+        if (lane == c) y = yc;
+#pragma unroll
+        for (int r = 0; r < c; ++r) g[r] -= __shfl_sync(0xffffffffu, R[r], c) * yc;
     }
-    double* out = H + (size_t)(kMaxInner + 1) * kMaxInner + 1;
-    for (int c = 0; c < kMaxInner; ++c) out[c] = (c < used) ? y[c] : 0.0;
+    if (lane < kMaxInner) {
+        const double nq = lane < K ? nrm[lane] : 0.0;
+        H[kBetaSlot + 1 + lane] = nq > 0.0 ? y / nq : 0.0;
+    }
 }
 
-// U_nv -= sum_{q<nv} (H[j][q] / |U_q|) U_q; |U_nv| goes to nrm[nv] and to
-// H[j][nv].  With lsq_k > 0 the last block then solves the k-step least
-// squares problem.
-__global__ void __launch_bounds__(kInnerThreads) k_inner_orth(float* U, size_t ld, int nv, double* H,
-                                                              double* nrm, int j, size_t n, double* part,
-                                                              unsigned* ticket, int lsq_k) {
-    __shared__ float hc[kMaxInner + 1];
-    if (threadIdx.x < nv)
-        hc[threadIdx.x] =
-            nrm[threadIdx.x] > 0.0 ? (float)(H[(size_t)j * (kMaxInner + 1) + threadIdx.x] / nrm[threadIdx.x]) : 0.f;
-    __syncthreads();
-    float* w = U + (size_t)nv * ld;
+// The norm of U_K orthogonalised as above (not stored: nothing reads it), and
+// the K-step least squares solution by the last block.
+template <int K>
+__global__ void __launch_bounds__(kInnerThreads) k_inner_last(const float* U, size_t ld, double* H, const double* nrm,
+                                                              double* part, unsigned* ticket) {
+    __shared__ float cs[kMaxInner];
+    double* hj = H + (size_t)(K - 1) * (kMaxInner + 1);
+    inner_factors(cs, hj, nrm, K);
     double s = 0.0;
-    const size_t stride = (size_t)gridDim.x * blockDim.x;
-    if ((n & 3) == 0 && (ld & 3) == 0) {  // 16-byte aligned vectors (6N divisible by 4): float4 loads
-        float4* w4 = reinterpret_cast<float4*>(w);
-        const float4* U4 = reinterpret_cast<const float4*>(U);
-        const size_t n4 = n >> 2, ld4 = ld >> 2;
-        for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n4; k += stride) {
-            float4 acc = w4[k];
-            for (int q = 0; q < nv; ++q) {
-                const float4 u = U4[(size_t)q * ld4 + k];
-                const float c = -hc[q];
-                acc.x = fmaf(c, u.x, acc.x);
-                acc.y = fmaf(c, u.y, acc.y);
-                acc.z = fmaf(c, u.z, acc.z);
-                acc.w = fmaf(c, u.w, acc.w);
-            }
-            w4[k] = acc;
-            s += (double)acc.x * acc.x;
-            s += (double)acc.y * acc.y;
-            s += (double)acc.z * acc.z;
-            s += (double)acc.w * acc.w;
-        }
-    } else {
-        for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += stride) {
-            float acc = w[k];
-            for (int q = 0; q < nv; ++q) acc = fmaf(-hc[q], U[(size_t)q * ld + k], acc);
-            w[k] = acc;
-            s += (double)acc * acc;
-        }
+    for (size_t k = 2 * (blockIdx.x * (size_t)kInnerThreads + threadIdx.x); k < ld;
+         k += 2 * (size_t)gridDim.x * kInnerThreads) {
+        const float2 u = inner_pair(U, ld, K, cs, k);
+        s += (double)u.x * u.x;
+        s += (double)u.y * u.y;
     }
     block_partial(s, part);
     if (!last_block(ticket)) return;
     if (threadIdx.x < 32) {
         const double t = sqrt(warp_sum_parts(part, gridDim.x));
         if (threadIdx.x == 0) {
-            nrm[nv] = t;
-            H[(size_t)j * (kMaxInner + 1) + nv] = t;
-            if (lsq_k > 0) inner_lsq(H, lsq_k);
+            hj[K] = t;
             *ticket = 0;
         }
+        __syncwarp();
+        inner_lsq<K>(H, nrm);
     }
 }
 
@@ -359,7 +368,7 @@ static int inner_alloc(fsd_handle* h) {
     const size_t n6 = 6 * N;
     FSD_CHECK_CUDA(cudaMalloc(&s->Vi, sizeof(float) * n6 * (kMaxInner + 1)));
     FSD_CHECK_CUDA(cudaMalloc(&s->Zi, sizeof(float) * n6 * kMaxInner));
-    const size_t nb = std::max<size_t>(kInnerBlocks, (8 * N + 255) / 256);
+    const size_t nb = std::max<size_t>(kInnerRowBlocks, (8 * N + 255) / 256);
     FSD_CHECK_CUDA(cudaMalloc(&s->part, sizeof(double) * (kMaxInner + 1) * nb));
     FSD_CHECK_CUDA(cudaMalloc(&s->H, sizeof(double) * ((kMaxInner + 1) * kMaxInner + 1 + kMaxInner)));
     FSD_CHECK_CUDA(cudaMalloc(&s->nrm, sizeof(double) * (kMaxInner + 1)));
@@ -373,39 +382,59 @@ bool precond_is_flexible(const fsd_handle* h) {
     return h->p.precond == FSD_PRECOND_LEARNED && h->p.learned_inner > 0 && !poly_active(h);
 }
 
+// Blocks of a kernel with eight lanes per row.
+static int inner_rows(int N) { return (8 * N + kInnerThreads - 1) / kInnerThreads; }
+
+// Blocks of a kernel with a warp per row: every warp takes about the same number of rows.
+static int inner_warps(int N) {
+    const int need = (N + 7) / 8, rounds = (need + kInnerRowBlocks - 1) / kInnerRowBlocks;
+    return (need + rounds - 1) / rounds;
+}
+
+// k_inner_last of k steps.
+template <int K = 1, class... Args>
+static void launch_inner_last(int k, cudaStream_t st, Args... args) {
+    if constexpr (K <= kMaxInner) {
+        if (k == K) k_inner_last<K><<<kInnerBlocks, kInnerThreads, 0, st>>>(args...);
+        else launch_inner_last<K + 1>(k, st, args...);
+    }
+}
+
 // Kernels of one inner solve on the right-hand side b into x, enqueued on st
-// (for graph capture).  Basis U_j is kept unnormalised with |U_j| in nrm[j];
-// each kernel applies the 1/|U_j| factors it needs.
+// (for graph capture).
 static int inner_enqueue(fsd_handle* h, const float* b, float* x, cudaStream_t st) {
     LearnedState* s = learned(h);
     const int N = h->p.N;
     const int k = h->p.learned_inner;
     const size_t n6 = 6 * (size_t)N;
-    const int rows = (8 * N + 255) / 256;
-    k_inner_rhs<<<kInnerBlocks, kInnerThreads, 0, st>>>(b, s->Vi, N, s->part, s->ticket, s->H, s->nrm);
+    const int rows = inner_rows(N), warps = inner_warps(N);
+    const int pairs = (int)((n6 / 2 + kInnerThreads - 1) / kInnerThreads);
+    k_inner_g<true><<<warps, kInnerThreads, 0, st>>>(s->g_rowptr, s->g_col, s->g_comp, b, s->Vi, s->Zi, N,
+                                                    s->H + kBetaSlot, s->nrm, s->part, s->ticket);
     for (int j = 0; j < k; ++j) {
-        float* uj = s->Vi + (size_t)j * n6;
+        double* hj = s->H + (size_t)j * (kMaxInner + 1);
         float* zj = s->Zi + (size_t)j * n6;
-        k_bsr_spmv_n<<<rows, 256, 0, st>>>(s->g_rowptr, s->g_col, s->g_val, uj, s->nrm + j, zj, N);
-        k_pruned_spmv_dots<<<rows, 256, 0, st>>>(s->a_pn, s->a_plist, s->a_blocks, zj, s->Vi, n6, j + 1,
-                                                 s->nrm, s->part, s->ticket, s->H, j, N);
-        k_inner_orth<<<kInnerBlocks, kInnerThreads, 0, st>>>(s->Vi, n6, j + 1, s->H, s->nrm, j, n6, s->part,
-                                                             s->ticket, j == k - 1 ? k : 0);
+        k_inner_a<<<rows, kInnerThreads, 0, st>>>(s->a_pn, s->a_plist, s->a_blocks, zj, s->Vi, n6, j + 1, s->nrm,
+                                                  s->part, s->ticket, s->H, j, N);
+        if (j == k - 1) break;
+        k_inner_orth<<<pairs, kInnerThreads, 0, st>>>(s->Vi, n6, j + 1, hj, s->nrm);
+        k_inner_g<false><<<warps, kInnerThreads, 0, st>>>(s->g_rowptr, s->g_col, s->g_comp, b, s->Vi + (j + 1) * n6,
+                                                         zj + n6, N, hj + j + 1, s->nrm + j + 1, s->part, s->ticket);
     }
-    k_inner_post<<<(11 * N + 255) / 256, 256, 0, st>>>(s->Zi, n6, k, s->H + (size_t)(kMaxInner + 1) * kMaxInner + 1,
-                                                       b, x, N);
+    launch_inner_last(k, st, s->Vi, n6, s->H, s->nrm, s->part, s->ticket);
+    k_inner_post<<<(11 * N + 255) / 256, 256, 0, st>>>(s->Zi, n6, k, s->H + kBetaSlot + 1, b, x, N);
     FSD_CHECK_CUDA(cudaGetLastError());
     return FSD_OK;
 }
 
-static int inner_kernels(int k) { return 2 + 3 * k; }
+static int inner_kernels(int k) { return 3 * k + 1; }
 
 // (Re)capture the inner solve when the arrays it reads were reallocated or k
 // changed.  The first and last kernel nodes (the only ones that touch b and
 // x) are kept so that each application can point them at its own vectors.
 static int inner_graph(fsd_handle* h, const float* b, float* x) {
     LearnedState* s = learned(h);
-    const void* key[8] = {s->g_rowptr, s->g_col, s->g_val, s->a_pn, s->a_plist, s->a_blocks, s->Vi, s->Zi};
+    const void* key[8] = {s->g_rowptr, s->g_col, s->g_comp, s->a_pn, s->a_plist, s->a_blocks, s->Vi, s->Zi};
     bool same = s->gexec && s->gkey_k == h->p.learned_inner;
     for (int i = 0; i < 8 && same; ++i) same = key[i] == s->gkey[i];
     if (same) return FSD_OK;
@@ -434,7 +463,7 @@ static int inner_graph(fsd_handle* h, const float* b, float* x) {
         if (t != cudaGraphNodeTypeKernel) continue;
         cudaKernelNodeParams kp;
         FSD_CHECK_CUDA(cudaGraphKernelNodeGetParams(nd, &kp));
-        if (kp.func == (void*)k_inner_rhs) s->node_rhs = nd;
+        if (kp.func == (void*)k_inner_g<true>) s->node_rhs = nd;
         if (kp.func == (void*)k_inner_post) s->node_post = nd;
     }
     if (!s->node_rhs || !s->node_post) {
@@ -458,22 +487,19 @@ static int inner_graph(fsd_handle* h, const float* b, float* x) {
 static int inner_bind(fsd_handle* h, const float* b, float* x) {
     LearnedState* s = learned(h);
     int N = h->p.N;
-    float* u0 = s->Vi;
-    double* part = s->part;
-    unsigned* ticket = s->ticket;
-    double* H = s->H;
-    double* nrm = s->nrm;
-    void* rhs_args[] = {&b, &u0, &N, &part, &ticket, &H, &nrm};
+    size_t ld = 6 * (size_t)N;
+    double* beta = s->H + kBetaSlot;
+    void* rhs_args[] = {&s->g_rowptr, &s->g_col, &s->g_comp, &b,       &s->Vi,    &s->Zi,
+                        &N,           &beta,     &s->nrm,   &s->part, &s->ticket};
     cudaKernelNodeParams kr = {};
-    kr.func = (void*)k_inner_rhs;
-    kr.gridDim = dim3(kInnerBlocks);
+    kr.func = (void*)k_inner_g<true>;
+    kr.gridDim = dim3(inner_warps(N));
     kr.blockDim = dim3(kInnerThreads);
     kr.kernelParams = rhs_args;
     FSD_CHECK_CUDA(cudaGraphExecKernelNodeSetParams(s->gexec, s->node_rhs, &kr));
     const float* Z = s->Zi;
-    size_t ld = 6 * (size_t)N;
     int k = h->p.learned_inner;
-    const double* c = s->H + (size_t)(kMaxInner + 1) * kMaxInner + 1;
+    const double* c = s->H + kBetaSlot + 1;
     void* post_args[] = {&Z, &ld, &k, &c, &b, &x, &N};
     cudaKernelNodeParams kp = {};
     kp.func = (void*)k_inner_post;
@@ -497,10 +523,9 @@ int precond_apply_learned(fsd_handle* h, const float* b, float* x) {
     cudaStream_t st = h->stream;
     if (poly_active(h)) return poly_apply(h, b, x);
     const int k = h->p.learned_inner;
-    int e;
+    int e = bsr_sync(h, false);  // after user-set blocks; built ones are in place
+    if (e != FSD_OK) return e;
     if (k == 0) {
-        e = bsr_sync(h);  // after user-set blocks; built ones are in place
-        if (e != FSD_OK) return e;
         BsrArgs a{};
         a.rowptr = s->g_rowptr;
         a.col = s->g_col;
@@ -577,8 +602,8 @@ int precond_build_learned(fsd_handle* h, const float4* pos) {
             if (e != FSD_OK) return e;
         }
     }
-    if (!poly && h->p.learned_inner == 0) {
-        e = bsr_sync(h);
+    if (!poly) {
+        e = bsr_sync(h, false);
         if (e != FSD_OK) return e;
     }
     h->pc_valid = true;

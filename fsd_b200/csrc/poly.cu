@@ -116,7 +116,7 @@ int poly_lambda(fsd_handle* h) {
     cudaStream_t st = h->stream;
     float* W = s->pbuf;
     float* U = s->pbuf + n6;
-    const int e = bsr_sync(h);
+    const int e = bsr_sync(h, true);
     if (e != FSD_OK) return e;
     const int rows = bsr_blocks(N), arows = std::min(rows, kPowerBlocks);
     gaussian(h, W, n6, 1, kStreamGain, 1.0f);
@@ -298,7 +298,7 @@ static int poly_bind(fsd_handle* h, const float* b, float* x) {
 
 int poly_apply(fsd_handle* h, const float* b, float* x) {
     LearnedState* s = learned(h);
-    int e = bsr_sync(h);
+    int e = bsr_sync(h, true);
     if (e != FSD_OK) return e;
     e = poly_graph(h, b, x);
     if (e != FSD_OK) return e;
