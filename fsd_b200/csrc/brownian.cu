@@ -52,6 +52,7 @@ __device__ __forceinline__ float4 normal4(uint32_t key, uint32_t step, uint32_t 
 }
 
 __global__ void k_normals(float* out, size_t n, uint32_t key, uint32_t step, uint32_t stream, float scale) {
+    pdl_wait();
     const size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     if (4 * q >= n) return;
     const float4 z = normal4(key, step, stream, (uint32_t)q);
@@ -64,7 +65,7 @@ __global__ void k_normals(float* out, size_t n, uint32_t key, uint32_t step, uin
 void gaussian(fsd_handle* h, float* out, size_t n, uint32_t step, uint32_t stream, float scale) {
     const size_t nq = (n + 3) / 4;
     count_launch();
-    k_normals<<<(unsigned)((nq + 255) / 256), 256, 0, h->stream>>>(out, n, h->seed_hashed, step, stream, scale);
+    launch_pdl(k_normals, (unsigned)((nq + 255) / 256), 256, 0, h->stream, out, n, h->seed_hashed, step, stream, scale);
 }
 
 // ----------------------------------------------------- wave-space noise field
@@ -154,6 +155,7 @@ __global__ void k_noise_spectrum(float2* __restrict__ grid, const float4* __rest
 // the mirror point.
 __global__ void k_noise_half(float2* __restrict__ spec, const float4* __restrict__ gridk, int Nx, int Ny, int Nz, int zp,
                              float fac, uint32_t key, uint32_t step, uint32_t stream) {
+    pdl_wait();
     const int l = blockIdx.x * blockDim.x + threadIdx.x;
     if (l > Nz / 2) return;
     const int i = blockIdx.y / Ny, j = blockIdx.y - i * Ny;
@@ -207,11 +209,13 @@ void dot_device(fsd_handle* h, const float* a, const float* b, size_t n, double*
 }
 
 __global__ void k_sum2(float* __restrict__ y, const float* __restrict__ a, const float* __restrict__ b, size_t n) {
+    pdl_wait();
     for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
         y[k] = a[k] + b[k];
 }
 __global__ void k_lincomb(const float* __restrict__ V, size_t ld, int m, const double* __restrict__ c,
                           float* __restrict__ y, size_t n, float scale) {
+    pdl_wait();
     for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x) {
         double acc = 0.0;
         for (int i = 0; i < m; ++i) acc += c[i] * (double)V[(size_t)i * ld + k];
@@ -316,6 +320,7 @@ __device__ __forceinline__ bool grid_sum(double& s, double* part, unsigned* tick
 // norm[0] = |x|.
 __global__ void __launch_bounds__(256) k_lz_norm(const float* __restrict__ x, size_t n, double* part, unsigned* ticket,
                                                  double* norm) {
+    pdl_wait();
     double s = 0.0;
     for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
         s += (double)x[k] * (double)x[k];
@@ -326,6 +331,7 @@ __global__ void __launch_bounds__(256) k_lz_norm(const float* __restrict__ x, si
 __global__ void __launch_bounds__(256) k_lz_alpha(float* __restrict__ w, const float* __restrict__ v,
                                                   const float* __restrict__ vprev, size_t n, int j, double* part,
                                                   unsigned* ticket, double* alpha, const double* __restrict__ beta) {
+    pdl_wait();
     const float nb = j > 0 ? (float)(-beta[j]) : 0.f;
     double s = 0.0;
     for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x) {
@@ -343,6 +349,7 @@ __global__ void __launch_bounds__(256) k_lz_alpha(float* __restrict__ w, const f
 __global__ void __launch_bounds__(256) k_lz_beta(float* __restrict__ w, const float* __restrict__ v, size_t n, int j,
                                                  double* part, unsigned* ticket, const double* __restrict__ alpha,
                                                  double* beta) {
+    pdl_wait();
     const float na = (float)(-alpha[j]);
     double s = 0.0;
     for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x) {
@@ -357,6 +364,7 @@ __global__ void __launch_bounds__(256) k_lz_beta(float* __restrict__ w, const fl
 // y = x / *norm (zero past an invariant subspace; first: past a zero vector).
 __global__ void k_lz_scale(float* __restrict__ y, const float* __restrict__ x, size_t n, const double* __restrict__ norm,
                            int first) {
+    pdl_wait();
     const double b = *norm;
     const float a = (first ? b > 0.0 : b >= kLzInvariant) ? (float)(1.0 / b) : 0.f;
     for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
@@ -383,9 +391,9 @@ int lanczos_sqrt(fsd_handle* h, size_t n, const float* x, float* y, int* m_io, f
     const double* beta = w.lz_host + (mmax + 2);  // beta[0] = |x|
     // v_1 = x / ||x||
     count_launch();
-    k_lz_norm<<<kDotBlocks, 256, 0, st>>>(x, n, w.dred, w.ticket, d_beta);
+    launch_pdl(k_lz_norm, kDotBlocks, 256, 0, st, x, n, w.dred, w.ticket, d_beta);
     count_launch();
-    k_lz_scale<<<nb, 256, 0, st>>>(V, x, n, d_beta, 1);
+    launch_pdl(k_lz_scale, nb, 256, 0, st, V, x, n, d_beta, 1);
     int done = 0;  // steps enqueued
     auto steps_to = [&](int k) -> int {
         for (; done < k; ++done) {
@@ -395,12 +403,12 @@ int lanczos_sqrt(fsd_handle* h, size_t n, const float* x, float* y, int* m_io, f
             if (e != FSD_OK) return e;
             ProfRegion pl(h, R_LANCZOS);
             count_launch();
-            k_lz_alpha<<<kDotBlocks, 256, 0, st>>>(next, v, done > 0 ? v - n : nullptr, n, done, w.dred, w.ticket,
+            launch_pdl(k_lz_alpha, kDotBlocks, 256, 0, st, next, v, done > 0 ? v - n : nullptr, n, done, w.dred, w.ticket,
                                                    d_alpha, d_beta);
             count_launch();
-            k_lz_beta<<<kDotBlocks, 256, 0, st>>>(next, v, n, done, w.dred, w.ticket, d_alpha, d_beta);
+            launch_pdl(k_lz_beta, kDotBlocks, 256, 0, st, next, v, n, done, w.dred, w.ticket, d_alpha, d_beta);
             count_launch();
-            k_lz_scale<<<nb, 256, 0, st>>>(next, next, n, d_beta + done + 1, 0);
+            launch_pdl(k_lz_scale, nb, 256, 0, st, next, next, n, d_beta + done + 1, 0);
         }
         FSD_CHECK_CUDA(cudaMemcpyAsync(w.lz_host, w.lz_dot, sizeof(double) * 2 * (mmax + 2), cudaMemcpyDeviceToHost, st));
         FSD_CHECK_CUDA(cudaStreamSynchronize(st));
@@ -451,7 +459,7 @@ int lanczos_sqrt(fsd_handle* h, size_t n, const float* x, float* y, int* m_io, f
     }
     FSD_CHECK_CUDA(cudaMemcpyAsync(w.lz_dot, z.data(), sizeof(double) * k, cudaMemcpyHostToDevice, st));
     count_launch();
-    k_lincomb<<<nb, 256, 0, st>>>(V, n, k, w.lz_dot, y, n, (float)(xnorm * scale));
+    launch_pdl(k_lincomb, nb, 256, 0, st, V, n, k, w.lz_dot, y, n, (float)(xnorm * scale));
     FSD_CHECK_CUDA(cudaGetLastError());
     *m_io = std::max(1, k - 1);
     if (iters) *iters = k;
@@ -474,7 +482,7 @@ int brownian_farfield(fsd_handle* h, const float4* pos, uint32_t step, float* ou
         ProfRegion prw(h, R_BROWNIAN_WAVE);
     count_launch();
     if (w.spec)
-        k_noise_half<<<dim3((g.Nz / 2 + 32) / 32, g.Nx * g.Ny), 32, 0, h->stream>>>(
+        launch_pdl(k_noise_half, dim3((g.Nz / 2 + 32) / 32, g.Nx * g.Ny), 32, 0, h->stream, 
             w.spec, w.gridk, g.Nx, g.Ny, g.Nz, wave_zp(g.Nz), fac, h->seed_hashed, step, kStreamFFWave);
     else
         k_noise_spectrum<<<(G + 255) / 256, 256, 0, h->stream>>>(w.grid, w.gridk, g.Nx, g.Ny, g.Nz, fac,
@@ -497,7 +505,7 @@ int brownian_farfield(fsd_handle* h, const float4* pos, uint32_t step, float* ou
     if (st != FSD_OK && st != FSD_ERR_LANCZOS_MAXIT) return st;
     // out = wave + real
     count_launch();
-    k_sum2<<<(int)std::min<size_t>(4 * 148, (n + 255) / 256), 256, 0, h->stream>>>(out11, w.lz_c, w.lz_b, n);
+    launch_pdl(k_sum2, (int)std::min<size_t>(4 * 148, (n + 255) / 256), 256, 0, h->stream, out11, w.lz_c, w.lz_b, n);
     FSD_CHECK_CUDA(cudaGetLastError());
     return st;
 }

@@ -53,6 +53,7 @@ int bsr_sync(fsd_handle* h, bool with_a) {
 // saddle pre and post steps (xs must not overlap b).
 template <int MODE>
 __global__ void __launch_bounds__(256) k_bsr_rows(BsrArgs a) {
+    pdl_wait();
     const int N = a.N;
     const int q = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kBsrRows + bsr_sub();
     const bool have = q < N;
@@ -135,11 +136,11 @@ int bsr_blocks(int N) { return (N + 8 * kBsrRows - 1) / (8 * kBsrRows); }
 void bsr_launch(int mode, const BsrArgs& a, cudaStream_t st) {
     const int grid = bsr_blocks(a.N);
     switch (mode) {
-        case kBsrFirst: k_bsr_rows<kBsrFirst><<<grid, 256, 0, st>>>(a); break;
-        case kBsrPlain: k_bsr_rows<kBsrPlain><<<grid, 256, 0, st>>>(a); break;
-        case kBsrLast: k_bsr_rows<kBsrLast><<<grid, 256, 0, st>>>(a); break;
-        case kBsrStep: k_bsr_rows<kBsrStep><<<grid, 256, 0, st>>>(a); break;
-        default: k_bsr_rows<kBsrOnce><<<grid, 256, 0, st>>>(a); break;
+        case kBsrFirst: launch_pdl(k_bsr_rows<kBsrFirst>, grid, 256, 0, st, a); break;
+        case kBsrPlain: launch_pdl(k_bsr_rows<kBsrPlain>, grid, 256, 0, st, a); break;
+        case kBsrLast: launch_pdl(k_bsr_rows<kBsrLast>, grid, 256, 0, st, a); break;
+        case kBsrStep: launch_pdl(k_bsr_rows<kBsrStep>, grid, 256, 0, st, a); break;
+        default: launch_pdl(k_bsr_rows<kBsrOnce>, grid, 256, 0, st, a); break;
     }
 }
 

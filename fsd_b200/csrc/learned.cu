@@ -151,6 +151,7 @@ __global__ void __launch_bounds__(kInnerThreads, 4) k_inner_g(const int* __restr
                                                               const float* __restrict__ G, const float* __restrict__ b,
                                                               float* U, float* __restrict__ z, int N, double* beta,
                                                               double* nrm, double* part, unsigned* ticket) {
+    pdl_wait();
     const int r = bsr_component<32>();
     const size_t offU = 11 * (size_t)N;
     double s = 0.0;
@@ -189,6 +190,7 @@ __global__ void __launch_bounds__(256) k_inner_a(const unsigned* __restrict__ pn
                                                           const float* __restrict__ z, float* U, size_t ld, int nv,
                                                           const double* __restrict__ nrm, double* part,
                                                           unsigned* ticket, double* H, int j, int N) {
+    pdl_wait();
     __shared__ double sh[kMaxInner + 1][8];
     const int gid = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = gid >> 3;  // rows in storage order: the kernel streams A
@@ -263,6 +265,7 @@ __device__ __forceinline__ float2 inner_pair(const float* U, size_t ld, int nv, 
 // U_nv -= sum_{q<nv} (H[j][q] / |U_q|) U_q, by pairs (ld = 6N is even).
 __global__ void __launch_bounds__(kInnerThreads) k_inner_orth(float* U, size_t ld, int nv, const double* __restrict__ hj,
                                                               const double* __restrict__ nrm) {
+    pdl_wait();
     __shared__ float cs[kMaxInner];
     inner_factors(cs, hj, nrm, nv);
     const size_t k = 2 * (blockIdx.x * (size_t)kInnerThreads + threadIdx.x);
@@ -323,6 +326,7 @@ __device__ __forceinline__ void inner_lsq(double* H, const double* nrm) {
 template <int K>
 __global__ void __launch_bounds__(kInnerThreads) k_inner_last(const float* U, size_t ld, double* H, const double* nrm,
                                                               double* part, unsigned* ticket) {
+    pdl_wait();
     __shared__ float cs[kMaxInner];
     double* hj = H + (size_t)(K - 1) * (kMaxInner + 1);
     inner_factors(cs, hj, nrm, K);
@@ -349,6 +353,7 @@ __global__ void __launch_bounds__(kInnerThreads) k_inner_last(const float* U, si
 // x = post(b, sum_i c_i Z_i): x[0:6N] = b - y, x[6N:11N] = b, x[11N:] = y.
 __global__ void k_inner_post(const float* __restrict__ Z, size_t ld, int k, const double* __restrict__ c,
                              const float* b, float* x, int N) {
+    pdl_wait();
     const int kk = blockIdx.x * blockDim.x + threadIdx.x;
     if (kk < 6 * N) {
         float acc = 0.f;
@@ -395,7 +400,7 @@ static int inner_warps(int N) {
 template <int K = 1, class... Args>
 static void launch_inner_last(int k, cudaStream_t st, Args... args) {
     if constexpr (K <= kMaxInner) {
-        if (k == K) k_inner_last<K><<<kInnerBlocks, kInnerThreads, 0, st>>>(args...);
+        if (k == K) launch_pdl(k_inner_last<K>, kInnerBlocks, kInnerThreads, 0, st, args...);
         else launch_inner_last<K + 1>(k, st, args...);
     }
 }
@@ -409,20 +414,20 @@ static int inner_enqueue(fsd_handle* h, const float* b, float* x, cudaStream_t s
     const size_t n6 = 6 * (size_t)N;
     const int rows = inner_rows(N), warps = inner_warps(N);
     const int pairs = (int)((n6 / 2 + kInnerThreads - 1) / kInnerThreads);
-    k_inner_g<true><<<warps, kInnerThreads, 0, st>>>(s->g_rowptr, s->g_col, s->g_comp, b, s->Vi, s->Zi, N,
+    launch_pdl(k_inner_g<true>, warps, kInnerThreads, 0, st, s->g_rowptr, s->g_col, s->g_comp, b, s->Vi, s->Zi, N,
                                                     s->H + kBetaSlot, s->nrm, s->part, s->ticket);
     for (int j = 0; j < k; ++j) {
         double* hj = s->H + (size_t)j * (kMaxInner + 1);
         float* zj = s->Zi + (size_t)j * n6;
-        k_inner_a<<<rows, kInnerThreads, 0, st>>>(s->a_pn, s->a_plist, s->a_blocks, zj, s->Vi, n6, j + 1, s->nrm,
+        launch_pdl(k_inner_a, rows, kInnerThreads, 0, st, s->a_pn, s->a_plist, s->a_blocks, zj, s->Vi, n6, j + 1, s->nrm,
                                                   s->part, s->ticket, s->H, j, N);
         if (j == k - 1) break;
-        k_inner_orth<<<pairs, kInnerThreads, 0, st>>>(s->Vi, n6, j + 1, hj, s->nrm);
-        k_inner_g<false><<<warps, kInnerThreads, 0, st>>>(s->g_rowptr, s->g_col, s->g_comp, b, s->Vi + (j + 1) * n6,
+        launch_pdl(k_inner_orth, pairs, kInnerThreads, 0, st, s->Vi, n6, j + 1, hj, s->nrm);
+        launch_pdl(k_inner_g<false>, warps, kInnerThreads, 0, st, s->g_rowptr, s->g_col, s->g_comp, b, s->Vi + (j + 1) * n6,
                                                          zj + n6, N, hj + j + 1, s->nrm + j + 1, s->part, s->ticket);
     }
     launch_inner_last(k, st, s->Vi, n6, s->H, s->nrm, s->part, s->ticket);
-    k_inner_post<<<(11 * N + 255) / 256, 256, 0, st>>>(s->Zi, n6, k, s->H + kBetaSlot + 1, b, x, N);
+    launch_pdl(k_inner_post, (11 * N + 255) / 256, 256, 0, st, s->Zi, n6, k, s->H + kBetaSlot + 1, b, x, N);
     FSD_CHECK_CUDA(cudaGetLastError());
     return FSD_OK;
 }

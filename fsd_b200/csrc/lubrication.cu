@@ -123,6 +123,7 @@ __device__ __forceinline__ float3 eps_dot(float3 r, float3 v) {
 template <bool PACKED>
 __global__ void __launch_bounds__(128) k_rfu(LubArgs a, const float* __restrict__ U, float* __restrict__ out,
                                              const float* __restrict__ saddle_x) {
+    pdl_wait();
     const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / kLubGroup;
     const int gl = threadIdx.x % kLubGroup;
     const bool valid = gid < a.N;
@@ -181,6 +182,7 @@ __global__ void __launch_bounds__(128) k_rfu(LubArgs a, const float* __restrict_
 // F += R_FE : E (Lubrication_RFE_kernel, Lubrication.cu:350-608).
 __global__ void __launch_bounds__(128) k_rfe(LubArgs a, float shear_rate, const float3* ori, const float* b2mask,
                                              float B2, float* __restrict__ out) {
+    pdl_wait();
     const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / kLubGroup;
     const int gl = threadIdx.x % kLubGroup;
     const bool valid = gid < a.N;
@@ -238,6 +240,7 @@ __device__ __forceinline__ float comp(float3 v, int k) { return k == 0 ? v.x : (
 
 // S -= R_SU U (Lubrication_RSU_kernel, Lubrication.cu:650-911).
 __global__ void __launch_bounds__(128) k_rsu(LubArgs a, const float* __restrict__ U, float* __restrict__ S) {
+    pdl_wait();
     const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / kLubGroup;
     const int gl = threadIdx.x % kLubGroup;
     const bool valid = gid < a.N;
@@ -285,6 +288,7 @@ __global__ void __launch_bounds__(128) k_rsu(LubArgs a, const float* __restrict_
 // within r^2 < 16 as the reference hard-codes.
 __global__ void __launch_bounds__(128) k_rse(LubArgs a, float shear_rate, const float3* ori, const float* b2mask,
                                              float B2, float* __restrict__ S) {
+    pdl_wait();
     const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / kLubGroup;
     const int gl = threadIdx.x % kLubGroup;
     const bool valid = gid < a.N;
@@ -356,29 +360,29 @@ static int lub_blocks(int N) { return (N * kLubGroup + 127) / 128; }
 void lub_rfu(fsd_handle* h, const float4* pos, const float* U, float* F, const float* saddle_x) {
     ProfRegion pr(h, R_RFU);
     count_launch();
-    k_rfu<false><<<lub_blocks(h->p.N), 128, 0, h->stream>>>(lub_args(h, pos, h->d_res_rfu), U, F, saddle_x);
+    launch_pdl(k_rfu<false>, lub_blocks(h->p.N), 128, 0, h->stream, lub_args(h, pos, h->d_res_rfu), U, F, saddle_x);
 }
 void lub_rfu_packed(fsd_handle* h, const float4* pos, float* F, const float* saddle_x) {
     ProfRegion pr(h, R_RFU);
     count_launch();
-    k_rfu<true><<<lub_blocks(h->p.N), 128, 0, h->stream>>>(lub_args(h, pos, h->d_res_rfu), h->w.u8, F, saddle_x);
+    launch_pdl(k_rfu<true>, lub_blocks(h->p.N), 128, 0, h->stream, lub_args(h, pos, h->d_res_rfu), h->w.u8, F, saddle_x);
 }
 void lub_rfe(fsd_handle* h, const float4* pos, float shear_rate, const float3* ori, const float* b2mask, float B2,
              float* F) {
     ProfRegion pr(h, R_LUB_OTHER);
     count_launch();
-    k_rfe<<<lub_blocks(h->p.N), 128, 0, h->stream>>>(lub_args(h, pos, h->d_res_g), shear_rate, ori, b2mask, B2, F);
+    launch_pdl(k_rfe, lub_blocks(h->p.N), 128, 0, h->stream, lub_args(h, pos, h->d_res_g), shear_rate, ori, b2mask, B2, F);
 }
 void lub_rsu(fsd_handle* h, const float4* pos, const float* U, float* S) {
     ProfRegion pr(h, R_LUB_OTHER);
     count_launch();
-    k_rsu<<<lub_blocks(h->p.N), 128, 0, h->stream>>>(lub_args(h, pos, h->d_res_g), U, S);
+    launch_pdl(k_rsu, lub_blocks(h->p.N), 128, 0, h->stream, lub_args(h, pos, h->d_res_g), U, S);
 }
 void lub_rse(fsd_handle* h, const float4* pos, float shear_rate, const float3* ori, const float* b2mask, float B2,
              float* S) {
     ProfRegion pr(h, R_LUB_OTHER);
     count_launch();
-    k_rse<<<lub_blocks(h->p.N), 128, 0, h->stream>>>(lub_args(h, pos, h->d_res_m), shear_rate, ori, b2mask, B2, S);
+    launch_pdl(k_rse, lub_blocks(h->p.N), 128, 0, h->stream, lub_args(h, pos, h->d_res_m), shear_rate, ori, b2mask, B2, S);
 }
 
 }  // namespace fsd

@@ -535,6 +535,7 @@ static void fft_x_green(fsd_handle* h) {
 __global__ void k_prep(const float* __restrict__ genF, const float4* __restrict__ pos, int N, float* __restrict__ rec,
                        const unsigned* __restrict__ parts, float4* __restrict__ sorted,
                        const float* __restrict__ saddle_x, float* __restrict__ u8) {
+    pdl_wait();
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= N) return;
     const int i = parts ? (int)parts[q] : q;
@@ -594,6 +595,7 @@ __device__ __forceinline__ int3 stencil_origin(float4 p, const Box& b, int Nx, i
 __global__ void __launch_bounds__(1024) k_col_count(const float4* __restrict__ pos, int N, Box b, int Nx, int Ny, int Nz,
                                                     int P, uint2* __restrict__ part, unsigned* __restrict__ col_count,
                                                     unsigned* __restrict__ col_start, unsigned* ticket) {
+    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < N) {
         const int3 s = stencil_origin(pos[i], b, Nx, Ny, Nz, P, nullptr);
@@ -612,6 +614,7 @@ __global__ void __launch_bounds__(1024) k_col_count(const float4* __restrict__ p
 // as (z, index); the column counters go back to zero for the next call.
 __global__ void k_col_fill(const uint2* __restrict__ part, int N, const unsigned* __restrict__ col_start, int ncol,
                            unsigned* __restrict__ col_count, uint2* __restrict__ items) {
+    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < ncol) col_count[i] = 0u;
     if (i >= N) return;
@@ -625,6 +628,7 @@ __global__ void __launch_bounds__(256) k_col_sort(const float4* __restrict__ pos
                                                   int ncol, int Nz, const uint2* __restrict__ items,
                                                   unsigned* __restrict__ bin_parts, unsigned* __restrict__ bin_start,
                                                   float4* __restrict__ sorted_pos) {
+    pdl_wait();
     const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (c >= ncol) return;
@@ -652,13 +656,13 @@ int mobility_bin_particles(fsd_handle* h, const float4* pos) {
     Workspace& w = h->w;
     const int N = h->p.N, Nx = h->g.Nx, Ny = h->g.Ny, Nz = h->g.Nz, ncol = Nx * Ny;
     count_launch();
-    k_col_count<<<(N + 1023) / 1024, 1024, 0, h->stream>>>(pos, N, h->box, Nx, Ny, Nz, h->g.P, w.bin_key, w.col_count,
+    launch_pdl(k_col_count, (N + 1023) / 1024, 1024, 0, h->stream, pos, N, h->box, Nx, Ny, Nz, h->g.P, w.bin_key, w.col_count,
                                                           w.col_start, w.bin_ticket);
     count_launch();
-    k_col_fill<<<(std::max(N, ncol) + 255) / 256, 256, 0, h->stream>>>(w.bin_key, N, w.col_start, ncol, w.col_count,
+    launch_pdl(k_col_fill, (std::max(N, ncol) + 255) / 256, 256, 0, h->stream, w.bin_key, N, w.col_start, ncol, w.col_count,
                                                                       w.bin_items);
     count_launch();
-    k_col_sort<<<(ncol + 7) / 8, 256, 0, h->stream>>>(pos, w.col_start, ncol, Nz, w.bin_items, w.bin_parts, w.bin_start,
+    launch_pdl(k_col_sort, (ncol + 7) / 8, 256, 0, h->stream, pos, w.col_start, ncol, Nz, w.bin_items, w.bin_parts, w.bin_start,
                                                      w.bin_pos);
     FSD_CHECK_CUDA(cudaGetLastError());
     return FSD_OK;
@@ -845,6 +849,7 @@ __device__ __forceinline__ void spread_stage(const SpreadArgs& a, const SpreadTi
 // quarter of TX TY TZ threads.
 template <int KP>
 __global__ void __launch_bounds__(128, 5) k_spread4(SpreadArgs a) {
+    pdl_wait();
     __shared__ StagedParticle sp[kSpreadCap];
     __shared__ int so[kSpreadCap];
     __shared__ unsigned scan_sh[32];
@@ -939,6 +944,7 @@ __global__ void __launch_bounds__(128, 5) k_spread4(SpreadArgs a) {
 // Needs TX % 2 == 0, TY % 4 == 0, TZ % 4 == 0 and TX TY TZ threads.
 template <int KP>
 __global__ void __launch_bounds__(256, 4) k_spread(SpreadArgs a) {
+    pdl_wait();
     __shared__ StagedParticle sp[kSpreadCap];
     __shared__ int so[kSpreadCap];  // packed origins, contiguous for the ballot
     __shared__ unsigned scan_sh[32];
@@ -1027,6 +1033,7 @@ __global__ void __launch_bounds__(256, 4) k_spread(SpreadArgs a) {
 // of contiguous cells; for tiles that are not multiples of the warp block
 // (grids with fewer than P + 3 nodes along an axis).
 __global__ void __launch_bounds__(256, 3) k_spread_rows(SpreadArgs a) {
+    pdl_wait();
     __shared__ StagedParticle sp[kSpreadCap];
     __shared__ unsigned scan_sh[32];
     __shared__ unsigned s_total;
@@ -1215,6 +1222,7 @@ __global__ void __launch_bounds__(256) k_contract(const float4* __restrict__ pos
                                                   const float2* __restrict__ grid, int N, Box b, int Nx, int Ny,
                                                   int Nz, int Prun, float hx, float hy, float hz, float prefac,
                                                   float expfac, bool local, float* __restrict__ out) {
+    pdl_wait();
     const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (w >= N) return;
@@ -1313,6 +1321,7 @@ constexpr size_t kRealWarpThreads = 148 * 896;  // seven blocks of 128 per SM
 
 template <int GROUP>
 __global__ void __launch_bounds__(128) k_real_combine(RealArgs a) {
+    pdl_wait();
     const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / GROUP;
     const int gl = threadIdx.x % GROUP;
     const int N = a.N;
@@ -1528,21 +1537,21 @@ static void spread(fsd_handle* h) {
     const size_t seg_bytes = sizeof(unsigned) * (4 * (size_t)EX * EY + 1);
     if (per_lane == 4) {
         if (g.P == 6)
-            k_spread4<6><<<ntiles, threads / 4, seg_bytes, h->stream>>>(a);
+            launch_pdl(k_spread4<6>, ntiles, threads / 4, seg_bytes, h->stream, a);
         else if (g.P == 8)
-            k_spread4<8><<<ntiles, threads / 4, seg_bytes, h->stream>>>(a);
+            launch_pdl(k_spread4<8>, ntiles, threads / 4, seg_bytes, h->stream, a);
         else
-            k_spread4<0><<<ntiles, threads / 4, seg_bytes, h->stream>>>(a);
+            launch_pdl(k_spread4<0>, ntiles, threads / 4, seg_bytes, h->stream, a);
     } else if (blocks && !(h->tune.set && h->tune.spread_rows)) {
         if (g.P == 6)
-            k_spread<6><<<ntiles, threads, seg_bytes, h->stream>>>(a);
+            launch_pdl(k_spread<6>, ntiles, threads, seg_bytes, h->stream, a);
         else if (g.P == 8)
-            k_spread<8><<<ntiles, threads, seg_bytes, h->stream>>>(a);
+            launch_pdl(k_spread<8>, ntiles, threads, seg_bytes, h->stream, a);
         else
-            k_spread<0><<<ntiles, threads, seg_bytes, h->stream>>>(a);
+            launch_pdl(k_spread<0>, ntiles, threads, seg_bytes, h->stream, a);
     } else {
         const size_t cell_bytes = sizeof(unsigned) * (2 * (size_t)EX * EY * EZ + 1);
-        k_spread_rows<<<ntiles, threads, cell_bytes, h->stream>>>(a);
+        launch_pdl(k_spread_rows, ntiles, threads, cell_bytes, h->stream, a);
     }
 }
 
@@ -1561,10 +1570,10 @@ static void contract(fsd_handle* h, const float4* pos) {
     const unsigned grid = (unsigned)(((size_t)N * 32 + 255) / 256);
     count_launch();
     if (g.P == 6)
-        k_contract<6><<<grid, 256, 0, h->stream>>>(pos, h->w.order, h->w.grid, N, h->box, g.Nx, g.Ny, g.Nz, g.P, g.hx,
+        launch_pdl(k_contract<6>, grid, 256, 0, h->stream, pos, h->w.order, h->w.grid, N, h->box, g.Nx, g.Ny, g.Nz, g.P, g.hx,
                                                    g.hy, g.hz, quadW * prefac, expfac, local, h->w.uwave);
     else
-        k_contract<0><<<grid, 256, 0, h->stream>>>(pos, h->w.order, h->w.grid, N, h->box, g.Nx, g.Ny, g.Nz, g.P, g.hx,
+        launch_pdl(k_contract<0>, grid, 256, 0, h->stream, pos, h->w.order, h->w.grid, N, h->box, g.Nx, g.Ny, g.Nz, g.P, g.hx,
                                                    g.hy, g.hz, quadW * prefac, expfac, local, h->w.uwave);
 }
 
@@ -1613,9 +1622,9 @@ void mobility_combine(fsd_handle* h, float* genU, bool wave, bool real,
     // neighbours; a small suspension does not fill the chip that way and is
     // bound by the chain of gathers per lane, which a whole warp shortens.
     if ((size_t)N * 32 <= kRealWarpThreads)
-        k_real_combine<32><<<(N + 3) / 4, 128, 0, h->stream>>>(r);
+        launch_pdl(k_real_combine<32>, (N + 3) / 4, 128, 0, h->stream, r);
     else
-        k_real_combine<8><<<(N + 15) / 16, 128, 0, h->stream>>>(r);
+        launch_pdl(k_real_combine<8>, (N + 15) / 16, 128, 0, h->stream, r);
 }
 
 // ---------------------------------------------------------------- autotuner
@@ -1742,7 +1751,7 @@ int mobility_apply(fsd_handle* h, const float4* pos, const float* genF, float* g
         if (st != FSD_OK) return st;
     }
     count_launch();
-    k_prep<<<(N + 255) / 256, 256, 0, h->stream>>>(genF, pos, N, real ? h->w.rec : nullptr,
+    launch_pdl(k_prep, (N + 255) / 256, 256, 0, h->stream, genF, pos, N, real ? h->w.rec : nullptr,
                                                    wave ? h->w.bin_parts : nullptr, h->w.bin_force, saddle_x,
                                                    h->w.u8);
     if (wave) {

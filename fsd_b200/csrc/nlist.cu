@@ -125,6 +125,7 @@ __global__ void __launch_bounds__(1024) k_cell_count(const float4* __restrict__ 
                                                      unsigned* __restrict__ key, unsigned* __restrict__ slot,
                                                      unsigned* __restrict__ count, unsigned* __restrict__ start,
                                                      unsigned* ticket) {
+    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) {
         const int3 c = cell_of(pos[i], b, nc);
@@ -139,6 +140,7 @@ __global__ void __launch_bounds__(1024) k_cell_count(const float4* __restrict__ 
 
 __global__ void k_cell_fill(const unsigned* __restrict__ key, const unsigned* __restrict__ slot, int n,
                             const unsigned* __restrict__ start, unsigned* __restrict__ items) {
+    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) items[start[key[i]] + slot[i]] = (unsigned)i;
 }
@@ -150,6 +152,7 @@ __global__ void __launch_bounds__(256) k_cell_sort(const float4* __restrict__ po
                                                    int ncells, const unsigned* __restrict__ items,
                                                    unsigned* __restrict__ parts, unsigned* __restrict__ order,
                                                    float4* __restrict__ sorted_pos) {
+    pdl_wait();
     const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (c >= ncells) return;
@@ -176,6 +179,7 @@ __global__ void __launch_bounds__(128) k_nlist_cells(const float4* __restrict__ 
                                                      unsigned* __restrict__ nneigh, unsigned* __restrict__ nlist,
                                                      int stride, int* max_count, float sub2,
                                                      unsigned* __restrict__ sub_n, unsigned* __restrict__ sub) {
+    pdl_wait();
     const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (w >= n) return;
@@ -313,16 +317,16 @@ int build_neighbor_list(fsd_handle* h, const float4* pos, int* max_count_host) {
         const int ncells = nc.x * nc.y * nc.z;
         FSD_CHECK_CUDA(cudaMemsetAsync(w.cell_count, 0, sizeof(unsigned) * w.ncell_pad, st));
         count_launch();
-        k_cell_count<<<(n + 1023) / 1024, 1024, 0, st>>>(pos, n, h->box, nc, w.part_cell, w.part_slot, w.cell_count,
+        launch_pdl(k_cell_count, (n + 1023) / 1024, 1024, 0, st, pos, n, h->box, nc, w.part_cell, w.part_slot, w.cell_count,
                                                          w.cell_start, w.cell_count + w.ncell_pad - 1);
         count_launch();
-        k_cell_fill<<<(n + 255) / 256, 256, 0, st>>>(w.part_cell, w.part_slot, n, w.cell_start, w.cell_items);
+        launch_pdl(k_cell_fill, (n + 255) / 256, 256, 0, st, w.part_cell, w.part_slot, n, w.cell_start, w.cell_items);
         count_launch();
-        k_cell_sort<<<(ncells + 7) / 8, 256, 0, st>>>(pos, w.cell_start, ncells, w.cell_items, w.cell_parts, w.order,
+        launch_pdl(k_cell_sort, (ncells + 7) / 8, 256, 0, st, pos, w.cell_start, ncells, w.cell_items, w.cell_parts, w.order,
                                                       w.cell_pos);
         count_launch();
         const float rsub = h->p.rlub + h->p.nlist_buffer;
-        k_nlist_cells<<<(n + 3) / 4, 128, 0, st>>>(pos, n, h->box, nc, w.cell_start, w.cell_parts, w.cell_pos, rlist2,
+        launch_pdl(k_nlist_cells, (n + 3) / 4, 128, 0, st, pos, n, h->box, nc, w.cell_start, w.cell_parts, w.cell_pos, rlist2,
                                                    w.nneigh, w.nlist, w.nl_stride, w.nl_overflow, rsub * rsub,
                                                    w.lub_n, w.lub_list);
     } else {
@@ -426,14 +430,14 @@ int neighbor_list_noalloc(const float4* pos, int n, Box b, float rlist, unsigned
         FSD_CHECK_CUDA(cudaMemsetAsync(count, 0, sizeof(unsigned) * ((ncells + 15) & ~15), st));
         FSD_CHECK_CUDA(cudaMemsetAsync(ticket, 0, sizeof(unsigned), st));
         count_launch();
-        k_cell_count<<<(n + 1023) / 1024, 1024, 0, st>>>(pos, n, b, nc, key, slot, count, start, ticket);
+        launch_pdl(k_cell_count, (n + 1023) / 1024, 1024, 0, st, pos, n, b, nc, key, slot, count, start, ticket);
         unsigned* items = count;  // the counts are not needed past the scan
         count_launch();
-        k_cell_fill<<<(n + 255) / 256, 256, 0, st>>>(key, slot, n, start, items);
+        launch_pdl(k_cell_fill, (n + 255) / 256, 256, 0, st, key, slot, n, start, items);
         count_launch();
-        k_cell_sort<<<(ncells + 7) / 8, 256, 0, st>>>(pos, start, ncells, items, parts, nullptr, nullptr);
+        launch_pdl(k_cell_sort, (ncells + 7) / 8, 256, 0, st, pos, start, ncells, items, parts, nullptr, nullptr);
         count_launch();
-        k_nlist_cells<<<(n + 3) / 4, 128, 0, st>>>(pos, n, b, nc, start, parts, nullptr, rlist2, nneigh, nlist, stride,
+        launch_pdl(k_nlist_cells, (n + 3) / 4, 128, 0, st, pos, n, b, nc, start, parts, nullptr, rlist2, nneigh, nlist, stride,
                                                    max_count, 0.f, nullptr, nullptr);
     } else {
         count_launch();

@@ -89,6 +89,7 @@ __device__ __forceinline__ double block_sum_d(double v, double* sh) {
 __global__ void __launch_bounds__(kRedThreads) k_multidot(const float* __restrict__ V, size_t ld, int nv,
                                                           const float* __restrict__ w, size_t n, double* part,
                                                           const int* done) {
+    pdl_wait();
     if (done && *done) return;
     __shared__ double sh[32];
     const size_t chunk = (n + gridDim.x - 1) / gridDim.x;
@@ -104,6 +105,7 @@ __global__ void __launch_bounds__(kRedThreads) k_multidot(const float* __restric
 
 // out[i] (+)= sum_b part[i * nb + b], one warp per i.
 __global__ void k_finish_dots(const double* part, int nb, int nv, double* out, bool accumulate, const int* done) {
+    pdl_wait();
     if (done && *done) return;
     const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
@@ -117,6 +119,7 @@ __global__ void k_finish_dots(const double* part, int nb, int nv, double* out, b
 // y = sum_i c[i] V_i.
 __global__ void k_combine(const float* __restrict__ V, size_t ld, int nv, const double* __restrict__ c,
                           float* __restrict__ y, size_t n) {
+    pdl_wait();
     __shared__ float cs[kMaxRestart + 1];
     for (int i = threadIdx.x; i < nv; i += blockDim.x) cs[i] = (float)c[i];
     __syncthreads();
@@ -129,6 +132,7 @@ __global__ void k_combine(const float* __restrict__ V, size_t ld, int nv, const 
 
 __global__ void k_scale_copy(const float* __restrict__ src, float* __restrict__ dst, size_t n, const double* norm,
                              const int* done) {
+    pdl_wait();
     if (done && *done) return;
     const double nv = *norm;
     const float s = nv > 0.0 ? (float)(1.0 / sqrt(nv)) : 0.0f;
@@ -137,11 +141,13 @@ __global__ void k_scale_copy(const float* __restrict__ src, float* __restrict__ 
 }
 
 __global__ void k_residual(const float* __restrict__ b, const float* __restrict__ Ax, float* __restrict__ r, size_t n) {
+    pdl_wait();
     for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
         r[k] = b[k] - Ax[k];
 }
 
 __global__ void k_axpy(float* __restrict__ x, const float* __restrict__ u, size_t n) {
+    pdl_wait();
     for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
         x[k] += u[k];
 }
@@ -175,6 +181,7 @@ struct GmresState {
 
 // Start of a cycle: r0 norm is in dots[0].
 __global__ void k_cycle_start(GmresState* s, const double* dots, double tol, int first) {
+    pdl_wait();
     const double beta2 = dots[0];
     if (first) {
         s->total = 0;
@@ -201,6 +208,7 @@ __global__ void k_cycle_start(GmresState* s, const double* dots, double tol, int
 constexpr int kLsqThreads = (kMaxRestart + 31) / 32 * 32;
 
 __global__ void __launch_bounds__(kLsqThreads) k_lsq(GmresState* s, int apply_t) {
+    pdl_wait();
     __shared__ double y[kMaxRestart];
     const int j = s->j, i = threadIdx.x;
     double g = i < j ? s->g[i] : 0.0;
@@ -229,6 +237,7 @@ struct GmresHost {
 };
 
 __global__ void k_export(const GmresState* s, GmresHost* o) {
+    pdl_wait();
     o->j = s->j;
     o->total = s->total;
     o->done = s->done;
@@ -268,6 +277,7 @@ constexpr int kPairSlice = 32;  // float4 per warp and slice
 __global__ void __launch_bounds__(kRedThreads, 2) k_dots_pair(const float* __restrict__ V, size_t ld, int j,
                                                               const float* __restrict__ w, size_t n, double* part,
                                                               const int* done, double* out, unsigned* ticket) {
+    pdl_wait();
     if (*done) return;
     __shared__ double red[kRedThreads / 32][32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -388,6 +398,7 @@ __device__ double tentative_resid(const double* col, int c, double hsub, const d
 __global__ void __launch_bounds__(kRedThreads, 2) k_dcgs_update(float* V, size_t ld, int j, const float* __restrict__ w,
                                                              size_t n, const double* __restrict__ dots,
                                                              GmresState* s, int m, double* part, unsigned* ticket) {
+    pdl_wait();
     if (s->done) return;
     __shared__ float ca[kMaxRestart + 1], cc[kMaxRestart + 1];
     __shared__ double sh[2][32];
@@ -593,24 +604,24 @@ int saddle_solve(fsd_handle* h, const float4* pos, const float* b, float* x, flo
             int e = saddle_multiply(h, pos, x, Ax, first);
             if (e != FSD_OK) return e;
             count_launch();
-            k_residual<<<vblocks, vthreads, 0, st>>>(b, Ax, r, n);
+            launch_pdl(k_residual, vblocks, vthreads, 0, st, b, Ax, r, n);
             count_launch();
-            k_multidot<<<nbl, kRedThreads, 0, st>>>(r, n, 1, r, n, part, nullptr);
+            launch_pdl(k_multidot, nbl, kRedThreads, 0, st, r, n, 1, r, n, part, nullptr);
             count_launch();
-            k_finish_dots<<<1, 32, 0, st>>>(part, nbl, 1, dots, false, nullptr);
+            launch_pdl(k_finish_dots, 1, 32, 0, st, part, nbl, 1, dots, false, nullptr);
             if (first) {
                 count_launch();
-                k_multidot<<<nbl, kRedThreads, 0, st>>>(b, n, 1, b, n, part, nullptr);
+                launch_pdl(k_multidot, nbl, kRedThreads, 0, st, b, n, 1, b, n, part, nullptr);
                 count_launch();
-                k_finish_dots<<<1, 32, 0, st>>>(part, nbl, 1, dots + 1, false, nullptr);
+                launch_pdl(k_finish_dots, 1, 32, 0, st, part, nbl, 1, dots + 1, false, nullptr);
             }
             count_launch();
-            k_cycle_start<<<1, 1, 0, st>>>(gs, dots, (double)tol, first ? 1 : 0);
+            launch_pdl(k_cycle_start, 1, 1, 0, st, gs, dots, (double)tol, first ? 1 : 0);
             count_launch();
-            k_scale_copy<<<vblocks, vthreads, 0, st>>>(r, V, n, dots, &gs->done);
+            launch_pdl(k_scale_copy, vblocks, vthreads, 0, st, r, V, n, dots, &gs->done);
             first = false;
             count_launch();
-            k_export<<<1, 1, 0, st>>>(gs, gh);
+            launch_pdl(k_export, 1, 1, 0, st, gs, gh);
             FSD_CHECK_CUDA(cudaStreamSynchronize(st));
             const bool converged_at_start = gh->done != 0;
             for (int j = 0; j < m && !converged_at_start; ++j) {
@@ -622,23 +633,23 @@ int saddle_solve(fsd_handle* h, const float4* pos, const float* b, float* x, flo
                 if (e != FSD_OK) return e;
                 ProfRegion pk(h, R_KRYLOV);
                 count_launch();
-                k_dots_pair<<<pbl, kRedThreads, 0, st>>>(V, ld, j, Ax, n, part, &gs->done, pfinish ? dots : nullptr,
+                launch_pdl(k_dots_pair, pbl, kRedThreads, 0, st, V, ld, j, Ax, n, part, &gs->done, pfinish ? dots : nullptr,
                                                          w.ticket);
                 if (!pfinish) {
                     count_launch();
-                    k_finish_dots<<<(2 * (j + 1) + 7) / 8, 256, 0, st>>>(part, pbl, 2 * (j + 1), dots, false, &gs->done);
+                    launch_pdl(k_finish_dots, (2 * (j + 1) + 7) / 8, 256, 0, st, part, pbl, 2 * (j + 1), dots, false, &gs->done);
                 }
                 count_launch();
-                k_dcgs_update<<<ubl, kRedThreads, 0, st>>>(V, ld, j, Ax, n, dots, gs, m, part, w.ticket);
+                launch_pdl(k_dcgs_update, ubl, kRedThreads, 0, st, V, ld, j, Ax, n, dots, gs, m, part, w.ticket);
                 if ((j % 4) == 3 || j == m - 1) {
                     count_launch();
-                    k_export<<<1, 1, 0, st>>>(gs, gh);
+                    launch_pdl(k_export, 1, 1, 0, st, gs, gh);
                     FSD_CHECK_CUDA(cudaStreamSynchronize(st));
                     if (gh->done) break;
                 }
             }
             count_launch();
-            k_export<<<1, 1, 0, st>>>(gs, gh);
+            launch_pdl(k_export, 1, 1, 0, st, gs, gh);
             FSD_CHECK_CUDA(cudaStreamSynchronize(st));
             if (getenv("FSD_DEBUG_GMRES"))
                 fprintf(stderr, "gmres cycle: j=%d total=%d resid=%.3e breakdown=%d\n", gh->j, gh->total, gh->resid,
@@ -647,18 +658,18 @@ int saddle_solve(fsd_handle* h, const float4* pos, const float* b, float* x, flo
             total = gh->total;
             if (jc > 0) {
                 count_launch();
-                k_lsq<<<1, kLsqThreads, 0, st>>>(gs, flexible ? 0 : 1);
+                launch_pdl(k_lsq, 1, kLsqThreads, 0, st, gs, flexible ? 0 : 1);
                 if (flexible) {  // x += Z y
                     count_launch();
-                    k_combine<<<vblocks, vthreads, 0, st>>>(w.Z, ld, jc, gs_y(gs), z, n);
+                    launch_pdl(k_combine, vblocks, vthreads, 0, st, w.Z, ld, jc, gs_y(gs), z, n);
                 } else {  // x += M^-1 V y
                     count_launch();
-                    k_combine<<<vblocks, vthreads, 0, st>>>(V, ld, jc, gs_y(gs), Ax, n);
+                    launch_pdl(k_combine, vblocks, vthreads, 0, st, V, ld, jc, gs_y(gs), Ax, n);
                     e = precond_apply(h, Ax, z);
                     if (e != FSD_OK) return e;
                 }
                 count_launch();
-                k_axpy<<<vblocks, vthreads, 0, st>>>(x, z, n);
+                launch_pdl(k_axpy, vblocks, vthreads, 0, st, x, z, n);
             }
             if (gh->breakdown == 1) {
                 status = FSD_ERR_BREAKDOWN;
@@ -675,11 +686,11 @@ int saddle_solve(fsd_handle* h, const float4* pos, const float* b, float* x, flo
         int e = saddle_multiply(h, pos, x, Ax, false);
         if (e != FSD_OK) return e;
         count_launch();
-        k_residual<<<vblocks, vthreads, 0, st>>>(b, Ax, r, n);
+        launch_pdl(k_residual, vblocks, vthreads, 0, st, b, Ax, r, n);
         count_launch();
-        k_multidot<<<nbl, kRedThreads, 0, st>>>(r, n, 1, r, n, part, nullptr);
+        launch_pdl(k_multidot, nbl, kRedThreads, 0, st, r, n, 1, r, n, part, nullptr);
         count_launch();
-        k_finish_dots<<<1, 32, 0, st>>>(part, nbl, 1, dots, false, nullptr);
+        launch_pdl(k_finish_dots, 1, 32, 0, st, part, nbl, 1, dots, false, nullptr);
         double host[2];
         FSD_CHECK_CUDA(cudaMemcpyAsync(host, dots, sizeof(double), cudaMemcpyDeviceToHost, st));
         FSD_CHECK_CUDA(cudaMemcpyAsync(host + 1, &gs->bnorm2, sizeof(double), cudaMemcpyDeviceToHost, st));

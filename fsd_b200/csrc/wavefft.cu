@@ -110,6 +110,7 @@ __device__ __forceinline__ int row_slot(int k) {
 template <class L>
 __global__ void __launch_bounds__(Plane<L>::threads) k_yz_fwd(const float2* __restrict__ grid, float2* __restrict__ spec,
                                                               int Nx, int zp, const float2* __restrict__ tw_global) {
+    pdl_wait();
     constexpr int N = L::N;
     extern __shared__ float2 smem[];
     float2* tw = smem;
@@ -163,6 +164,7 @@ __global__ void __launch_bounds__(Plane<L>::threads) k_yz_fwd(const float2* __re
 template <class L>
 __global__ void __launch_bounds__(Plane<L>::threads) k_yz_inv(const float2* __restrict__ spec, float2* __restrict__ grid,
                                                               int Nx, int zp, const float2* __restrict__ tw_global) {
+    pdl_wait();
     constexpr int N = L::N;
     extern __shared__ float2 smem[];
     float2* tw = smem;
@@ -229,6 +231,7 @@ template <class L, bool GREEN>
 __global__ void __launch_bounds__(XPass<L>::threads, XPass<L>::blocks) k_x_pass(float2* __restrict__ spec, const float4* __restrict__ table,
                                                               const float4* __restrict__ gridk, int Ny, int Nz, int zp,
                                                               const float2* __restrict__ tw_global) {
+    pdl_wait();
     constexpr int N = L::N;
     extern __shared__ float2 smem[];
     float2* tw = smem;
@@ -423,10 +426,10 @@ static void yz(fsd_handle* h, bool inv) {
         if (!smem_limit_ok(fn, Plane<L>::smem, "plane transform shared memory")) return;
         count_launch();
         if (inv)
-            k_yz_inv<L><<<6 * g.Nx, Plane<L>::threads, Plane<L>::smem, h->stream>>>(h->w.spec, h->w.grid, g.Nx,
+            launch_pdl(k_yz_inv<L>, 6 * g.Nx, Plane<L>::threads, Plane<L>::smem, h->stream, h->w.spec, h->w.grid, g.Nx,
                                                                                    wave_zp(g.Nz), tw);
         else
-            k_yz_fwd<L><<<6 * g.Nx, Plane<L>::threads, Plane<L>::smem, h->stream>>>(h->w.grid, h->w.spec, g.Nx,
+            launch_pdl(k_yz_fwd<L>, 6 * g.Nx, Plane<L>::threads, Plane<L>::smem, h->stream, h->w.grid, h->w.spec, g.Nx,
                                                                                    wave_zp(g.Nz), tw);
     });
 }
@@ -441,10 +444,10 @@ static void x_pass(fsd_handle* h, bool green) {
         count_launch();
         const int nb = g.Ny * (zp / kXz);
         if (green)
-            k_x_pass<L, true><<<nb, XPass<L>::threads, XPass<L>::smem, h->stream>>>(
+            launch_pdl(k_x_pass<L, true>, nb, XPass<L>::threads, XPass<L>::smem, h->stream, 
                 h->w.spec, h->w.green_table, h->w.gridk, g.Ny, g.Nz, zp, h->w.twiddle);
         else
-            k_x_pass<L, false><<<nb, XPass<L>::threads, XPass<L>::smem, h->stream>>>(
+            launch_pdl(k_x_pass<L, false>, nb, XPass<L>::threads, XPass<L>::smem, h->stream, 
                 h->w.spec, h->w.green_table, h->w.gridk, g.Ny, g.Nz, zp, h->w.twiddle);
     });
 }

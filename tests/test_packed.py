@@ -158,3 +158,22 @@ def test_products_with_user_blocks_of_any_row_length(cuda, N):
     got = s.precond_apply(x).cpu().numpy()
     assert rel(got, O.saddle_precond(b.astype(np.float32).astype(np.float64), G, N)) < 1e-5
     s.close()
+
+
+@pytest.mark.parametrize("N", [8, 295, 2368, 2369, 3000])
+def test_overlapped_launches_keep_their_order(cuda, N):
+    """Chains of dependent launches on either side of the grid size up to which they overlap: the same bits in
+    every repetition, interleaved with other products, and the pair sums against the oracle."""
+    pos = packed(N, 2.2, N)
+    s, p = solver(pos)
+    rng = np.random.default_rng(N)
+    F, U = rng.standard_normal(11 * N).astype(np.float32), dev(rng.standard_normal(6 * N))
+    x = dev(rng.standard_normal(17 * N))
+    Fd = dev(F)
+    first = [s.mobility(p, Fd), s.rfu(p, U), s.saddle_multiply(p, x)]
+    for _ in range(10):
+        for a, b in zip(first, (s.mobility(p, Fd), s.rfu(p, U), s.saddle_multiply(p, x))):
+            assert torch.equal(a, b)
+    ref = O.Problem(pos, L, 0.0, table=ewald_golden()).mobility(F, parts=2)
+    assert rel(s.mobility(p, Fd, parts=2).cpu(), ref) < 1e-5
+    s.close()
