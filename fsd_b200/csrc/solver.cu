@@ -522,9 +522,7 @@ __global__ void __launch_bounds__(kRedThreads, 2) k_dcgs_update(float* V, size_t
                 s->j = j + 1;
                 const double rt = tentative_resid(ccur, j, hsub, scs, ssn, s);
                 const bool bad = !(hsub > 1e-300) || !(rt == rt);
-                // the iterate's error is some hundred times its residual, so a stop just at the tolerance
-                // is decided by rounding: a quarter below it costs an iteration at most
-                if (rt <= 0.75 * s->tol || j + 1 >= m || bad) {
+                if (rt <= s->tol || j + 1 >= m || bad) {
                     givens_column(ccur, j, hsub, scs, ssn, s);
                     if (bad) s->breakdown = (hsub > 1e-300) ? 2 : 1;
                     s->done = 1;

@@ -10,7 +10,9 @@ the two-stage Runge-Kutta integrator (Integrator.cu:232-438).
 * One Runge-Kutta step at kT = 0 with shear, a squirmer term and directors
   against the oracle's two stages and the oracle's velocities at x and at the
   predictor: displacements 1e-4, directors 1e-5, images exactly, and the
-  reported velocity (the mean of the stages) 1e-4 (GMRES to 1e-6).
+  reported velocity (the mean of the stages) 1e-4.  The velocity's error is
+  91 to 127 times the residual at which the solve stops (tolerances 3e-7 to
+  1e-6), so GMRES goes to 5e-7: 6.4e-5 at most.
 """
 from __future__ import annotations
 
@@ -88,7 +90,7 @@ def test_runge_kutta_step_matches_oracle(cuda):
     ori = rng.standard_normal((N, 3))
     ori = (ori / np.linalg.norm(ori, axis=1, keepdims=True)).astype(np.float32)
     mask = rng.random(N).astype(np.float32)
-    s = FSD(N, (Lc, Lc, Lc, xy), T=0.0, dt=dt, sqm_B1=B1, solver_tol=1e-6, gmres_max_iter=4000, precond="learned",
+    s = FSD(N, (Lc, Lc, Lc, xy), T=0.0, dt=dt, sqm_B1=B1, solver_tol=5e-7, gmres_max_iter=4000, precond="learned",
             integrator=1)
     p = torch.as_tensor(pos).cuda().view(-1).contiguous()
     o = torch.as_tensor(ori).cuda().view(-1).contiguous()
