@@ -181,7 +181,8 @@ struct TuneChoice {
     int TX = 0, TY = 0, TZ = 0;  // spreading tile
     int Bxy = 0, Bz = 0;         // FFT lines per block (x/y passes, z pass)
     int Bg = 0;                  // z-run length of the fused x-pass + Green kernel
-    int spread_rows = 0;         // 1: one node per thread walking stencil rows; 0: warp node blocks
+    int spread_rows = 0;         // spreading form: 0 warp node blocks, one node per lane; 1 one node per thread,
+                                 // walking stencil rows; 2 four nodes per lane (tile-relative separations only)
     bool set = false;
 };
 

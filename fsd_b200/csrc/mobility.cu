@@ -30,6 +30,7 @@
 #include "fsd_green.cuh"
 #include "fsd_kernels.cuh"
 #include "fsd_profile.h"
+#include "fsd_spread.h"
 #include "fsd_wavefft.h"
 
 namespace fsd {
@@ -1474,14 +1475,6 @@ __global__ void __launch_bounds__(128) k_real_combine(RealArgs a) {
 }
 
 // ------------------------------------------------------------------ drivers
-// Node-particle separations stay below (T + P) cells per axis, plus the
-// tilt's x shift; below half the box they are their own minimum image.
-static bool spread_local(const fsd_handle* h, int TX, int TY, int TZ) {
-    const GridParams& g = h->g;
-    const float tilt = 1.0f + fabsf(h->box.xy);
-    return (TX + g.P) * tilt < 0.5f * g.Nx && (TY + g.P) * tilt < 0.5f * g.Ny && (TZ + g.P) * tilt < 0.5f * g.Nz;
-}
-
 static void spread(fsd_handle* h) {
     const GridParams& g = h->g;
     SpreadArgs a;
@@ -1500,49 +1493,23 @@ static void spread(fsd_handle* h) {
     const float xisq = h->p.xi * h->p.xi;
     a.prefac = (2.0 * xisq / kPiRef / g.eta) * sqrtf(2.0 * xisq / kPiRef / g.eta);
     a.expfac = 2.0 * xisq / g.eta;
-    auto local = [&](int TX, int TY, int TZ) { return spread_local(h, TX, TY, TZ); };
-    auto tiles = [&](int TX, int TY, int TZ) {
-        return ((g.Nx + TX - 1) / TX) * ((g.Ny + TY - 1) / TY) * ((g.Nz + TZ - 1) / TZ);
-    };
-    int per_lane = 1;
-    if (h->tune.set && h->tune.TX > 0) {
-        a.TX = h->tune.TX;
-        a.TY = h->tune.TY;
-        a.TZ = h->tune.TZ;
-        per_lane = h->tune.spread_rows == 2 ? 4 : 1;
-    } else {
-        // Four nodes per lane on 8 x 8 x 8 tiles when separations are
-        // tile-relative and the tiles, four warps each, fill the chip four
-        // times over (with fewer warps in flight each tile's serial walk over
-        // its particles shows: 34 us against 17.8 with one node per lane at
-        // N = 8000, phi = 0.45; 47 against 52 at N = 32768, 72^3).  Else one node per
-        // lane on smaller tiles, which stage each particle more often but are
-        // more, and keep separations tile-relative in a smaller box.
-        const int shapes[4][5] = {{8, 8, 8, 4, 4 * 148}, {4, 8, 8, 1, 2 * 148}, {4, 4, 8, 1, 2 * 148}, {4, 4, 4, 1, 0}};
-        for (int k = 0; k < 4; ++k) {
-            a.TX = std::min(shapes[k][0], g.Nx - g.P + 1);
-            a.TY = std::min(shapes[k][1], g.Ny - g.P + 1);
-            a.TZ = std::min(shapes[k][2], g.Nz - g.P + 1);
-            per_lane = shapes[k][3];
-            if (k < 3 && a.TX == shapes[k][0] && a.TY == shapes[k][1] && a.TZ == shapes[k][2] &&
-                tiles(a.TX, a.TY, a.TZ) >= shapes[k][4] && local(a.TX, a.TY, a.TZ))
-                break;
-        }
-    }
-    a.local = local(a.TX, a.TY, a.TZ);
-    const int ntiles = tiles(a.TX, a.TY, a.TZ), threads = a.TX * a.TY * a.TZ;
+    const SpreadChoice c = spread_choice(g, h->box.xy, h->tune);
+    a.TX = c.TX;
+    a.TY = c.TY;
+    a.TZ = c.TZ;
+    a.local = c.local;
+    const int ntiles = spread_tiles(g, c.TX, c.TY, c.TZ), threads = c.TX * c.TY * c.TZ;
     const int EX = a.TX + g.P - 1, EY = a.TY + g.P - 1, EZ = a.TZ + g.P - 1;
-    const bool blocks = a.TX % 2 == 0 && a.TY % 4 == 0 && a.TZ % 4 == 0;
     count_launch();
     const size_t seg_bytes = sizeof(unsigned) * (4 * (size_t)EX * EY + 1);
-    if (per_lane == 4) {
+    if (c.form == kSpreadFour) {
         if (g.P == 6)
             launch_pdl(k_spread4<6>, ntiles, threads / 4, seg_bytes, h->stream, a);
         else if (g.P == 8)
             launch_pdl(k_spread4<8>, ntiles, threads / 4, seg_bytes, h->stream, a);
         else
             launch_pdl(k_spread4<0>, ntiles, threads / 4, seg_bytes, h->stream, a);
-    } else if (blocks && !(h->tune.set && h->tune.spread_rows)) {
+    } else if (c.form == kSpreadBlocks) {
         if (g.P == 6)
             launch_pdl(k_spread<6>, ntiles, threads, seg_bytes, h->stream, a);
         else if (g.P == 8)
@@ -1682,7 +1649,7 @@ static int autotune(fsd_handle* h) {
                     if (rows < 2 && (T < 64 || T > 256)) continue;
                     if (!rows && !(TX % 2 == 0 && TY % 4 == 0 && TZ % 4 == 0)) continue;
                     if (rows == 2 && !(TX % 4 == 0 && TY % 4 == 0 && TZ % 8 == 0 && T <= 512 && T >= 128 &&
-                                       spread_local(h, TX, TY, TZ)))
+                                       spread_local(g, h->box.xy, TX, TY, TZ)))
                         continue;
                     h->tune = TuneChoice{TX, TY, TZ, 0, 0, 0, rows, true};
                     const float ms = time_ms(h, [&] { spread(h); });

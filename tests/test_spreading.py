@@ -7,7 +7,12 @@ cluster of m particles adds m random terms per node, whose rounding grows no fas
 """
 from __future__ import annotations
 
+import ctypes as C
 import math
+import os
+import shutil
+import subprocess
+from pathlib import Path
 
 import numpy as np
 import pytest
@@ -53,3 +58,89 @@ def test_spread_uneven_bins(cuda, n, N, size, xy, err):
     ref = O.generalized_velocity(u, np.transpose(D, (0, 2, 1)), N)
     got = got.cpu().numpy()
     assert np.linalg.norm(got - ref) / np.linalg.norm(ref) < 1e-5
+
+
+@pytest.fixture(scope="module")
+def choose(tmp_path_factory):
+    """spread_choice of fsd_spread.h, compiled on its own: (TX, TY, TZ, form, local)."""
+    gxx, inc = shutil.which("g++"), Path(os.environ.get("CUDA_HOME", "/usr/local/cuda")) / "include"
+    if gxx is None or not (inc / "cuda_runtime.h").exists():
+        pytest.skip("no host compiler or CUDA headers")
+    d = tmp_path_factory.mktemp("spread")
+    (d / "choice.cpp").write_text("""#include "fsd_spread.h"
+extern "C" void choice(const int* grid, float xy, const int* tune, int* out) {
+    fsd::GridParams g;
+    g.Nx = grid[0], g.Ny = grid[1], g.Nz = grid[2], g.P = grid[3];
+    TuneChoice t;
+    t.TX = tune[0], t.TY = tune[1], t.TZ = tune[2], t.spread_rows = tune[3], t.set = tune[0] > 0;
+    const fsd::SpreadChoice c = fsd::spread_choice(g, xy, t);
+    out[0] = c.TX, out[1] = c.TY, out[2] = c.TZ, out[3] = c.form, out[4] = c.local;
+}
+""")
+    csrc = Path(__file__).resolve().parents[1] / "fsd_b200" / "csrc"
+    subprocess.run([gxx, "-std=c++17", "-shared", "-fPIC", f"-I{csrc}", f"-I{inc}", "-o", str(d / "choice.so"),
+                    str(d / "choice.cpp")], check=True)
+    f = C.CDLL(str(d / "choice.so")).choice
+    f.argtypes = [C.POINTER(C.c_int), C.c_float, C.POINTER(C.c_int), C.POINTER(C.c_int)]
+
+    def call(grid, xy, tune=(0, 0, 0, 0)):
+        out = (C.c_int * 5)()
+        f((C.c_int * 4)(*grid), xy, (C.c_int * 4)(*tune), out)
+        return tuple(out)
+
+    return call
+
+
+@pytest.mark.parametrize("tile", [(4, 4, 8), (8, 8, 8), (4, 8, 16), (4, 4, 32)])
+def test_four_nodes_per_lane_only_on_local_tiles(choose, tile):
+    """A tuned tile with four nodes per lane holds for the tilts at which its separations are tile-relative and
+    gives way to the built-in choice at the others (the kernel does not take minimum images)."""
+    kept = left = 0
+    for n in range(12, 151):
+        for P in (6, 8, 10):
+            if n - P + 1 < max(tile):
+                continue
+            for xy in (0.0, 0.1, -0.3, 0.45, -0.5):
+                got = choose((n, n, n, P), xy, (*tile, 2))
+                if all((t + P) * (1 + abs(xy)) < 0.5 * n for t in tile):
+                    assert got == (*tile, 2, 1)
+                    kept += 1
+                else:
+                    assert got == choose((n, n, n, P), xy)
+                    assert got[3] != 2 or got[4]
+                    left += 1
+    assert kept and left
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,N", [(60, 4000), (60, 16000), (36, 3000), (32, 1500), (54, 30000)])
+def test_tuned_spreading_at_another_tilt(cuda, n, N):
+    """Tiles tuned without tilt, then a tilt at which a tuned tile's separations need not be tile-relative, on the
+    tuned handle and on a second one that takes its choice from the cache.  Against a handle that was not tuned; the
+    forms round separations of up to half the box (4e-6 at 60 nodes) in different places, 8e-7 of the product."""
+    L = (edge(n, 1e-3),) * 3
+    rng = np.random.default_rng(n * N)
+    frac = rng.random((N, 3)) - 0.5
+    F = torch.as_tensor(rng.standard_normal(11 * N).astype(np.float32)).cuda()
+
+    def at(xy):
+        pos = np.zeros((N, 4), np.float32)
+        pos[:, 1:3] = frac[:, 1:] * L[0]
+        pos[:, 0] = frac[:, 0] * L[0] + xy * pos[:, 1]
+        return torch.as_tensor(pos).cuda().view(-1)
+
+    def handle(xy, tune):
+        return FSD(N, (*L, xy), xi=XI, gmres_restart=2, lanczos_max=4, autotune=tune)
+
+    plain = handle(0.0, 0)
+    tuned = handle(0.0, 1)
+    tuned.mobility(at(0.0), F, parts=1)
+    cached = handle(0.45, 1)
+    for xy in (0.45, -0.3, 0.0):
+        for s in (plain, tuned, cached):
+            s.set_box(*L, xy)
+        ref = plain.mobility(at(xy), F, parts=1)
+        for s in (tuned, cached):
+            assert (s.mobility(at(xy), F, parts=1) - ref).norm() < 2e-6 * ref.norm()
+    for s in (plain, tuned, cached):
+        s.close()
