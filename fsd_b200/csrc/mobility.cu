@@ -1032,7 +1032,8 @@ __global__ void __launch_bounds__(256, 4) k_spread(SpreadArgs a) {
 
 // The same sums with one node per thread, which walks its P x P (x, y) rows
 // of contiguous cells; for tiles that are not multiples of the warp block
-// (grids with fewer than P + 3 nodes along an axis).
+// (grids with fewer than P + 3 nodes along an axis).  Needs whole warps, at
+// least TX TY TZ threads.
 __global__ void __launch_bounds__(256, 3) k_spread_rows(SpreadArgs a) {
     pdl_wait();
     __shared__ StagedParticle sp[kSpreadCap];
@@ -1517,8 +1518,9 @@ static void spread(fsd_handle* h) {
         else
             launch_pdl(k_spread<0>, ntiles, threads, seg_bytes, h->stream, a);
     } else {
+        // whole warps: the block's scan of the particle counts leaves a partial one out
         const size_t cell_bytes = sizeof(unsigned) * (2 * (size_t)EX * EY * EZ + 1);
-        launch_pdl(k_spread_rows, ntiles, threads, cell_bytes, h->stream, a);
+        launch_pdl(k_spread_rows, ntiles, (threads + 31) & ~31, cell_bytes, h->stream, a);
     }
 }
 

@@ -144,3 +144,28 @@ def test_tuned_spreading_at_another_tilt(cuda, n, N):
             assert (s.mobility(at(xy), F, parts=1) - ref).norm() < 2e-6 * ref.norm()
     for s in (plain, tuned, cached):
         s.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("P,strain", [(10, 1.0), (11, 1.15), (12, 1.3)])
+@pytest.mark.parametrize("grid", [(12, 12, 12), (30, 30, 12), (12, 30, 24), (27, 12, 20)])
+def test_spread_on_grids_as_wide_as_the_stencil(cuda, grid, P, strain):
+    """Axes with one to three nodes more than the stencil has, P - 1: tiles of 1 to 48 nodes, which are no whole
+    warps.  The oracle and tolerance of the other spreading tests."""
+    N = 301
+    L = tuple(edge(n, 1e-3) for n in grid)
+    rng = np.random.default_rng(sum(grid) + P)
+    frac = rng.random((N, 3)) - 0.5
+    pos = np.zeros((N, 4), np.float32)
+    pos[:, :3] = frac * np.array(L)
+    s = FSD(N, (*L, 0.0), xi=XI, max_strain=strain, gmres_restart=2, lanczos_max=4)
+    info = s.pse_info()
+    assert (info.Nx, info.Ny, info.Nz, info.P) == (*grid, P)
+    F = torch.as_tensor(rng.standard_normal(11 * N).astype(np.float32)).cuda()
+    got = s.mobility(torch.as_tensor(pos).cuda().view(-1), F, parts=1).cpu().numpy()
+    s.close()
+    gp = {k: getattr(info, k) for k in ("Nx", "Ny", "Nz", "P", "eta", "hx", "hy", "hz")}
+    Ff, Cp = O.split_generalized(F.cpu().numpy().astype(np.float64), N)
+    u, D = O.wave_space(pos, Ff, Cp, L, 0.0, gp, XI)
+    ref = O.generalized_velocity(u, np.transpose(D, (0, 2, 1)), N)
+    assert np.linalg.norm(got - ref) / np.linalg.norm(ref) < 1e-5
