@@ -153,7 +153,7 @@ __global__ void k_noise_spectrum(float2* __restrict__ grid, const float4* __rest
 // The same field as half spectra (z <= Nz / 2) of the 11 real grids: each
 // point takes the draws of its pair's smaller index, conjugated when that is
 // the mirror point.
-__global__ void k_noise_half(float2* __restrict__ spec, const float4* __restrict__ gridk, int Nx, int Ny, int Nz, int zp,
+__global__ void k_noise_half(float2* spec, const float4* __restrict__ gridk, int Nx, int Ny, int Nz, int zp,
                              float fac, uint32_t key, uint32_t step, uint32_t stream) {
     pdl_wait();
     const int l = blockIdx.x * blockDim.x + threadIdx.x;
@@ -208,13 +208,13 @@ void dot_device(fsd_handle* h, const float* a, const float* b, size_t n, double*
     k_sum_parts<<<1, 32, 0, h->stream>>>(h->w.dred, kDotBlocks, out);
 }
 
-__global__ void k_sum2(float* __restrict__ y, const float* __restrict__ a, const float* __restrict__ b, size_t n) {
+__global__ void k_sum2(float* y, const float* a, const float* b, size_t n) {
     pdl_wait();
     for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
         y[k] = a[k] + b[k];
 }
-__global__ void k_lincomb(const float* __restrict__ V, size_t ld, int m, const double* __restrict__ c,
-                          float* __restrict__ y, size_t n, float scale) {
+__global__ void k_lincomb(const float* V, size_t ld, int m, const double* c,
+                          float* y, size_t n, float scale) {
     pdl_wait();
     for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x) {
         double acc = 0.0;
@@ -318,7 +318,7 @@ __device__ __forceinline__ bool grid_sum(double& s, double* part, unsigned* tick
 }
 
 // norm[0] = |x|.
-__global__ void __launch_bounds__(256) k_lz_norm(const float* __restrict__ x, size_t n, double* part, unsigned* ticket,
+__global__ void __launch_bounds__(256) k_lz_norm(const float* x, size_t n, double* part, unsigned* ticket,
                                                  double* norm) {
     pdl_wait();
     double s = 0.0;
@@ -328,9 +328,9 @@ __global__ void __launch_bounds__(256) k_lz_norm(const float* __restrict__ x, si
 }
 
 // w -= beta_j v_{j-1}; alpha_j = v_j . w.
-__global__ void __launch_bounds__(256) k_lz_alpha(float* __restrict__ w, const float* __restrict__ v,
-                                                  const float* __restrict__ vprev, size_t n, int j, double* part,
-                                                  unsigned* ticket, double* alpha, const double* __restrict__ beta) {
+__global__ void __launch_bounds__(256) k_lz_alpha(float* w, const float* v,
+                                                  const float* vprev, size_t n, int j, double* part,
+                                                  unsigned* ticket, double* alpha, const double* beta) {
     pdl_wait();
     const float nb = j > 0 ? (float)(-beta[j]) : 0.f;
     double s = 0.0;
@@ -346,8 +346,8 @@ __global__ void __launch_bounds__(256) k_lz_alpha(float* __restrict__ w, const f
 }
 
 // w -= alpha_j v_j; beta_{j+1} = |w|.
-__global__ void __launch_bounds__(256) k_lz_beta(float* __restrict__ w, const float* __restrict__ v, size_t n, int j,
-                                                 double* part, unsigned* ticket, const double* __restrict__ alpha,
+__global__ void __launch_bounds__(256) k_lz_beta(float* w, const float* v, size_t n, int j,
+                                                 double* part, unsigned* ticket, const double* alpha,
                                                  double* beta) {
     pdl_wait();
     const float na = (float)(-alpha[j]);
@@ -362,7 +362,7 @@ __global__ void __launch_bounds__(256) k_lz_beta(float* __restrict__ w, const fl
 }
 
 // y = x / *norm (zero past an invariant subspace; first: past a zero vector).
-__global__ void k_lz_scale(float* __restrict__ y, const float* __restrict__ x, size_t n, const double* __restrict__ norm,
+__global__ void k_lz_scale(float* y, const float* x, size_t n, const double* norm,
                            int first) {
     pdl_wait();
     const double b = *norm;

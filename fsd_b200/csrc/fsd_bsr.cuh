@@ -34,7 +34,7 @@ __device__ __forceinline__ int bsr_component() {
 // the component lanes; row = its 36 n floats, ld(j, k) loads operand pair k
 // (components 2k, 2k + 1) of particle j.  All lanes of the warp take part.
 template <int W = 16, class LD>
-__device__ __forceinline__ float bsr_row(const float* __restrict__ row, const int* __restrict__ cols, int n, LD ld) {
+__device__ __forceinline__ float bsr_row(const float* row, const int* cols, int n, LD ld) {
     const int l = threadIdx.x & (W - 1);
     const int np = 3 * n;  // pairs per component
     unsigned long long acc[6] = {0, 0, 0, 0, 0, 0};
@@ -42,7 +42,7 @@ __device__ __forceinline__ float bsr_row(const float* __restrict__ row, const in
     for (int p = l; p < np; p += W, m += W) {
         unsigned long long g[6];
 #pragma unroll
-        for (int r = 0; r < 6; ++r) g[r] = __ldg(m + r * np);
+        for (int r = 0; r < 6; ++r) g[r] = m[r * np];
         const int e = p / 3;
         const float2 x = ld(cols[e], p - 3 * e);
         unsigned long long x2;
@@ -83,7 +83,7 @@ __device__ __forceinline__ float bsr_row(const float* __restrict__ row, const in
 struct BsrPlain {
     const float* x;
     __device__ __forceinline__ float2 operator()(int j, int k) const {
-        return __ldg(reinterpret_cast<const float2*>(x) + (3 * j + k));
+        return reinterpret_cast<const float2*>(x)[3 * j + k];
     }
 };
 struct BsrSaddle {

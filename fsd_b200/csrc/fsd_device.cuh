@@ -57,10 +57,16 @@ __device__ __forceinline__ void wrap_position(float3& w, int3& img, const Box& b
     else if (w.z < -b.Lz / 2) { w.z += b.Lz; img.z--; }
 }
 
-// 32 bytes in one load (32-byte aligned, read-only for the kernel).  A gather
-// costs the L1 one tag lookup per lane and instruction, so records of 32 bytes
-// take half the lookups of two float4.
+// 32 bytes in one load (32-byte aligned).  A gather costs the L1 one tag lookup
+// per lane and instruction, so records of 32 bytes take half the lookups of two
+// float4.  Volatile, so it stays behind pdl_wait(); the kernel must not write
+// what it reads.  load8_const: tables that no overlapped kernel writes.
 __device__ __forceinline__ void load8(const float* p, float* v) {
+    asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+                 : "l"(p));
+}
+__device__ __forceinline__ void load8_const(const float* p, float* v) {
     asm volatile("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                  : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
                  : "l"(p));
@@ -160,6 +166,13 @@ __device__ __forceinline__ void block_partial(double v, double* part) {
 // about a microsecond per launch, then overlap the previous kernel.  Every
 // thread waits before anything else, so a kernel's completion implies that of
 // all before it.
+//
+// Such a kernel's lifetime begins while its predecessor still writes, so data
+// from the stream is read by ordinary loads: no __ldg and no ld.global.nc, which
+// presume data that does not change meanwhile, and no __restrict__ pointer, whose
+// accesses a compiler may move across the wait.  What is written once, or by
+// launches that are not overlapped (tables, the matrix A of the inner GMRES), may
+// go the read-only way.
 //
 // Grids of more than two blocks per SM are launched the ordinary way: blocks
 // that come up early crowd the SMs that have room, and the overlap is short

@@ -147,8 +147,8 @@ constexpr int kBetaSlot = (kMaxInner + 1) * kMaxInner;  // in H: beta, then the 
 // Z_j = G U_j, a warp per row on G's copy by components, and |U_j|; FIRST:
 // U_0 = b[0:6N] - b[11N:17N], taken from b in the gathers too.
 template <bool FIRST>
-__global__ void __launch_bounds__(kInnerThreads, 4) k_inner_g(const int* __restrict__ rowptr, const int* __restrict__ col,
-                                                              const float* __restrict__ G, const float* __restrict__ b,
+__global__ void __launch_bounds__(kInnerThreads, 4) k_inner_g(const int* rowptr, const int* col,
+                                                              const float* G, const float* b,
                                                               float* U, float* __restrict__ z, int N, double* beta,
                                                               double* nrm, double* part, unsigned* ticket) {
     pdl_wait();
@@ -184,12 +184,10 @@ __global__ void __launch_bounds__(kInnerThreads, 4) k_inner_g(const int* __restr
 
 // w = A z / |U_j| over the pruned list (self included), written to the basis
 // slot U_nv, fused with the dots H[j][q] = (U_q . w) / |U_q| for q < nv = j + 1.
-__global__ void __launch_bounds__(256) k_inner_a(const unsigned* __restrict__ pn,
-                                                          const unsigned* __restrict__ plist,
-                                                          const float* __restrict__ A,
-                                                          const float* __restrict__ z, float* U, size_t ld, int nv,
-                                                          const double* __restrict__ nrm, double* part,
-                                                          unsigned* ticket, double* H, int j, int N) {
+__global__ void __launch_bounds__(256) k_inner_a(const unsigned* __restrict__ pn, const unsigned* __restrict__ plist,
+                                                 const float* __restrict__ A, const float* z, float* U, size_t ld, int nv,
+                                                 const double* nrm, double* part, unsigned* ticket, double* H, int j,
+                                                 int N) {
     pdl_wait();
     __shared__ double sh[kMaxInner + 1][8];
     const int gid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -263,8 +261,8 @@ __device__ __forceinline__ float2 inner_pair(const float* U, size_t ld, int nv, 
 }
 
 // U_nv -= sum_{q<nv} (H[j][q] / |U_q|) U_q, by pairs (ld = 6N is even).
-__global__ void __launch_bounds__(kInnerThreads) k_inner_orth(float* U, size_t ld, int nv, const double* __restrict__ hj,
-                                                              const double* __restrict__ nrm) {
+__global__ void __launch_bounds__(kInnerThreads) k_inner_orth(float* U, size_t ld, int nv, const double* hj,
+                                                              const double* nrm) {
     pdl_wait();
     __shared__ float cs[kMaxInner];
     inner_factors(cs, hj, nrm, nv);
@@ -351,7 +349,7 @@ __global__ void __launch_bounds__(kInnerThreads) k_inner_last(const float* U, si
 }
 
 // x = post(b, sum_i c_i Z_i): x[0:6N] = b - y, x[6N:11N] = b, x[11N:] = y.
-__global__ void k_inner_post(const float* __restrict__ Z, size_t ld, int k, const double* __restrict__ c,
+__global__ void k_inner_post(const float* Z, size_t ld, int k, const double* c,
                              const float* b, float* x, int N) {
     pdl_wait();
     const int kk = blockIdx.x * blockDim.x + threadIdx.x;

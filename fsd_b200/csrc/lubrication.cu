@@ -50,8 +50,8 @@ __device__ __forceinline__ bool lub_interp(const float* __restrict__ tab, float 
     if (ind >= kResRows - 1) return false;
     float lo[L], hi[L];
     const float* p = tab + (size_t)ind * RS;
-    load8(p, lo);
-    load8(p + RS, hi);
+    load8_const(p, lo);
+    load8_const(p + RS, hi);
     if constexpr (L > 8) {
         const float4 a = __ldg(reinterpret_cast<const float4*>(p + 8)), b = __ldg(reinterpret_cast<const float4*>(p + RS + 8));
         lo[8] = a.x;
@@ -69,7 +69,7 @@ __device__ __forceinline__ bool lub_interp(const float* __restrict__ tab, float 
 
 // U and W of particle j: PACKED from records of 8, else from the 6N vector.
 template <bool PACKED>
-__device__ __forceinline__ void load_uw(const float* __restrict__ U, unsigned j, float3& u, float3& w) {
+__device__ __forceinline__ void load_uw(const float* U, unsigned j, float3& u, float3& w) {
     if constexpr (PACKED) {
         float v[8];
         load8(U + 8 * (size_t)j, v);
@@ -79,7 +79,7 @@ __device__ __forceinline__ void load_uw(const float* __restrict__ U, unsigned j,
         const float* p = U + 6 * (size_t)j;
         if ((reinterpret_cast<uintptr_t>(U) & 7) == 0) {  // 6-vectors start on 8 bytes
             const float2* q = reinterpret_cast<const float2*>(p);
-            const float2 a = __ldg(q), b = __ldg(q + 1), c = __ldg(q + 2);
+            const float2 a = q[0], b = q[1], c = q[2];
             u = make_float3(a.x, a.y, b.x);
             w = make_float3(b.y, c.x, c.y);
         } else {
@@ -121,8 +121,8 @@ __device__ __forceinline__ float3 eps_dot(float3 r, float3 v) {
 // F = R_FU U (Lubrication_RFU_kernel, Lubrication.cu:69-309).  With saddle_x,
 // writes saddle_x[6i + c] - F instead (Saddle.cu:141-148).
 template <bool PACKED>
-__global__ void __launch_bounds__(128) k_rfu(LubArgs a, const float* __restrict__ U, float* __restrict__ out,
-                                             const float* __restrict__ saddle_x) {
+__global__ void __launch_bounds__(128) k_rfu(LubArgs a, const float* U, float* out,
+                                             const float* saddle_x) {
     pdl_wait();
     const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / kLubGroup;
     const int gl = threadIdx.x % kLubGroup;
@@ -181,7 +181,7 @@ __global__ void __launch_bounds__(128) k_rfu(LubArgs a, const float* __restrict_
 
 // F += R_FE : E (Lubrication_RFE_kernel, Lubrication.cu:350-608).
 __global__ void __launch_bounds__(128) k_rfe(LubArgs a, float shear_rate, const float3* ori, const float* b2mask,
-                                             float B2, float* __restrict__ out) {
+                                             float B2, float* out) {
     pdl_wait();
     const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / kLubGroup;
     const int gl = threadIdx.x % kLubGroup;
@@ -239,7 +239,7 @@ __host__ __device__ constexpr int sb_of(int k) { return k < 3 ? k : 5 - k; }
 __device__ __forceinline__ float comp(float3 v, int k) { return k == 0 ? v.x : (k == 1 ? v.y : v.z); }
 
 // S -= R_SU U (Lubrication_RSU_kernel, Lubrication.cu:650-911).
-__global__ void __launch_bounds__(128) k_rsu(LubArgs a, const float* __restrict__ U, float* __restrict__ S) {
+__global__ void __launch_bounds__(128) k_rsu(LubArgs a, const float* U, float* S) {
     pdl_wait();
     const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / kLubGroup;
     const int gl = threadIdx.x % kLubGroup;
@@ -287,7 +287,7 @@ __global__ void __launch_bounds__(128) k_rsu(LubArgs a, const float* __restrict_
 // S += R_SE : E (Lubrication_RSE_kernel, Lubrication.cu:953-1230); pairs
 // within r^2 < 16 as the reference hard-codes.
 __global__ void __launch_bounds__(128) k_rse(LubArgs a, float shear_rate, const float3* ori, const float* b2mask,
-                                             float B2, float* __restrict__ S) {
+                                             float B2, float* S) {
     pdl_wait();
     const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / kLubGroup;
     const int gl = threadIdx.x % kLubGroup;

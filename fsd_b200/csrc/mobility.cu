@@ -533,9 +533,9 @@ static void fft_x_green(fsd_handle* h) {
 //   sorted  12 floats in bin order (with `parts`): the spreading kernel's pairs
 //           (Fx,Fy,Cxx,Cxy) (Cxz,Cyx,Cyy,Cyz) (Czx,Czy,Fz,0);
 //   u8      8 floats (with `saddle_x`): the saddle vector's U and W.
-__global__ void k_prep(const float* __restrict__ genF, const float4* __restrict__ pos, int N, float* __restrict__ rec,
-                       const unsigned* __restrict__ parts, float4* __restrict__ sorted,
-                       const float* __restrict__ saddle_x, float* __restrict__ u8) {
+__global__ void k_prep(const float* genF, const float4* pos, int N, float* rec,
+                       const unsigned* parts, float4* sorted,
+                       const float* saddle_x, float* u8) {
     pdl_wait();
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= N) return;
@@ -593,9 +593,9 @@ __device__ __forceinline__ int3 stencil_origin(float4 p, const Box& b, int Nx, i
 // bin starts of the column's Nz nodes, so no pass over all nodes is scanned
 // (at 72^3: 5184 columns instead of 373248 bins; 18 -> 9 us for nine launches
 // before).
-__global__ void __launch_bounds__(1024) k_col_count(const float4* __restrict__ pos, int N, Box b, int Nx, int Ny, int Nz,
-                                                    int P, uint2* __restrict__ part, unsigned* __restrict__ col_count,
-                                                    unsigned* __restrict__ col_start, unsigned* ticket) {
+__global__ void __launch_bounds__(1024) k_col_count(const float4* pos, int N, Box b, int Nx, int Ny, int Nz,
+                                                    int P, uint2* part, unsigned* col_count,
+                                                    unsigned* col_start, unsigned* ticket) {
     pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < N) {
@@ -613,8 +613,8 @@ __global__ void __launch_bounds__(1024) k_col_count(const float4* __restrict__ p
 
 // Particles into their columns (in the order the atomics gave; ranked below),
 // as (z, index); the column counters go back to zero for the next call.
-__global__ void k_col_fill(const uint2* __restrict__ part, int N, const unsigned* __restrict__ col_start, int ncol,
-                           unsigned* __restrict__ col_count, uint2* __restrict__ items) {
+__global__ void k_col_fill(const uint2* part, int N, const unsigned* col_start, int ncol,
+                           unsigned* col_count, uint2* items) {
     pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < ncol) col_count[i] = 0u;
@@ -625,10 +625,10 @@ __global__ void k_col_fill(const uint2* __restrict__ part, int N, const unsigned
 
 // One warp per column.  A member's place is the number of members below it in
 // (z, index); each lane then finds the starts of its share of the nodes.
-__global__ void __launch_bounds__(256) k_col_sort(const float4* __restrict__ pos, const unsigned* __restrict__ col_start,
-                                                  int ncol, int Nz, const uint2* __restrict__ items,
-                                                  unsigned* __restrict__ bin_parts, unsigned* __restrict__ bin_start,
-                                                  float4* __restrict__ sorted_pos) {
+__global__ void __launch_bounds__(256) k_col_sort(const float4* pos, const unsigned* col_start,
+                                                  int ncol, int Nz, const uint2* items,
+                                                  unsigned* bin_parts, unsigned* bin_start,
+                                                  float4* sorted_pos) {
     pdl_wait();
     const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
@@ -1220,10 +1220,10 @@ __global__ void __launch_bounds__(256, 3) k_spread_rows(SpreadArgs a) {
 // well under half the box) each node's separation is the stencil origin's
 // minimum image plus the node's fixed offset in the sheared grid.
 template <int KP>
-__global__ void __launch_bounds__(256) k_contract(const float4* __restrict__ pos, const unsigned* __restrict__ order,
-                                                  const float2* __restrict__ grid, int N, Box b, int Nx, int Ny,
+__global__ void __launch_bounds__(256) k_contract(const float4* pos, const unsigned* order,
+                                                  const float2* grid, int N, Box b, int Nx, int Ny,
                                                   int Nz, int Prun, float hx, float hy, float hz, float prefac,
-                                                  float expfac, bool local, float* __restrict__ out) {
+                                                  float expfac, bool local, float* out) {
     pdl_wait();
     const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
@@ -1253,6 +1253,19 @@ __global__ void __launch_bounds__(256) k_contract(const float4* __restrict__ pos
         ix -= (ix >= Nx) ? Nx : 0;
         iy -= (iy >= Ny) ? Ny : 0;
         iz -= (iz >= Nz) ? Nz : 0;
+        const float2* gp = grid + ((size_t)ix * Ny + iy) * Nz + iz;
+        float2 q0, q1, q2, q3, q4, q5;  // (Ux,Uy) (XX,XY) (XZ,YX) (YY,YZ) (ZX,ZY) (Uz,-)
+        auto nodes = [&] {
+            q0 = gp[0];
+            q1 = gp[G];
+            q2 = gp[2 * G];
+            q3 = gp[3 * G];
+            q4 = gp[4 * G];
+            q5 = gp[5 * G];
+        };
+        // ahead of the weight where the loop is not unrolled (P = 8, N = 7351: 30 us against 36 behind it; P = 6,
+        // N = 32768: 46 against 45)
+        if (KP == 0) nodes();
         float3 r;
         if (local) {
             r = make_float3(r0.x + (hx * tx + b.xy * (hy * ty)), r0.y + hy * ty, r0.z + hz * tz);
@@ -1266,10 +1279,7 @@ __global__ void __launch_bounds__(256) k_contract(const float4* __restrict__ pos
         }
         const float rsq = r.x * r.x + r.y * r.y + r.z * r.z;
         const float wgt = prefac * expf(-expfac * rsq);
-        const size_t g = ((size_t)ix * Ny + iy) * Nz + iz;
-        const float2 q0 = __ldg(grid + g), q1 = __ldg(grid + G + g), q2 = __ldg(grid + 2 * G + g),
-                     q3 = __ldg(grid + 3 * G + g), q4 = __ldg(grid + 4 * G + g), q5 = __ldg(grid + 5 * G + g);
-        // q0=(Ux,Uy) q1=(XX,XY) q2=(XZ,YX) q3=(YY,YZ) q4=(ZX,ZY) q5=(Uz,-)
+        if (KP > 0) nodes();
         acc[0] += wgt * q0.x;
         acc[1] += wgt * q0.y;
         acc[2] += wgt * q5.x;
@@ -1358,8 +1368,8 @@ __global__ void __launch_bounds__(128) k_real_combine(RealArgs a) {
             // Clamped so that a distance rounding up to the cutoff stays inside the table.
             const int r_ind = min(max(__float2int_rd(a.row_scale * (dist - a.ewald_dr)), 0), a.ewald_n - 1);
             float lo[8], hi[8];
-            load8(a.table + 8 * (size_t)r_ind, lo);
-            load8(a.table + 8 * (size_t)r_ind + 8, hi);
+            load8_const(a.table + 8 * (size_t)r_ind, lo);
+            load8_const(a.table + 8 * (size_t)r_ind + 8, hi);
             const float fac = fmaf(-(float)(r_ind + 1), a.ewald_dr, dist) * a.inv_dr;
             const float f1 = lo[0] + (hi[0] - lo[0]) * fac;
             const float f2 = lo[1] + (hi[1] - lo[1]) * fac;

@@ -121,9 +121,9 @@ __device__ __forceinline__ int3 cell_of(float4 p, const Box& b, int3 nc) {
 
 // Cell and slot within it (in the order the atomics gave) of each particle;
 // the last block scans the counts.
-__global__ void __launch_bounds__(1024) k_cell_count(const float4* __restrict__ pos, int n, Box b, int3 nc,
-                                                     unsigned* __restrict__ key, unsigned* __restrict__ slot,
-                                                     unsigned* __restrict__ count, unsigned* __restrict__ start,
+__global__ void __launch_bounds__(1024) k_cell_count(const float4* pos, int n, Box b, int3 nc,
+                                                     unsigned* key, unsigned* slot,
+                                                     unsigned* count, unsigned* start,
                                                      unsigned* ticket) {
     pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -138,8 +138,8 @@ __global__ void __launch_bounds__(1024) k_cell_count(const float4* __restrict__ 
     block_scan_counts(count, start, nc.x * nc.y * nc.z);
 }
 
-__global__ void k_cell_fill(const unsigned* __restrict__ key, const unsigned* __restrict__ slot, int n,
-                            const unsigned* __restrict__ start, unsigned* __restrict__ items) {
+__global__ void k_cell_fill(const unsigned* key, const unsigned* slot, int n,
+                            const unsigned* start, unsigned* items) {
     pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) items[start[key[i]] + slot[i]] = (unsigned)i;
@@ -148,10 +148,10 @@ __global__ void k_cell_fill(const unsigned* __restrict__ key, const unsigned* __
 // One warp per cell: a member's place is the number of smaller indices.
 // sorted_pos (optional) receives the positions in that order, index in w;
 // order (optional) a copy of parts.
-__global__ void __launch_bounds__(256) k_cell_sort(const float4* __restrict__ pos, const unsigned* __restrict__ start,
-                                                   int ncells, const unsigned* __restrict__ items,
-                                                   unsigned* __restrict__ parts, unsigned* __restrict__ order,
-                                                   float4* __restrict__ sorted_pos) {
+__global__ void __launch_bounds__(256) k_cell_sort(const float4* pos, const unsigned* start,
+                                                   int ncells, const unsigned* items,
+                                                   unsigned* parts, unsigned* order,
+                                                   float4* sorted_pos) {
     pdl_wait();
     const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
@@ -172,13 +172,13 @@ __global__ void __launch_bounds__(256) k_cell_sort(const float4* __restrict__ po
 
 // Rows of the neighbour list, and of the sub-list within sub2 (optional), one
 // warp per particle in cell order.
-__global__ void __launch_bounds__(128) k_nlist_cells(const float4* __restrict__ pos, int n, Box b, int3 nc,
-                                                     const unsigned* __restrict__ cstart,
-                                                     const unsigned* __restrict__ cparts,
-                                                     const float4* __restrict__ sorted_pos, float rlist2,
-                                                     unsigned* __restrict__ nneigh, unsigned* __restrict__ nlist,
+__global__ void __launch_bounds__(128) k_nlist_cells(const float4* pos, int n, Box b, int3 nc,
+                                                     const unsigned* cstart,
+                                                     const unsigned* cparts,
+                                                     const float4* sorted_pos, float rlist2,
+                                                     unsigned* nneigh, unsigned* nlist,
                                                      int stride, int* max_count, float sub2,
-                                                     unsigned* __restrict__ sub_n, unsigned* __restrict__ sub) {
+                                                     unsigned* sub_n, unsigned* sub) {
     pdl_wait();
     const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;

@@ -86,8 +86,8 @@ __device__ __forceinline__ double block_sum_d(double v, double* sh) {
 }
 
 // part[i * nblocks + block] = sum over this block's slice of V_i . w, i < nv.
-__global__ void __launch_bounds__(kRedThreads) k_multidot(const float* __restrict__ V, size_t ld, int nv,
-                                                          const float* __restrict__ w, size_t n, double* part,
+__global__ void __launch_bounds__(kRedThreads) k_multidot(const float* V, size_t ld, int nv,
+                                                          const float* w, size_t n, double* part,
                                                           const int* done) {
     pdl_wait();
     if (done && *done) return;
@@ -117,8 +117,8 @@ __global__ void k_finish_dots(const double* part, int nb, int nv, double* out, b
 }
 
 // y = sum_i c[i] V_i.
-__global__ void k_combine(const float* __restrict__ V, size_t ld, int nv, const double* __restrict__ c,
-                          float* __restrict__ y, size_t n) {
+__global__ void k_combine(const float* V, size_t ld, int nv, const double* c,
+                          float* y, size_t n) {
     pdl_wait();
     __shared__ float cs[kMaxRestart + 1];
     for (int i = threadIdx.x; i < nv; i += blockDim.x) cs[i] = (float)c[i];
@@ -130,7 +130,7 @@ __global__ void k_combine(const float* __restrict__ V, size_t ld, int nv, const 
     }
 }
 
-__global__ void k_scale_copy(const float* __restrict__ src, float* __restrict__ dst, size_t n, const double* norm,
+__global__ void k_scale_copy(const float* src, float* dst, size_t n, const double* norm,
                              const int* done) {
     pdl_wait();
     if (done && *done) return;
@@ -140,13 +140,13 @@ __global__ void k_scale_copy(const float* __restrict__ src, float* __restrict__ 
         dst[k] = src[k] * s;
 }
 
-__global__ void k_residual(const float* __restrict__ b, const float* __restrict__ Ax, float* __restrict__ r, size_t n) {
+__global__ void k_residual(const float* b, const float* Ax, float* r, size_t n) {
     pdl_wait();
     for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
         r[k] = b[k] - Ax[k];
 }
 
-__global__ void k_axpy(float* __restrict__ x, const float* __restrict__ u, size_t n) {
+__global__ void k_axpy(float* x, const float* u, size_t n) {
     pdl_wait();
     for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
         x[k] += u[k];
@@ -274,8 +274,8 @@ __global__ void k_export(const GmresState* s, GmresHost* o) {
 constexpr int kPairVecs = 16;
 constexpr int kPairSlice = 32;  // float4 per warp and slice
 
-__global__ void __launch_bounds__(kRedThreads, 2) k_dots_pair(const float* __restrict__ V, size_t ld, int j,
-                                                              const float* __restrict__ w, size_t n, double* part,
+__global__ void __launch_bounds__(kRedThreads, 2) k_dots_pair(const float* V, size_t ld, int j,
+                                                              const float* w, size_t n, double* part,
                                                               const int* done, double* out, unsigned* ticket) {
     pdl_wait();
     if (*done) return;
@@ -395,8 +395,8 @@ __device__ double tentative_resid(const double* col, int c, double hsub, const d
 // commits column j or leaves it pending.  Every block computes the same
 // coefficients.  Only the last block touches the state after every block has
 // read `done`; its serial work runs on shared-memory copies.
-__global__ void __launch_bounds__(kRedThreads, 2) k_dcgs_update(float* V, size_t ld, int j, const float* __restrict__ w,
-                                                             size_t n, const double* __restrict__ dots,
+__global__ void __launch_bounds__(kRedThreads, 2) k_dcgs_update(float* V, size_t ld, int j, const float* w,
+                                                             size_t n, const double* dots,
                                                              GmresState* s, int m, double* part, unsigned* ticket) {
     pdl_wait();
     if (s->done) return;

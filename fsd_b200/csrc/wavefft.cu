@@ -108,7 +108,7 @@ __device__ __forceinline__ int row_slot(int k) {
 // stored position; positions that are padding (natural() skips them) are
 // never used.
 template <class L>
-__global__ void __launch_bounds__(Plane<L>::threads) k_yz_fwd(const float2* __restrict__ grid, float2* __restrict__ spec,
+__global__ void __launch_bounds__(Plane<L>::threads) k_yz_fwd(const float2* grid, float2* spec,
                                                               int Nx, int zp, const float2* __restrict__ tw_global) {
     pdl_wait();
     constexpr int N = L::N;
@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(Plane<L>::threads) k_yz_fwd(const float2* __re
 }
 
 template <class L>
-__global__ void __launch_bounds__(Plane<L>::threads) k_yz_inv(const float2* __restrict__ spec, float2* __restrict__ grid,
+__global__ void __launch_bounds__(Plane<L>::threads) k_yz_inv(const float2* spec, float2* grid,
                                                               int Nx, int zp, const float2* __restrict__ tw_global) {
     pdl_wait();
     constexpr int N = L::N;
@@ -228,7 +228,7 @@ struct XPass {
 };
 
 template <class L, bool GREEN>
-__global__ void __launch_bounds__(XPass<L>::threads, XPass<L>::blocks) k_x_pass(float2* __restrict__ spec, const float4* __restrict__ table,
+__global__ void __launch_bounds__(XPass<L>::threads, XPass<L>::blocks) k_x_pass(float2* spec, const float4* __restrict__ table,
                                                               const float4* __restrict__ gridk, int Ny, int Nz, int zp,
                                                               const float2* __restrict__ tw_global) {
     pdl_wait();
