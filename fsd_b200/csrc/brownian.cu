@@ -487,8 +487,7 @@ int brownian_farfield(fsd_handle* h, const float4* pos, uint32_t step, float* ou
     else
         k_noise_spectrum<<<(G + 255) / 256, 256, 0, h->stream>>>(w.grid, w.gridk, g.Nx, g.Ny, g.Nz, fac,
                                                                  h->seed_hashed, step, kStreamFFWave);
-    const int e = mobility_wave_from_spectrum(h, pos);
-    if (e != FSD_OK) return e;
+    mobility_wave_from_spectrum(h, pos);
     // Combine into generalized layout (wave part only).
     mobility_combine(h, w.lz_c, true, false, nullptr);
     }

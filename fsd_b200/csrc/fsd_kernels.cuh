@@ -28,8 +28,8 @@ void mobility_set_gridk(fsd_handle* h);
 int mobility_apply(fsd_handle* h, const float4* pos, const float* genF, float* genU, int parts,
                    const float* saddle_x, bool rebin);
 // Wave-space part driven by a grid already holding spectra (Brownian):
-// inverse FFT + contraction into w.uwave (bins the particles at pos).
-int mobility_wave_from_spectrum(fsd_handle* h, const float4* pos);
+// inverse FFT + contraction into w.uwave.
+void mobility_wave_from_spectrum(fsd_handle* h, const float4* pos);
 void mobility_combine(fsd_handle* h, float* genU, bool wave, bool real, const float* saddle_x);
 
 // lubrication.cu

@@ -1556,9 +1556,7 @@ static void contract(fsd_handle* h, const float4* pos) {
                                                    g.hy, g.hz, quadW * prefac, expfac, local, h->w.uwave);
 }
 
-int mobility_wave_from_spectrum(fsd_handle* h, const float4* pos) {
-    const int st = mobility_bin_particles(h, pos);
-    if (st != FSD_OK) return st;
+void mobility_wave_from_spectrum(fsd_handle* h, const float4* pos) {
     {
         ProfRegion pr(h, R_FFT);
         if (h->w.spec) {
@@ -1570,7 +1568,6 @@ int mobility_wave_from_spectrum(fsd_handle* h, const float4* pos) {
     }
     ProfRegion pr(h, R_CONTRACT);
     contract(h, pos);
-    return FSD_OK;
 }
 
 void mobility_combine(fsd_handle* h, float* genU, bool wave, bool real,
