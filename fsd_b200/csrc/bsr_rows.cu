@@ -1,6 +1,6 @@
 // Products of the learned preconditioner's inner polynomial (and of the
 // approximate inverse applied once), each fused with the step around it, and
-// the copies of G and A that all row products read (fsd_bsr.cuh).
+// the by-component layout of blocks that all row products read (fsd_bsr.cuh).
 #include "fsd_bsr.cuh"
 #include "fsd_device.cuh"
 #include "fsd_kernels.cuh"
@@ -9,39 +9,67 @@
 
 namespace fsd {
 
-// Row i of the blocks at src (block CSR, or padded rows of kPrunedCap blocks
-// when pn is given) by components at the same offset of dst.
-__global__ void __launch_bounds__(256) k_bsr_layout(const int* __restrict__ rowptr, const unsigned* __restrict__ pn, int N,
+// Rows of blocks (block CSR, or padded rows of kPrunedCap blocks) by components
+// at dst + 36 rowptr[i].
+__global__ void __launch_bounds__(256) k_bsr_layout(const int* __restrict__ rowptr, bool padded, int N,
                                                     const float* __restrict__ src, float* __restrict__ dst) {
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (i >= N) return;
-    const size_t e0 = pn ? (size_t)i * kPrunedCap : (size_t)rowptr[i];
-    const int n = pn ? (int)pn[i] : rowptr[i + 1] - rowptr[i];
-    src += 36 * e0;
-    dst += 36 * e0;
+    const int n = rowptr[i + 1] - rowptr[i];
+    src += 36 * (padded ? (size_t)i * kPrunedCap : (size_t)rowptr[i]);
+    dst += 36 * (size_t)rowptr[i];
     for (int t = threadIdx.x & 31; t < 36 * n; t += 32) {
         const int r = t / (6 * n), k = t - r * 6 * n, e = k / 6, c = k - 6 * e;
         dst[t] = src[36 * e + 6 * r + c];
     }
 }
 
-// Brings the copies up to date with G, and with A for the polynomial.
-int bsr_sync(fsd_handle* h, bool with_a) {
+// A caller's blocks (checked, g_rowptr in place) into G.  They may lie on
+// another device, so they are fetched by a copy first.
+int bsr_import(fsd_handle* h, int nnzb, const float* blocks) {
     LearnedState* s = learned(h);
-    const int N = h->p.N, grid = (N + 7) / 8;
-    if (s->g_dirty) {
-        if (!s->g_comp) FSD_CHECK_CUDA(cudaMalloc(&s->g_comp, sizeof(float) * 36 * (size_t)s->g_cap));
+    if (nnzb == 0) return FSD_OK;
+    const size_t bytes = sizeof(float) * 36 * (size_t)nnzb;
+    float* tmp = nullptr;
+    FSD_CHECK_CUDA(cudaMalloc(&tmp, bytes));
+    cudaError_t e = cudaMemcpyAsync(tmp, blocks, bytes, cudaMemcpyDeviceToDevice, h->stream);
+    if (e == cudaSuccess) {
         count_launch();
-        k_bsr_layout<<<grid, 256, 0, h->stream>>>(s->g_rowptr, nullptr, N, s->g_val, s->g_comp);
-        s->g_dirty = false;
+        k_bsr_layout<<<(h->p.N + 7) / 8, 256, 0, h->stream>>>(s->g_rowptr, false, h->p.N, tmp, s->g_val);
+        e = cudaGetLastError();
     }
-    if (with_a && s->a_dirty && s->a_blocks) {
-        if (!s->a_comp) FSD_CHECK_CUDA(cudaMalloc(&s->a_comp, sizeof(float) * 36 * (size_t)N * kPrunedCap));
-        count_launch();
-        k_bsr_layout<<<grid, 256, 0, h->stream>>>(nullptr, s->a_pn, N, s->a_blocks, s->a_comp);
-        s->a_dirty = false;
+    cudaFree(tmp);  // waits for the copy and the layout
+    FSD_CHECK_CUDA(e);
+    return FSD_OK;
+}
+
+// Brings the polynomial's copy of A up to date: only the blocks that the
+// pruned list holds (25 MB of its 151 MB of padded rows at N = 32768, phi = 0.4).
+int bsr_sync_a(fsd_handle* h) {
+    LearnedState* s = learned(h);
+    const int N = h->p.N;
+    cudaStream_t st = h->stream;
+    if (!s->a_dirty || !s->a_blocks) return FSD_OK;
+    if (!s->a_rowptr) {
+        FSD_CHECK_CUDA(cudaMalloc(&s->a_rowptr, sizeof(int) * (N + 1)));
+        FSD_CHECK_CUDA(cudaMalloc(&s->a_scan, sizeof(unsigned) * scan_scratch_elems(N)));
     }
+    exclusive_scan(s->a_pn, (unsigned*)s->a_rowptr, N, s->a_scan, st);
+    int nnzb = 0;
+    FSD_CHECK_CUDA(cudaMemcpyAsync(&nnzb, s->a_rowptr + N, sizeof(int), cudaMemcpyDeviceToHost, st));
+    FSD_CHECK_CUDA(cudaStreamSynchronize(st));
+    if (nnzb > s->a_cap) {
+        if (s->a_comp) cudaFree(s->a_comp);
+        s->a_comp = nullptr;
+        s->a_cap = 0;
+        const int cap = nnzb + nnzb / 8 + 1024;
+        FSD_CHECK_CUDA(cudaMalloc(&s->a_comp, sizeof(float) * 36 * (size_t)cap));
+        s->a_cap = cap;
+    }
+    count_launch();
+    k_bsr_layout<<<(N + 7) / 8, 256, 0, st>>>(s->a_rowptr, true, N, s->a_blocks, s->a_comp);
     FSD_CHECK_CUDA(cudaGetLastError());
+    s->a_dirty = false;
     return FSD_OK;
 }
 
@@ -75,19 +103,9 @@ __global__ void __launch_bounds__(256) k_bsr_rows(BsrArgs a) {
             e_c = a.B2 ? a.B2[i6] : 0.f;
         }
     }
-    const float* row;
-    const int* cols;
-    int n;
-    if (MODE == kBsrStep) {  // A: padded rows of the pruned list
-        row = a.val + 36 * (size_t)i * kPrunedCap;
-        cols = a.col + (size_t)i * kPrunedCap;
-        n = have ? (int)a.pn[i] : 0;
-    } else {
-        const int q0 = a.rowptr[i];
-        row = a.val + 36 * (size_t)q0;
-        cols = a.col + q0;
-        n = have ? a.rowptr[i + 1] - q0 : 0;
-    }
+    const int q0 = a.rowptr[i], n = have ? a.rowptr[i + 1] - q0 : 0;
+    const float* row = a.val + 36 * (size_t)q0;
+    const int* cols = a.col + (MODE == kBsrStep ? (size_t)i * kPrunedCap : (size_t)q0);  // A: the padded pruned list
     float acc;
     if constexpr (MODE == kBsrFirst || MODE == kBsrOnce)
         acc = bsr_row(row, cols, n, BsrSaddle{MODE == kBsrFirst ? a.x : a.b, offU});

@@ -1,5 +1,5 @@
 // Block-sparse row products for the learned preconditioner (6x6 fp32 blocks):
-// 16 or 32 lanes per row, on a copy of the matrix laid out by components.
+// 16 or 32 lanes per row, on a matrix laid out by components.
 //
 // Row i with n blocks is 36 n contiguous floats; component r of the row's
 // result is the dot product of 6 n consecutive floats (r 6n + 6 e + c for block

@@ -7,12 +7,12 @@
 
 namespace fsd {
 
-// Fused block-sparse products (bsr_rows.cu) on the copies of G (block
-// CSR, rowptr) and A (padded pruned-list rows, pn) that fsd_bsr.cuh lays out.
+// Fused block-sparse products (bsr_rows.cu) on rows of blocks by components
+// (fsd_bsr.cuh): G, with its columns at rowptr, and the copy of A, whose columns
+// are the padded pruned list.
 enum { kBsrFirst = 0, kBsrPlain = 1, kBsrLast = 2, kBsrStep = 3, kBsrOnce = 4 };
 struct BsrArgs {
     const int* rowptr;
-    const unsigned* pn;
     const int* col;
     const float* val;
     int N;
@@ -30,10 +30,12 @@ struct BsrArgs {
 const void* bsr_kernel(int mode);
 int bsr_blocks(int N);
 void bsr_launch(int mode, const BsrArgs& a, cudaStream_t st);
-int bsr_sync(fsd_handle* h, bool with_a);
+int bsr_import(fsd_handle* h, int nnzb, const float* blocks);
+int bsr_sync_a(fsd_handle* h);
 
 struct LearnedState {
-    // G in block-CSR over particles (original order), 6x6 row-major fp32 blocks
+    // G in block-CSR over particles (original order): 6x6 fp32 blocks, each row's
+    // 36 n floats by components (fsd_bsr.cuh)
     int* g_rowptr = nullptr;
     int* g_col = nullptr;
     float* g_val = nullptr;
@@ -43,11 +45,13 @@ struct LearnedState {
     const unsigned* a_pn = nullptr;
     const unsigned* a_plist = nullptr;
     const float* a_blocks = nullptr;
-    // copies for the row products (fsd_bsr.cuh), rewritten before the next
-    // application after G or A changed
-    float* g_comp = nullptr;
+    // its copy by components for the polynomial (a_rowptr: offsets in blocks),
+    // rewritten by the build, or before the next application after it changed
+    int* a_rowptr = nullptr;
+    unsigned* a_scan = nullptr;
     float* a_comp = nullptr;
-    bool g_dirty = true, a_dirty = true;
+    int a_cap = 0;
+    bool a_dirty = true;
     // inner GMRES work space
     int inner_cap = -1;
     float* Vi = nullptr;      // kMaxInner x 6N basis U_j, unnormalised, then A z of the current step

@@ -33,7 +33,7 @@ void learned_free(fsd_handle* h) {
     LearnedState* s = (LearnedState*)h->learned;
     if (!s) return;
     mpnn_free(h);
-    void* ptrs[] = {s->g_comp, s->a_comp, s->g_rowptr, s->g_col,   s->g_val,     s->Vi,        s->Zi,        s->part,   s->H,
+    void* ptrs[] = {s->a_rowptr, s->a_scan, s->a_comp, s->g_rowptr, s->g_col,   s->g_val,     s->Vi,        s->Zi,        s->part,   s->H,
                     s->nrm,      s->ticket,  s->sp_sets,   s->sp_size,   s->sp_rowptr, s->sp_scan, s->sp_bucket,
                     s->sp_cnt};
     for (void* p : ptrs)
@@ -55,10 +55,8 @@ int learned_reserve(fsd_handle* h, int nnzb) {
     if (nnzb + 8 > s->g_cap) {
         if (s->g_col) cudaFree(s->g_col);
         if (s->g_val) cudaFree(s->g_val);
-        if (s->g_comp) cudaFree(s->g_comp);
         s->g_col = nullptr;
         s->g_val = nullptr;
-        s->g_comp = nullptr;
         s->g_cap = 0;
         // headroom, so that pattern growth from step to step rarely reallocates
         const int cap = nnzb + nnzb / 8 + 1024;
@@ -89,16 +87,12 @@ int learned_set_blocks(fsd_handle* h, int nnzb, const int* d_rowptr, const int* 
     if (e != FSD_OK) return e;
     LearnedState* s = learned(h);
     FSD_CHECK_CUDA(cudaMemcpyAsync(s->g_rowptr, d_rowptr, sizeof(int) * (N + 1), cudaMemcpyDeviceToDevice, h->stream));
-    if (nnzb) {
+    if (nnzb)
         FSD_CHECK_CUDA(cudaMemcpyAsync(s->g_col, d_col, sizeof(int) * (size_t)nnzb, cudaMemcpyDeviceToDevice,
                                        h->stream));
-        FSD_CHECK_CUDA(cudaMemcpyAsync(s->g_val, d_val, sizeof(float) * 36 * (size_t)nnzb, cudaMemcpyDeviceToDevice,
-                                       h->stream));
-    }
     s->g_nnzb = nnzb;
-    s->g_dirty = true;
     s->g_user = true;
-    return FSD_OK;
+    return bsr_import(h, nnzb, d_val);
 }
 
 // ----------------------------------------------------------- inner solve
@@ -144,7 +138,7 @@ constexpr int kInnerRowBlocks = 4 * 148;  // at most: every block resident, its 
 constexpr int kInnerThreads = 256;
 constexpr int kBetaSlot = (kMaxInner + 1) * kMaxInner;  // in H: beta, then the k coefficients
 
-// Z_j = G U_j, a warp per row on G's copy by components, and |U_j|; FIRST:
+// Z_j = G U_j, a warp per row on G by components, and |U_j|; FIRST:
 // U_0 = b[0:6N] - b[11N:17N], taken from b in the gathers too.
 template <bool FIRST>
 __global__ void __launch_bounds__(kInnerThreads, 4) k_inner_g(const int* rowptr, const int* col,
@@ -412,7 +406,7 @@ static int inner_enqueue(fsd_handle* h, const float* b, float* x, cudaStream_t s
     const size_t n6 = 6 * (size_t)N;
     const int rows = inner_rows(N), warps = inner_warps(N);
     const int pairs = (int)((n6 / 2 + kInnerThreads - 1) / kInnerThreads);
-    launch_pdl(k_inner_g<true>, warps, kInnerThreads, 0, st, s->g_rowptr, s->g_col, s->g_comp, b, s->Vi, s->Zi, N,
+    launch_pdl(k_inner_g<true>, warps, kInnerThreads, 0, st, s->g_rowptr, s->g_col, s->g_val, b, s->Vi, s->Zi, N,
                                                     s->H + kBetaSlot, s->nrm, s->part, s->ticket);
     for (int j = 0; j < k; ++j) {
         double* hj = s->H + (size_t)j * (kMaxInner + 1);
@@ -421,7 +415,7 @@ static int inner_enqueue(fsd_handle* h, const float* b, float* x, cudaStream_t s
                                                   s->part, s->ticket, s->H, j, N);
         if (j == k - 1) break;
         launch_pdl(k_inner_orth, pairs, kInnerThreads, 0, st, s->Vi, n6, j + 1, hj, s->nrm);
-        launch_pdl(k_inner_g<false>, warps, kInnerThreads, 0, st, s->g_rowptr, s->g_col, s->g_comp, b, s->Vi + (j + 1) * n6,
+        launch_pdl(k_inner_g<false>, warps, kInnerThreads, 0, st, s->g_rowptr, s->g_col, s->g_val, b, s->Vi + (j + 1) * n6,
                                                          zj + n6, N, hj + j + 1, s->nrm + j + 1, s->part, s->ticket);
     }
     launch_inner_last(k, st, s->Vi, n6, s->H, s->nrm, s->part, s->ticket);
@@ -437,7 +431,7 @@ static int inner_kernels(int k) { return 3 * k + 1; }
 // x) are kept so that each application can point them at its own vectors.
 static int inner_graph(fsd_handle* h, const float* b, float* x) {
     LearnedState* s = learned(h);
-    const void* key[8] = {s->g_rowptr, s->g_col, s->g_comp, s->a_pn, s->a_plist, s->a_blocks, s->Vi, s->Zi};
+    const void* key[8] = {s->g_rowptr, s->g_col, s->g_val, s->a_pn, s->a_plist, s->a_blocks, s->Vi, s->Zi};
     bool same = s->gexec && s->gkey_k == h->p.learned_inner;
     for (int i = 0; i < 8 && same; ++i) same = key[i] == s->gkey[i];
     if (same) return FSD_OK;
@@ -492,7 +486,7 @@ static int inner_bind(fsd_handle* h, const float* b, float* x) {
     int N = h->p.N;
     size_t ld = 6 * (size_t)N;
     double* beta = s->H + kBetaSlot;
-    void* rhs_args[] = {&s->g_rowptr, &s->g_col, &s->g_comp, &b,       &s->Vi,    &s->Zi,
+    void* rhs_args[] = {&s->g_rowptr, &s->g_col, &s->g_val, &b,       &s->Vi,    &s->Zi,
                         &N,           &beta,     &s->nrm,   &s->part, &s->ticket};
     cudaKernelNodeParams kr = {};
     kr.func = (void*)k_inner_g<true>;
@@ -526,13 +520,11 @@ int precond_apply_learned(fsd_handle* h, const float* b, float* x) {
     cudaStream_t st = h->stream;
     if (poly_active(h)) return poly_apply(h, b, x);
     const int k = h->p.learned_inner;
-    int e = bsr_sync(h, false);  // after user-set blocks; built ones are in place
-    if (e != FSD_OK) return e;
     if (k == 0) {
         BsrArgs a{};
         a.rowptr = s->g_rowptr;
         a.col = s->g_col;
-        a.val = s->g_comp;
+        a.val = s->g_val;
         a.N = N;
         a.b = b;
         a.xs = x;
@@ -541,7 +533,7 @@ int precond_apply_learned(fsd_handle* h, const float* b, float* x) {
         FSD_CHECK_CUDA(cudaGetLastError());
         return FSD_OK;
     }
-    e = inner_graph(h, b, x);
+    int e = inner_graph(h, b, x);
     if (e != FSD_OK) return e;
     e = inner_bind(h, b, x);
     if (e != FSD_OK) return e;
@@ -604,10 +596,6 @@ int precond_build_learned(fsd_handle* h, const float4* pos) {
             e = mpnn_poly_calibrate(h, h->p.learned_poly, ++s->poly_builds);
             if (e != FSD_OK) return e;
         }
-    }
-    if (!poly) {
-        e = bsr_sync(h, false);
-        if (e != FSD_OK) return e;
     }
     h->pc_valid = true;
     return FSD_OK;

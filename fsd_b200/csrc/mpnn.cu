@@ -390,8 +390,8 @@ __device__ __forceinline__ void axis_block_grad(const float* dB, float3 r, float
     for (int k = 0; k < 6; ++k) go[k] = g[k];
 }
 
-// Correction added to G (block CSR of the two-hop sets; row i = [self,
-// edges of i]).  One thread per row.
+// Correction added to G (block CSR of the two-hop sets by components; row i =
+// [self, edges of i]).  One thread per row.
 __global__ void k_head_blocks(const unsigned* __restrict__ rowptr, const float4* __restrict__ rhat,
                               const float* __restrict__ oe, const float* __restrict__ on, const float* __restrict__ J,
                               int N, float* G) {
@@ -399,6 +399,7 @@ __global__ void k_head_blocks(const unsigned* __restrict__ rowptr, const float4*
     if (i >= N) return;
     const unsigned b = rowptr[i], e = rowptr[i + 1];
     const size_t base = (size_t)b + i;
+    const int ld = 6 * (int)(1 + e - b);  // of a component's run in the row
     float Ji[36];
     for (int k = 0; k < 36; ++k) Ji[k] = J[(size_t)i * 36 + k];
     float S[36];
@@ -412,12 +413,12 @@ __global__ void k_head_blocks(const unsigned* __restrict__ rowptr, const float4*
         axis_block(oe + (size_t)f * kMpHeadE + 6, r, B);
         for (int k = 0; k < 36; ++k) S[k] += B[k];
         axis_block(oe + (size_t)f * kMpHeadE, r, B);
-        float* out = G + (base + 1 + (f - b)) * 36;
+        float* out = G + base * 36 + 6 * (1 + (f - b));
         for (int a = 0; a < 6; ++a)
             for (int c = 0; c < 6; ++c) {
                 float s = 0.f;
                 for (int q = 0; q < 6; ++q) s += Ji[a * 6 + q] * B[q * 6 + c];
-                out[a * 6 + c] += s;
+                out[a * ld + c] += s;
             }
     }
     float* out = G + base * 36;
@@ -425,7 +426,7 @@ __global__ void k_head_blocks(const unsigned* __restrict__ rowptr, const float4*
         for (int c = 0; c < 6; ++c) {
             float s = 0.f;
             for (int q = 0; q < 6; ++q) s += Ji[a * 6 + q] * S[q * 6 + c];
-            out[a * 6 + c] += s;
+            out[a * ld + c] += s;
         }
 }
 
@@ -472,7 +473,7 @@ __global__ void k_head_bwd(const unsigned* __restrict__ rowptr, const float4* __
 }
 
 // ------------------------------------------------------------------ loss
-// u = G Z for P probe columns stored probe-major (P x 6N).
+// u = G Z (G by components) for P probe columns stored probe-major (P x 6N).
 __global__ void k_bsr_multi(const int* __restrict__ rowptr, const int* __restrict__ col, const float* __restrict__ G,
                             const float* __restrict__ Z, float* __restrict__ U, int N, int P) {
     const int gid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -480,12 +481,14 @@ __global__ void k_bsr_multi(const int* __restrict__ rowptr, const int* __restric
     if (i >= N) return;
     const unsigned gmask = 0xffu << (threadIdx.x & 24);
     const size_t n6 = 6 * (size_t)N;
+    const int e0 = rowptr[i], e1 = rowptr[i + 1];
+    const float* Gr = G + (size_t)e0 * 36 + (r < 6 ? r : 0) * 6 * (size_t)(e1 - e0);
     for (int p = 0; p < P; ++p) {
         float acc = 0.f;
-        for (int e = rowptr[i]; e < rowptr[i + 1]; ++e) {
+        for (int e = e0; e < e1; ++e) {
             const int j = col[e];
             const float xj = (r < 6) ? Z[p * n6 + 6 * j + r] : 0.f;
-            const float* Ge = G + (size_t)e * 36 + (r < 6 ? r : 0) * 6;
+            const float* Ge = Gr + 6 * (e - e0);
 #pragma unroll
             for (int c = 0; c < 6; ++c) {
                 const float xc = __shfl_sync(gmask, xj, c, 8);
@@ -895,7 +898,6 @@ static int mp_head(fsd_handle* h) {
     const int N = s->N;
     count_launch();
     k_head_blocks<<<(N + 127) / 128, 128, 0, h->stream>>>(s->cnt, s->rhat, s->oe, s->on, s->J, N, ls->g_val);
-    ls->g_dirty = true;
     FSD_CHECK_CUDA(cudaGetLastError());
     return FSD_OK;
 }

@@ -43,7 +43,7 @@ constexpr int kPowerBlocks = 6 * 148;
 __global__ void k_set_double(double* p, double v) { *p = v; }
 
 // W = A U, |W| into nrm[0] and kLambdaMargin |W| into pc[kMaxPoly] by the last block.
-__global__ void __launch_bounds__(256) k_power_a(const unsigned* __restrict__ pn, const int* __restrict__ plist,
+__global__ void __launch_bounds__(256) k_power_a(const int* __restrict__ rowptr, const int* __restrict__ plist,
                                                  const float* __restrict__ A, const float* __restrict__ U, int N,
                                                  float* __restrict__ W, double* part, unsigned* ticket, double* nrm,
                                                  float* pc) {
@@ -54,7 +54,8 @@ __global__ void __launch_bounds__(256) k_power_a(const unsigned* __restrict__ pn
         const int q = t0 * kBsrRows + bsr_sub();
         const bool have = q < N;
         const int i = have ? q : 0;
-        const float acc = bsr_row(A + 36 * (size_t)i * kPrunedCap, plist + (size_t)i * kPrunedCap, have ? (int)pn[i] : 0,
+        const int q0 = rowptr[i];
+        const float acc = bsr_row(A + 36 * (size_t)q0, plist + (size_t)i * kPrunedCap, have ? rowptr[i + 1] - q0 : 0,
                                   BsrPlain{U});
         if (have && rc >= 0) {
             W[6 * (size_t)i + rc] = acc;
@@ -116,7 +117,7 @@ int poly_lambda(fsd_handle* h) {
     cudaStream_t st = h->stream;
     float* W = s->pbuf;
     float* U = s->pbuf + n6;
-    const int e = bsr_sync(h, true);
+    const int e = bsr_sync_a(h);
     if (e != FSD_OK) return e;
     const int rows = bsr_blocks(N), arows = std::min(rows, kPowerBlocks);
     gaussian(h, W, n6, 1, kStreamGain, 1.0f);
@@ -124,10 +125,10 @@ int poly_lambda(fsd_handle* h) {
     k_set_double<<<1, 1, 0, st>>>(s->pnrm, std::sqrt((double)n6));
     for (int it = 0; it < kPowerIters; ++it) {
         count_launch();
-        k_power_g<<<rows, 256, 0, st>>>(s->g_rowptr, s->g_col, s->g_comp, W, s->pnrm, N, U);
+        k_power_g<<<rows, 256, 0, st>>>(s->g_rowptr, s->g_col, s->g_val, W, s->pnrm, N, U);
         count_launch();
-        k_power_a<<<arows, 256, 0, st>>>(s->a_pn, (const int*)s->a_plist, s->a_comp, U, N, W, s->ppart, s->pticket, s->pnrm,
-                                        s->pc);
+        k_power_a<<<arows, 256, 0, st>>>(s->a_rowptr, (const int*)s->a_plist, s->a_comp, U, N, W, s->ppart, s->pticket,
+                                         s->pnrm, s->pc);
     }
     FSD_CHECK_CUDA(cudaGetLastError());
     return FSD_OK;
@@ -152,7 +153,7 @@ static BsrArgs g_args(const LearnedState* s, int N) {
     BsrArgs a{};
     a.rowptr = s->g_rowptr;
     a.col = s->g_col;
-    a.val = s->g_comp;
+    a.val = s->g_val;
     a.N = N;
     a.pc = s->pc;
     return a;
@@ -160,7 +161,7 @@ static BsrArgs g_args(const LearnedState* s, int N) {
 
 static BsrArgs a_args(const LearnedState* s, int N) {
     BsrArgs a{};
-    a.pn = s->a_pn;
+    a.rowptr = s->a_rowptr;
     a.col = (const int*)s->a_plist;
     a.val = s->a_comp;
     a.N = N;
@@ -229,8 +230,8 @@ static int poly_kernels(int k) { return 2 * k - 1; }
 
 static int poly_graph(fsd_handle* h, const float* b, float* x) {
     LearnedState* s = learned(h);
-    const void* key[10] = {s->g_rowptr, s->g_col,  s->g_comp, s->a_pn, s->a_plist,
-                           s->a_comp, s->pbuf, s->pc,    nullptr, nullptr};
+    const void* key[10] = {s->g_rowptr, s->g_col, s->g_val, s->a_rowptr, s->a_plist,
+                           s->a_comp,   s->pbuf,  s->pc,    nullptr,     nullptr};
     bool same = s->pexec && s->pkey_k == h->p.learned_poly;
     for (int i = 0; i < 10 && same; ++i) same = key[i] == s->pkey[i];
     if (same) return FSD_OK;
@@ -298,7 +299,7 @@ static int poly_bind(fsd_handle* h, const float* b, float* x) {
 
 int poly_apply(fsd_handle* h, const float* b, float* x) {
     LearnedState* s = learned(h);
-    int e = bsr_sync(h, true);
+    int e = bsr_sync_a(h);
     if (e != FSD_OK) return e;
     e = poly_graph(h, b, x);
     if (e != FSD_OK) return e;

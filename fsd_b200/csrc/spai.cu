@@ -336,8 +336,8 @@ __global__ void __launch_bounds__(32 * WARPS) k_spai_solve(const unsigned* __res
         }
         __syncthreads();
     }
-    // Column c of G: block (s_a, c) = X block a, stored in row s_a at the
-    // position of c in that row's set (the sets are mutual unless one was
+    // Column c of G: block (s_a, c) = X block a, stored (by components) in row s_a
+    // at the position of c in that row's set (the sets are mutual unless one was
     // truncated; a block without a slot is dropped).  A failed factorisation
     // (never expected: the normal matrix of a full-rank A[:, S] is SPD) leaves
     // the block-Jacobi inverse in column c.
@@ -347,9 +347,10 @@ __global__ void __launch_bounds__(32 * WARPS) k_spai_solve(const unsigned* __res
             const int* Ss = sets + (size_t)sa * kSpaiCap;
             const unsigned hit = __ballot_sync(0xffffffffu, lane < (int)ns[sa] && Ss[lane] == c);
             if (!hit) continue;
-            float* out = g_val + (size_t)(rowptr[sa] + __ffs(hit) - 1) * 36;
+            float* out = g_val + (size_t)rowptr[sa] * 36 + 6 * (__ffs(hit) - 1);
+            const int ld = 6 * (int)ns[sa];
             const double* X = H + tri_block(m, a);
-            for (int k = lane; k < 36; k += 32) out[k] = (float)X[6 * (k % 6) + k / 6];
+            for (int k = lane; k < 36; k += 32) out[(k / 6) * ld + k % 6] = (float)X[6 * (k % 6) + k / 6];
         }
     } else if (threadIdx.x == 0) {
         atomicAdd(fail, 1);
@@ -367,7 +368,7 @@ __global__ void __launch_bounds__(32 * WARPS) k_spai_solve(const unsigned* __res
                 }
         }
         for (int r = 0; r < 6; ++r)
-            for (int q = 0; q < 6; ++q) g_val[(size_t)rowptr[c] * 36 + r * 6 + q] = (float)M[r][6 + q];
+            for (int q = 0; q < 6; ++q) g_val[(size_t)rowptr[c] * 36 + r * 6 * m + q] = (float)M[r][6 + q];
     }
 }
 
@@ -432,7 +433,6 @@ int spai_build(fsd_handle* h) {
     if (es != FSD_OK) return es;
     FSD_CHECK_CUDA(cudaGetLastError());
     s->g_nnzb = nnzb;
-    s->g_dirty = true;
     return FSD_OK;
 }
 
