@@ -1253,18 +1253,18 @@ __global__ void __launch_bounds__(256) k_contract(const float4* pos, const unsig
         ix -= (ix >= Nx) ? Nx : 0;
         iy -= (iy >= Ny) ? Ny : 0;
         iz -= (iz >= Nz) ? Nz : 0;
-        const float2* gp = grid + ((size_t)ix * Ny + iy) * Nz + iz;
         float2 q0, q1, q2, q3, q4, q5;  // (Ux,Uy) (XX,XY) (XZ,YX) (YY,YZ) (ZX,ZY) (Uz,-)
         auto nodes = [&] {
-            q0 = gp[0];
-            q1 = gp[G];
-            q2 = gp[2 * G];
-            q3 = gp[3 * G];
-            q4 = gp[4 * G];
-            q5 = gp[5 * G];
+            const size_t g = ((size_t)ix * Ny + iy) * Nz + iz;
+            q0 = grid[g];
+            q1 = grid[G + g];
+            q2 = grid[2 * G + g];
+            q3 = grid[3 * G + g];
+            q4 = grid[4 * G + g];
+            q5 = grid[5 * G + g];
         };
         // ahead of the weight where the loop is not unrolled (P = 8, N = 7351: 30 us against 36 behind it; P = 6,
-        // N = 32768: 46 against 45)
+        // N = 32768: 46 against 43)
         if (KP == 0) nodes();
         float3 r;
         if (local) {
