@@ -12,6 +12,7 @@
 #include "fsd_mpnn.h"
 #include "fsd_solver.h"
 #include "fsd_profile.h"
+#include "fsd_spread.h"
 #include "fsd_wavefft.h"
 
 namespace fsd {
@@ -81,7 +82,7 @@ static int allocate(fsd_handle* h) {
     FSD_TRY(dalloc(&w.order, N));
     FSD_TRY(dalloc(&w.lub_n, N));
     FSD_TRY(init_particle_order(h));
-    const size_t ncol = (size_t)h->g.Nx * h->g.Ny;
+    const size_t ncol = bin_columns(h->g);
     FSD_TRY(dalloc(&w.bin_key, 2 * (size_t)N));
     FSD_TRY(dalloc(&w.bin_items, N));
     const size_t ncol_pad = (ncol + 15) & ~(size_t)15;  // scanned in runs of 16

@@ -90,7 +90,7 @@ struct Workspace {
     // particles binned by spreading-stencil origin (one bin per grid node)
     uint2* bin_key = nullptr;      // (column, slot) and (z, -) of each particle's stencil origin
     uint2* bin_items = nullptr;    // (z, particle) by column, unsorted within it
-    unsigned* col_count = nullptr; // per (x, y) column, zero between calls
+    unsigned* col_count = nullptr; // per column (bin_columns), zero between calls
     unsigned* col_start = nullptr;
     unsigned* bin_ticket = nullptr;
     unsigned* bin_start = nullptr; // first member of each node's bin

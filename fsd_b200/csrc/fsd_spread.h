@@ -1,4 +1,5 @@
-// Which spreading kernel runs, and on what tile (host code; mobility.cu).
+// Which spreading kernel runs, on what tile, and the columns particles are
+// binned by (host code; mobility.cu).
 #pragma once
 
 #include <math.h>
@@ -8,6 +9,15 @@
 #include "fsd_internal.h"
 
 namespace fsd {
+
+// Binning columns: one per (x, y) up to 160 nodes along z, else as many pieces of
+// equal length at most that.  A warp ranks a column's members against one another
+// and counts them once per 32 nodes, so its work grows with the square of the
+// length: with whole columns of 1563 nodes and 78 members (16 x 16 x 1563,
+// N = 20000) a wave-space product takes 464 us, with pieces 382.
+inline int bin_pieces(int Nz) { return (Nz + 159) / 160; }
+inline int bin_piece_nodes(int Nz) { return (Nz + bin_pieces(Nz) - 1) / bin_pieces(Nz); }
+inline size_t bin_columns(const GridParams& g) { return (size_t)g.Nx * g.Ny * bin_pieces(g.Nz); }
 
 enum { kSpreadBlocks = 0, kSpreadRows = 1, kSpreadFour = 2 };  // TuneChoice::spread_rows
 

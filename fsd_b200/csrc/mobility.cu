@@ -587,27 +587,29 @@ __device__ __forceinline__ int3 stencil_origin(float4 p, const Box& b, int Nx, i
 }
 
 // Particles binned by stencil origin (x, y, z), one bin per grid node, each
-// bin's members by index.  Three launches: the (x, y) column of each origin is
-// counted (the last block scans the columns), particles drop into their
-// column, and a warp per column ranks its members by (z, index) and writes the
-// bin starts of the column's Nz nodes, so no pass over all nodes is scanned
-// (at 72^3: 5184 columns instead of 373248 bins; 18 -> 9 us for nine launches
-// before).
+// bin's members by index.  Three launches: the (x, y) column of each origin (a
+// piece of it on long axes, bin_pieces) is counted (the last block scans the
+// columns), particles drop into their column, and a warp per column ranks its
+// members by (z, index) and writes the bin starts of the column's nodes, so no
+// pass over all nodes is scanned (at 72^3: 5184 columns instead of 373248 bins;
+// 18 -> 9 us for nine launches before).
+template <bool PIECES>
 __global__ void __launch_bounds__(1024) k_col_count(const float4* pos, int N, Box b, int Nx, int Ny, int Nz,
-                                                    int P, uint2* part, unsigned* col_count,
+                                                    int P, int pieces, int zs, uint2* part, unsigned* col_count,
                                                     unsigned* col_start, unsigned* ticket) {
     pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < N) {
         const int3 s = stencil_origin(pos[i], b, Nx, Ny, Nz, P, nullptr);
-        const unsigned col = (unsigned)(s.x * Ny + s.y);
+        unsigned col = (unsigned)(s.x * Ny + s.y);
+        if (PIECES) col = col * pieces + s.z / zs;
         const unsigned slot = atomicAdd(&col_count[col], 1u);
         part[2 * (size_t)i] = make_uint2(col, slot);
         part[2 * (size_t)i + 1] = make_uint2((unsigned)s.z, 0u);
     }
     __threadfence();
     if (!last_block(ticket)) return;
-    block_scan_counts(col_count, col_start, Nx * Ny);
+    block_scan_counts(col_count, col_start, PIECES ? Nx * Ny * pieces : Nx * Ny);
     if (threadIdx.x == 0) *ticket = 0;
 }
 
@@ -625,8 +627,9 @@ __global__ void k_col_fill(const uint2* part, int N, const unsigned* col_start, 
 
 // One warp per column.  A member's place is the number of members below it in
 // (z, index); each lane then finds the starts of its share of the nodes.
+template <bool PIECES>
 __global__ void __launch_bounds__(256) k_col_sort(const float4* pos, const unsigned* col_start,
-                                                  int ncol, int Nz, const uint2* items,
+                                                  int ncol, int Nz, int pieces, int zs, const uint2* items,
                                                   unsigned* bin_parts, unsigned* bin_start,
                                                   float4* sorted_pos) {
     pdl_wait();
@@ -645,26 +648,33 @@ __global__ void __launch_bounds__(256) k_col_sort(const float4* pos, const unsig
         bin_parts[s0 + rank] = me.y;
         sorted_pos[s0 + rank] = make_float4(p.x, p.y, p.z, __uint_as_float(me.x));
     }
-    for (int z = lane; z < Nz; z += 32) {
+    int xy = c, z0 = 0;
+    if (PIECES) {
+        xy = c / pieces;
+        z0 = (c - xy * pieces) * zs;
+    }
+    const int z1 = PIECES ? min(Nz, z0 + zs) : Nz;
+    for (int z = z0 + lane; z < z1; z += 32) {
         unsigned below = 0;
         for (unsigned k = 0; k < n; ++k) below += items[s0 + k].x < (unsigned)z ? 1u : 0u;
-        bin_start[(size_t)c * Nz + z] = s0 + below;
+        bin_start[(size_t)xy * Nz + z] = s0 + below;
     }
-    if (c == ncol - 1 && lane == 0) bin_start[(size_t)ncol * Nz] = s0 + n;
+    if (c == ncol - 1 && lane == 0) bin_start[(size_t)(xy + 1) * Nz] = s0 + n;
 }
 
 int mobility_bin_particles(fsd_handle* h, const float4* pos) {
     Workspace& w = h->w;
-    const int N = h->p.N, Nx = h->g.Nx, Ny = h->g.Ny, Nz = h->g.Nz, ncol = Nx * Ny;
+    const int N = h->p.N, Nx = h->g.Nx, Ny = h->g.Ny, Nz = h->g.Nz;
+    const int ncol = (int)bin_columns(h->g), pieces = bin_pieces(Nz), zs = bin_piece_nodes(Nz);
     count_launch();
-    launch_pdl(k_col_count, (N + 1023) / 1024, 1024, 0, h->stream, pos, N, h->box, Nx, Ny, Nz, h->g.P, w.bin_key, w.col_count,
-                                                          w.col_start, w.bin_ticket);
+    launch_pdl(pieces > 1 ? k_col_count<true> : k_col_count<false>, (N + 1023) / 1024, 1024, 0, h->stream, pos, N, h->box,
+               Nx, Ny, Nz, h->g.P, pieces, zs, w.bin_key, w.col_count, w.col_start, w.bin_ticket);
     count_launch();
     launch_pdl(k_col_fill, (std::max(N, ncol) + 255) / 256, 256, 0, h->stream, w.bin_key, N, w.col_start, ncol, w.col_count,
-                                                                      w.bin_items);
+               w.bin_items);
     count_launch();
-    launch_pdl(k_col_sort, (ncol + 7) / 8, 256, 0, h->stream, pos, w.col_start, ncol, Nz, w.bin_items, w.bin_parts, w.bin_start,
-                                                     w.bin_pos);
+    launch_pdl(pieces > 1 ? k_col_sort<true> : k_col_sort<false>, (ncol + 7) / 8, 256, 0, h->stream, pos, w.col_start, ncol,
+               Nz, pieces, zs, w.bin_items, w.bin_parts, w.bin_start, w.bin_pos);
     FSD_CHECK_CUDA(cudaGetLastError());
     return FSD_OK;
 }

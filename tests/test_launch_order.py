@@ -33,7 +33,7 @@ def functions(text):
 
 ALL = {(f, n): (k, s, b) for f, t in SOURCES.items() for k, n, s, b in functions(t)}
 OVERLAPPED = {k: v for k, v in ALL.items() if v[0] and "pdl_wait()" in v[2]}
-LAUNCHED = {m for t in SOURCES.values() for m in re.findall(r"launch_pdl\((k_\w+)", t)}
+LAUNCHED = {k for t in SOURCES.values() for m in re.findall(r"launch_pdl\(([^,]*)", t) for k in re.findall(r"\bk_\w+", m)}
 
 
 def test_every_overlapped_launch_is_of_a_kernel_that_waits_first():

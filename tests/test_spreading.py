@@ -62,7 +62,8 @@ def test_spread_uneven_bins(cuda, n, N, size, xy, err):
 
 @pytest.fixture(scope="module")
 def choose(tmp_path_factory):
-    """spread_choice of fsd_spread.h, compiled on its own: (TX, TY, TZ, form, local)."""
+    """fsd_spread.h compiled on its own: spread_choice as (TX, TY, TZ, form, local), then the binning columns as
+    (pieces of an axis, nodes per piece, columns)."""
     gxx, inc = shutil.which("g++"), Path(os.environ.get("CUDA_HOME", "/usr/local/cuda")) / "include"
     if gxx is None or not (inc / "cuda_runtime.h").exists():
         pytest.skip("no host compiler or CUDA headers")
@@ -75,6 +76,7 @@ extern "C" void choice(const int* grid, float xy, const int* tune, int* out) {
     t.TX = tune[0], t.TY = tune[1], t.TZ = tune[2], t.spread_rows = tune[3], t.set = tune[0] > 0;
     const fsd::SpreadChoice c = fsd::spread_choice(g, xy, t);
     out[0] = c.TX, out[1] = c.TY, out[2] = c.TZ, out[3] = c.form, out[4] = c.local;
+    out[5] = fsd::bin_pieces(g.Nz), out[6] = fsd::bin_piece_nodes(g.Nz), out[7] = (int)fsd::bin_columns(g);
 }
 """)
     csrc = Path(__file__).resolve().parents[1] / "fsd_b200" / "csrc"
@@ -83,10 +85,10 @@ extern "C" void choice(const int* grid, float xy, const int* tune, int* out) {
     f = C.CDLL(str(d / "choice.so")).choice
     f.argtypes = [C.POINTER(C.c_int), C.c_float, C.POINTER(C.c_int), C.POINTER(C.c_int)]
 
-    def call(grid, xy, tune=(0, 0, 0, 0)):
-        out = (C.c_int * 5)()
+    def call(grid, xy, tune=(0, 0, 0, 0), part=slice(5)):
+        out = (C.c_int * 8)()
         f((C.c_int * 4)(*grid), xy, (C.c_int * 4)(*tune), out)
-        return tuple(out)
+        return tuple(out)[part]
 
     return call
 
@@ -110,6 +112,46 @@ def test_four_nodes_per_lane_only_on_local_tiles(choose, tile):
                     assert got[3] != 2 or got[4]
                     left += 1
     assert kept and left
+
+
+def test_binning_columns_are_short(choose):
+    """A warp's work on a column grows with the square of its length: at most 160 nodes, in pieces that cover the
+    axis with none empty."""
+    for nz in range(12, 4000):
+        pieces, nodes, columns = choose((12, 16, nz, 6), 0.0, part=slice(5, 8))
+        assert nodes <= 160 and (pieces - 1) * nodes < nz <= pieces * nodes
+        assert columns == 12 * 16 * pieces
+        assert pieces == 1 or nz > 160
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("grid,N,size", [((12, 12, 162), 300, 1.0), ((15, 12, 432), 2000, 1.0), ((12, 12, 512), 900, 0.1),
+                                         ((12, 16, 324), 1500, 1.0)])
+def test_spread_on_axes_of_several_pieces(cuda, grid, N, size):
+    """Particles spread over the box, and clustered around the middle of the long axis, where pieces meet, and its
+    end, where they wrap.  Oracle and tolerance as for the other spreading tests, on axes short enough for it: the
+    Green function's sin k - k cos k in FP32 cancels to 3 eps / k^2, 1e-3 of the factors of the lowest mode at 500
+    nodes, which is 1e-5 of the product when particles fill the box."""
+    L = tuple(edge(n, 1e-3) for n in grid)
+    rng = np.random.default_rng(grid[2] + N)
+    frac = rng.random((N, 3)) - 0.5
+    frac[:, 2] = size * frac[:, 2] + (0.0 if size == 1.0 else np.where(np.arange(N) % 2, 0.5, 0.0))
+    frac -= np.floor(frac + 0.5)
+    pos = np.zeros((N, 4), np.float32)
+    pos[:, :3] = frac * np.array(L)
+    s = FSD(N, (*L, 0.0), xi=XI, gmres_restart=2, lanczos_max=4)
+    info = s.pse_info()
+    assert (info.Nx, info.Ny, info.Nz) == grid
+    F = torch.as_tensor(rng.standard_normal(11 * N).astype(np.float32)).cuda()
+    p = torch.as_tensor(pos).cuda().view(-1)
+    got = s.mobility(p, F, parts=1)
+    assert torch.equal(s.mobility(p, F, parts=1), got)
+    s.close()
+    gp = {k: getattr(info, k) for k in ("Nx", "Ny", "Nz", "P", "eta", "hx", "hy", "hz")}
+    Ff, Cp = O.split_generalized(F.cpu().numpy().astype(np.float64), N)
+    u, D = O.wave_space(pos, Ff, Cp, L, 0.0, gp, XI)
+    ref = O.generalized_velocity(u, np.transpose(D, (0, 2, 1)), N)
+    assert np.linalg.norm(got.cpu().numpy() - ref) / np.linalg.norm(ref) < 1e-5
 
 
 @pytest.mark.gpu
