@@ -61,8 +61,8 @@ def test_approximate_inverse_of_every_set_size(cuda, N):
 @pytest.mark.parametrize("N", [1, 2, 5, 31, 33, 257, 700])
 @pytest.mark.parametrize("xy", [0.0, -0.5])
 def test_pair_sums_of_small_and_odd_sizes(cuda, N, xy):
-    """Real-space mobility and the four lubrication products; the velocity also from an address that is a
-    multiple of four bytes only.  FP32 pair sums: 1e-6 expected, 1e-5 allowed."""
+    """Real-space mobility and the four lubrication products, with a strain of its own on every particle; the velocity
+    also from an address that is a multiple of four bytes only.  FP32 pair sums: 1e-6 expected, 1e-5 allowed."""
     pos = packed(N, 2.03, N)
     s, p = solver(pos, xy)
     pr = O.Problem(pos, L, xy, table=ewald_golden())
@@ -77,9 +77,20 @@ def test_pair_sums_of_small_and_odd_sizes(cuda, N, xy):
     odd = torch.zeros(6 * N + 1, device="cuda")
     odd[1:] = dev(U)
     assert torch.equal(s.rfu(p, odd[1:]), got)
-    sl = s.rsu(p, dev(U)).cpu().numpy()
-    assert torch.equal(s.rsu(p, odd[1:]).cpu(), torch.as_tensor(sl))
-    assert np.isfinite(sl).all() and np.isfinite(s.rfe(p, 0.7).cpu().numpy()).all()
+    sl = s.rsu(p, dev(U))
+    assert torch.equal(s.rsu(p, odd[1:]), sl)
+    ori = rng.standard_normal((N, 3))
+    ori = (ori / np.linalg.norm(ori, axis=1, keepdims=True)).astype(np.float32)
+    mask = rng.random(N).astype(np.float32)
+    active = dict(ori=ori, b2mask=mask, B2=-0.5)
+    args = (pr.L, xy, pr.rows, pr.tdist, pr.tvals)
+    for got, ref in ((sl, O.rsu(pos, U, *args)),
+                     (s.rfe(p, 0.7, dev(ori), dev(mask), -0.5), O.rfe(pos, 0.7, *args, **active)),
+                     (s.rse(p, 0.7, dev(ori), dev(mask), -0.5), O.rse(pos, 0.7, *args, **active))):
+        if N == 1:
+            assert not got.any() and not ref.any()
+        else:
+            assert rel(got.cpu(), ref) < 1e-5
     s.close()
 
 
