@@ -120,7 +120,7 @@ __device__ __forceinline__ double group_sum_d(double v) {
 
 // Last-block reduction: the threads that wrote this block's partials have
 // fenced them; the block that takes the last ticket sees every block's
-// partials and resets the ticket.
+// partials, and the caller resets the ticket there.
 __device__ __forceinline__ bool last_block(unsigned* ticket) {
     __shared__ bool last;
     __syncthreads();

@@ -512,8 +512,9 @@ static int inner_bind(fsd_handle* h, const float* b, float* x) {
 // k steps of GMRES on that matrix from a zero guess, right-preconditioned by
 // G; the map b -> x then depends on b nonlinearly, which the flexible outer
 // GMRES allows.  The inner solve is one CUDA graph launch reading b and
-// writing x directly; no host synchronisation.  b and x may be the same
-// vector.
+// writing x directly; no host synchronisation.  With inner steps or the
+// polynomial b and x may be the same vector; G applied once gathers from b
+// while it writes x, so they must not overlap.
 int precond_apply_learned(fsd_handle* h, const float* b, float* x) {
     LearnedState* s = learned(h);
     const int N = h->p.N;

@@ -19,9 +19,9 @@
 // lines elsewhere) and after: 72^3 y+z 21.6 -> 13.9 us forward, 12.8 us
 // inverse, x pass 51.4 -> 20.4 us; 120^3 y+z 249 -> 70 and 67 us, x pass
 // 318 -> 76 us; 27^3 y+z 5.6 -> 4.6 and 4.2 us, x pass 10.2 -> 4.6 us.
-// Lengths above 150, and those without two register-sized factors (125, 162),
-// keep the generic lines, as do boxes with Ny != Nz: their plane does not fit
-// in shared memory, or has no kernel here.
+// The generic lines are kept for lengths without two register-sized factors
+// (125, 162), for boxes with Ny != Nz and for lengths above 150: a plane of 160
+// (16 x 10, 220 KB) would be the last to fit in shared memory, and has no kernel.
 #include "fsd_device.cuh"
 #include "fsd_dft.cuh"
 #include "fsd_green.cuh"
