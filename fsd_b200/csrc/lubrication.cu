@@ -13,7 +13,7 @@
 // gathers per pair, 38 us per R_FU product at N = 32768, phi = 0.4 (30 to 55 us
 // for the others).  Each product's functions now sit in rows of 8 or 16 floats
 // with the row's distance, read in 32-byte loads, and a saddle product takes U
-// from packed records of 8: 27 us per R_FU product.
+// from packed records of 8: 28 us per R_FU product.
 #include "fsd_device.cuh"
 #include "fsd_kernels.cuh"
 #include "fsd_profile.h"

@@ -852,10 +852,12 @@ __device__ __forceinline__ void spread_stage(const SpreadArgs& a, const SpreadTi
 // Every node is written once with its contributions added in staged order: no
 // atomics, the same sums in every run.
 //
-// Issue-bound.  Walking the extended tile's cells twice per tile, one node per
-// lane and scalar products took 51 M warp instructions and 73 us per call at
-// N = 32768, 72^3 (264 us at N = 131072, 120^3); rows of bins and packed
-// products with one node per lane 34.5 M and 52 us (182 us).
+// Bound by issue (59 % of the cycles) and the wait of dependent multiply-adds,
+// with 29 % of the warps resident: 28 M warp instructions and 47 us per call at
+// N = 32768, 72^3.  Walking the extended tile's cells twice per tile, one node
+// per lane and scalar products took 51 M and 73 us (264 us at N = 131072,
+// 120^3); rows of bins and packed products with one node per lane 34.5 M and
+// 52 us (182 us).
 // Needs tile-relative separations, TX % 4 == 0, TY % 4 == 0, TZ % 8 == 0 and a
 // quarter of TX TY TZ threads.
 template <int KP>
