@@ -24,22 +24,12 @@ __global__ void __launch_bounds__(256) k_bsr_layout(const int* __restrict__ rowp
     }
 }
 
-// A caller's blocks (checked, g_rowptr in place) into G.  They may lie on
-// another device, so they are fetched by a copy first.
-int bsr_import(fsd_handle* h, int nnzb, const float* blocks) {
+// Blocks in block CSR (rowptr in place) into G.
+int bsr_import(fsd_handle* h, const float* blocks) {
     LearnedState* s = learned(h);
-    if (nnzb == 0) return FSD_OK;
-    const size_t bytes = sizeof(float) * 36 * (size_t)nnzb;
-    float* tmp = nullptr;
-    FSD_CHECK_CUDA(cudaMalloc(&tmp, bytes));
-    cudaError_t e = cudaMemcpyAsync(tmp, blocks, bytes, cudaMemcpyDeviceToDevice, h->stream);
-    if (e == cudaSuccess) {
-        count_launch();
-        k_bsr_layout<<<(h->p.N + 7) / 8, 256, 0, h->stream>>>(s->g_rowptr, false, h->p.N, tmp, s->g_val);
-        e = cudaGetLastError();
-    }
-    cudaFree(tmp);  // waits for the copy and the layout
-    FSD_CHECK_CUDA(e);
+    count_launch();
+    k_bsr_layout<<<(h->p.N + 7) / 8, 256, 0, h->stream>>>(s->g_rowptr, false, h->p.N, blocks, s->g_val);
+    FSD_CHECK_CUDA(cudaGetLastError());
     return FSD_OK;
 }
 

@@ -30,7 +30,7 @@ struct BsrArgs {
 const void* bsr_kernel(int mode);
 int bsr_blocks(int N);
 void bsr_launch(int mode, const BsrArgs& a, cudaStream_t st);
-int bsr_import(fsd_handle* h, int nnzb, const float* blocks);
+int bsr_import(fsd_handle* h, const float* blocks);
 int bsr_sync_a(fsd_handle* h);
 
 struct LearnedState {

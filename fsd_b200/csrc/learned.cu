@@ -67,6 +67,25 @@ int learned_reserve(fsd_handle* h, int nnzb) {
     return FSD_OK;
 }
 
+// A checked block-CSR G from the caller's arrays, which may lie on another
+// device; `staged` receives its blocks as they came.
+static int learned_take_blocks(fsd_handle* h, int nnzb, const int* d_rowptr, const int* d_col, const float* d_val,
+                               float* staged) {
+    const int N = h->p.N;
+    const size_t nb = (size_t)nnzb;
+    const int e = learned_reserve(h, nnzb);
+    if (e != FSD_OK) return e;
+    LearnedState* s = learned(h);
+    FSD_CHECK_CUDA(cudaMemcpyAsync(s->g_rowptr, d_rowptr, sizeof(int) * (N + 1), cudaMemcpyDeviceToDevice, h->stream));
+    if (nnzb) {
+        FSD_CHECK_CUDA(cudaMemcpyAsync(s->g_col, d_col, sizeof(int) * nb, cudaMemcpyDeviceToDevice, h->stream));
+        FSD_CHECK_CUDA(cudaMemcpyAsync(staged, d_val, sizeof(float) * 36 * nb, cudaMemcpyDeviceToDevice, h->stream));
+    }
+    s->g_nnzb = nnzb;
+    s->g_user = true;
+    return nnzb ? bsr_import(h, staged) : FSD_OK;
+}
+
 // Copy a caller's block-CSR G after checking its structure on the host, so
 // that no kernel ever indexes outside the vectors it reads.
 int learned_set_blocks(fsd_handle* h, int nnzb, const int* d_rowptr, const int* d_col, const float* d_val) {
@@ -83,16 +102,13 @@ int learned_set_blocks(fsd_handle* h, int nnzb, const int* d_rowptr, const int* 
         if (rp[i + 1] < rp[i]) return FSD_ERR_BAD_PARAMS;
     for (int c : cl)
         if (c < 0 || c >= N) return FSD_ERR_BAD_PARAMS;
-    const int e = learned_reserve(h, nnzb);
-    if (e != FSD_OK) return e;
-    LearnedState* s = learned(h);
-    FSD_CHECK_CUDA(cudaMemcpyAsync(s->g_rowptr, d_rowptr, sizeof(int) * (N + 1), cudaMemcpyDeviceToDevice, h->stream));
-    if (nnzb)
-        FSD_CHECK_CUDA(cudaMemcpyAsync(s->g_col, d_col, sizeof(int) * (size_t)nnzb, cudaMemcpyDeviceToDevice,
-                                       h->stream));
-    s->g_nnzb = nnzb;
-    s->g_user = true;
-    return bsr_import(h, nnzb, d_val);
+    // the blocks as they came, until they are laid out by components; taken
+    // before anything of the present G changes
+    float* staged = nullptr;
+    if (nnzb) FSD_CHECK_CUDA(cudaMalloc(&staged, sizeof(float) * 36 * (size_t)nnzb));
+    const int e = learned_take_blocks(h, nnzb, d_rowptr, d_col, d_val, staged);
+    if (staged) cudaFree(staged);  // waits for the layout
+    return e;
 }
 
 // ----------------------------------------------------------- inner solve
